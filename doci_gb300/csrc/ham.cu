@@ -69,7 +69,8 @@ void ham_release(doci_ham *h) {
   if (!h) return;
   cudaStream_t st = h->stream;
   void *bufs[] = {h->d_binom, h->d_Kmir64, h->d_Kmir32, h->d_tab64, h->d_diag, h->d_diag32, h->d_stage_x,
-                  h->d_stage_y, h->d_rows, h->d_rowstart, h->d_pblocks, h->d_pblocks_host, h->d_kfrag, h->d_tc_err};  // d_rem/d_ins/d_ins_t/d_tab_off are shared (per-process cache)
+                  h->d_stage_y, h->d_rows, h->d_rowstart, h->d_pblocks, h->d_pblocks_host, h->d_kfrag, h->d_tc_err,
+                  h->d_wstart, h->d_wunits};  // d_rem/d_ins/d_ins_t/d_tab_off are shared (per-process cache)
   for (void *p : bufs) release_async(p, st);
   if (h->h_diag) cudaFreeHost(h->h_diag);
   if (st) {
@@ -108,6 +109,9 @@ void ham_release(doci_ham *h) {
   h->d_rows = h->d_rowstart = nullptr;
   h->d_pblocks = nullptr;
   h->d_kfrag = nullptr;
+  h->d_wstart = h->d_wunits = nullptr;
+  h->d_wtab_a = h->d_wtab_b = nullptr;
+  h->wsplit = 0;
   h->d_tc_err = nullptr;
   h->npblocks = 0;
   h->d_rem = h->d_ins = h->d_ins_t = h->d_tab_off = nullptr;
@@ -208,6 +212,8 @@ int ham_build(doci_ham *h, const Integrals &in) {
   int st = launch_diagonal(h, h->stream);
   if (st) return st;
   st = ham_build_rows(h);
+  if (st) return st;
+  st = ham_build_pair_warp(h);
   if (st) return st;
   DOCI_CUDA(cudaStreamSynchronize(h->stream));
   return DOCI_OK;

@@ -102,6 +102,11 @@ struct doci_ham {
   uint32_t *d_pblocks = nullptr;
   int npblocks = 0;
   void *d_kfrag = nullptr;
+  // warp-per-unit pair form (sigma_pair_warp.cu): its column orbitals (0: does
+  // not fit), row starts by row-part mask and unit list (masks, four per tile)
+  int wsplit = 0, nwquads = 0;
+  uint32_t *d_wstart = nullptr, *d_wunits = nullptr;
+  const void *d_wtab_a = nullptr, *d_wtab_b = nullptr;  // insertion tables (per-process cache)
   // doci_sigma_host on the pair forms: x and sigma cross the host link in
   // pieces (chunk_off) on copy_stream while the pair units run in groups,
   // alternately on the handle's stream and side_stream (host_plan.h):
@@ -164,6 +169,10 @@ int launch_pair(const doci_ham *h, const float *x, float *y, cudaStream_t s);
 // overlapped with the unit groups; y = dy on stream s, and, for a pinned hy,
 // the pieces of dy copied to hy as they become final (all done when s is)
 int launch_pair_host(doci_ham *h, const float *hx, float *dx, float *dy, float *hy, cudaStream_t s);
+// warp-per-unit pair form on the tensor cores (sigma_pair_warp.cu), FP32 only
+int ham_build_pair_warp(doci_ham *h);
+bool pair_warp_fits(const doci_ham *h);
+int launch_pair_warp(const doci_ham *h, const float *x, float *y, cudaStream_t s);
 // FP64-accurate pair form in float-float arithmetic (sigma_pair.cu)
 bool pair_ff_fits(const doci_ham *h);
 int launch_pair_ff(const doci_ham *h, const double *x, double *y, cudaStream_t s);
@@ -173,6 +182,7 @@ int launch_pair_ff_host(doci_ham *h, const double *hx, double *dx, double *dy, d
 // A device wait that runs out writes a nonzero code to *d_err (spin_limit:
 // try_wait iterations per wait).
 constexpr long kTcSpinLimit = 1L << 20;  // try_wait polls per wait (seconds at most)
+long tc_spin_limit();
 bool tc_fits(const doci_ham *h);
 int tc_launches(const doci_ham *h);
 int launch_tc(const doci_ham *h, const float *x, float *y, cudaStream_t s, int *d_err, long spin_limit);

@@ -843,7 +843,7 @@ SigmaPlan plan_kind(const doci_ham *h, int precision, bool allow_pair, int kind)
     // mma.sync pair form: the automatic FP32 choice where it fits and the
     // space gives every SM blocks of work (measured fastest there)
     const bool want_pair = kind == 6 || kind == 8 || (kind == 0 && h->npblocks >= device_sm_count());
-    if (want_pair && pair_fits(h)) return {6, 2};  // init pass + pair pass
+    if (want_pair && pair_fits(h)) return {6, 2};  // zero (or diag x) pass + pair pass
   }
   // float-float sigma (FP64 accuracy in FP32 arithmetic): the pair form, or
   // the phase-ordered row pass where the pair tiling does not fit; the x
@@ -899,6 +899,10 @@ int launch_sigma(const doci_ham *h, const void *x, void *y, int precision, cudaS
       return pair_fits(h) ? launch_pair(h, static_cast<const float *>(x), static_cast<float *>(y), st)
                           : launch_row<float>(h, x, y, st, 1);
     case 6:
+      // from 10 orbitals on the warp-per-unit form (faster at every size measured
+      // from L=18 on: 18.8 -> 16.7 us there, 33.9 -> 19.1 ms at L=32)
+      if (pair_warp_fits(h))
+        return launch_pair_warp(h, static_cast<const float *>(x), static_cast<float *>(y), st);
       return launch_pair(h, static_cast<const float *>(x), static_cast<float *>(y), st);
     case 1:
       return f64 ? launch_typed<double>(h, x, y, st) : launch_typed<float>(h, x, y, st);

@@ -1,0 +1,503 @@
+// sigma_pair_warp.cu -- FP32 sigma in the (N-1)-pair form (sigma_pair.cu has
+// the regrouping: sigma[T] = diag[T] x[T] + sum_{i in T} Y_{T\i}[i],
+// Y_S = X_S K), one warp per unit, the product with K on the 5th-generation
+// tensor cores.  This is what kind 6 runs from 10 orbitals on.
+//
+// A warp walks the sets of one unit (pair_warp_index.cuh), 32 at a time, one
+// set per lane, which is also the set's lane in tensor memory.  The unit's own
+// row, at most C(12,6) = 924 elements, has its x and its sums in shared memory
+// private to the warp: the random accesses of the column orbitals stay on
+// chip, and since S -> S u o is one to one the sums are plain
+// read-modify-writes, one orbital after the other, with no atomics.  The rows
+// of the row-part holes are read and added to at the set's own column, 32
+// consecutive elements at a time.  The orbital axis is not compacted, so K
+// (high and low TF32 parts, 64 x 32, the B operand) is the same for every unit
+// and four warps with units of their own share one 128-row MMA tile.
+//
+// TF32 three ways (x high x K high, x high x K low, x low x K high): the first
+// two as one MMA of 64 columns, since an MMA of 128 rows takes the same 51
+// cycles for 32 and for 64 columns on GB300 (24.6 ns in a run of 96; 72 cycles
+// at 128 columns).  The two halves are added when they are read back.
+//
+// Column orbitals: 12 as long as that leaves four units per resident warp,
+// else 10 as long as each has one, else 8.  Larger rows mean fewer set-ups
+// and fewer row-part orbitals to look at, smaller ones more units to spread.
+// Measured (us, 12 / 10 / 8): L=32 N=16 19,120 / 22,940 / 38,470;
+// L=26 N=13 347 / 362 / 562; L=24 N=12 107 / 103 / 138;
+// L=22 N=11 70 / 38 / 46; L=21 N=9 70 / 27.6 / 25.1; L=18 N=9 69 / 27 / 16.8.
+//
+// Measured against the one-block-per-unit mma.sync kernel of sigma_pair.cu:
+// L=32 N=16 33.9 -> 19.1 ms, L=28 N=14 1.82 -> 1.23 ms, L=27 N=11 524 -> 331 us,
+// L=20 N=10 28.0 -> 20.9 us.  Bound by instruction issue and the latency of the
+// hole rows (about 600 warp instructions per 32 sets; 16 warps per SM by the
+// 128 tensor-memory columns of a tile).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+#include <vector>
+
+#include "addressing.cuh"
+#include "internal.h"
+#include "pair_warp_index.cuh"
+
+namespace doci {
+namespace {
+
+constexpr int kWgs = 4;                     // warpgroups: tiles in flight
+constexpr int kThreads = 128 * kWgs;
+constexpr uint32_t kTmemCols = 512;         // per warpgroup: A high 32 | A low 32 | D 64
+// tcgen05 instruction descriptor: D FP32, A and B TF32, both K-major, M = 128
+__host__ __device__ constexpr uint32_t idesc(uint32_t n) {
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+}
+constexpr int kOffBar = 64 * 128;           // after K: 64 rows (high, low) x 32 columns, swizzled
+constexpr int kOffStart = kOffBar + 128;    // row starts of a warp's hole rows, 24 per warp
+constexpr int kOffRows = kOffStart + 4 * 24 * (kThreads / 32);
+constexpr size_t kMinSmem = 120 * 1024;     // one block per SM: it allocates all of the tensor memory
+
+struct PwShape {
+  uint32_t D;
+  int L, N, na, nquads;
+  long spin_limit;
+  uint32_t n[16];    // C(P, j), 0 from j = P + 1
+  uint32_t off[16];  // first set of j elements in the tables
+};
+
+__device__ __forceinline__ uint32_t su32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ float lds(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts(uint32_t a, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+// *p where on, else 0; *p += v where on (predicated: `on` is the same in the whole warp or the lane is idle)
+__device__ __forceinline__ float ldg_if(const float *p, uint32_t on) {
+  float v;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}\n"
+      : "=&f"(v)
+      : "l"(p), "r"(on));
+  return v;
+}
+__device__ __forceinline__ void red_if(float *p, float v, uint32_t on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q red.global.add.f32 [%0], %1;\n\t}\n" ::"l"(p), "f"(v),
+               "r"(on)
+               : "memory");
+}
+// (a0, a1) + (b0, b1) and - in one instruction (FP32, round to nearest)
+__device__ __forceinline__ void add2(float &a0, float &a1, float b0, float b1) {
+  asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\tadd.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, "
+      "p;\n\t}\n"
+      : "+f"(a0), "+f"(a1)
+      : "f"(b0), "f"(b1));
+}
+__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(a), "r"(parity), "r"(1000u)
+      : "memory");
+  return ok != 0;
+}
+// the four warps of a warpgroup meet; true when any of them failed
+__device__ __forceinline__ bool group_meet(int wg, bool fail) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, "
+      "q;\n\t}\n"
+      : "=r"(r)
+      : "r"(static_cast<uint32_t>(fail)), "r"(wg + 1)
+      : "memory");
+  return r != 0;
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
+  // K-major, 128-byte swizzle: leading offset unused (16 B), 8-row groups 1024 B apart, version 1
+  return static_cast<uint64_t>((addr >> 4) & 0x3FFFu) | (static_cast<uint64_t>(1) << 16) |
+         (static_cast<uint64_t>(1024 >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
+         (static_cast<uint64_t>(2) << 61);
+}
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t id, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d),
+      "r"(a), "l"(b), "r"(id), "r"(acc));
+}
+__device__ __forceinline__ void tld16(uint32_t t, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(t));
+}
+__device__ __forceinline__ void tst16(uint32_t t, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(t),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+// nearest TF32 (10-bit mantissa), ties away from zero: half a TF32 ulp added to
+// the magnitude, the low 13 bits cut (two integer instructions; cvt.rna.tf32
+// measured about five)
+__device__ __forceinline__ uint32_t tf32_rna(float f) { return (__float_as_uint(f) + 0x1000u) & 0xffffe000u; }
+// byte offset of element (row r, column k) of a 128-byte-swizzled K-major tile of 32 FP32 per row
+__host__ __device__ __forceinline__ uint32_t sw128(uint32_t r, uint32_t k) {
+  return (r >> 3) * 1024u + (r & 7u) * 128u + ((((k >> 2) ^ r) & 7u) << 4) + (k & 3u) * 4u;
+}
+
+template <int P>
+__global__ void __launch_bounds__(kThreads, 1)
+sigma_pair_warp_kernel(const __grid_constant__ PwShape s, const uint32_t *__restrict__ units,
+                       const uint32_t *__restrict__ rowstart, const uint4 *__restrict__ tab_a,
+                       const uint2 *__restrict__ tab_b, const float *__restrict__ g_ksplit,
+                       const float *__restrict__ diag, const float *__restrict__ x, float *__restrict__ y,
+                       int *__restrict__ err) {
+  constexpr int NR = 32 - P;
+  constexpr int XC = pw::cells(P);
+  extern __shared__ __align__(1024) uint8_t sm[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = warp >> 2, w4 = warp & 3;
+  const uint32_t base = su32(sm);
+  if (base & 1023u) {  // the swizzled K tile needs a 1024-byte aligned base
+    if (tid == 0) atomicCAS(err, 0, 3);
+    return;
+  }
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + kOffBar + 64);
+  const uint32_t bar = base + kOffBar + 8 * wg;
+  float *xo = reinterpret_cast<float *>(sm + kOffRows) + warp * 2 * XC, *yo = xo + XC;
+  const uint32_t xa = su32(xo), ra = base + kOffStart + warp * 96;
+
+  for (int e = tid; e < 64 * 32; e += kThreads) {
+    const int r = e >> 5, k = e & 31;
+    *reinterpret_cast<float *>(sm + sw128(r, k)) = g_ksplit[(r >> 5) * 1024 + (r & 31) * 32 + k];
+  }
+  if (tid == 0) {
+    for (int i = 0; i < kWgs; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(base + kOffBar + 8 * i));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (lane == 0) xo[XC - 1] = 0.f;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tslot)),
+                 "r"(kTmemCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = *tslot;
+  const uint32_t tg = tmem + 128u * wg, tw = tg + (static_cast<uint32_t>(32 * w4) << 16);
+  const int nks = (s.L + 7) >> 3;  // >= 2 (L >= 10)
+  const uint64_t desc = smem_desc(base);
+
+  uint32_t waited = 0, issued = 0;
+  bool fail = false, stop = false;
+  for (int q = blockIdx.x * kWgs + wg; q < s.nquads && !stop; q += gridDim.x * kWgs) {
+    const uint32_t mask = units[4 * q + w4];
+    const int jp = s.N - 1 - __popc(units[4 * q]);
+    const uint32_t n_s = jp >= 0 ? s.n[jp] : 0u;
+    const bool real = mask != pw::kNone;
+    const uint32_t n_own = real ? s.n[jp + 1] : 0u;
+    const uint32_t holes = real ? ~mask & ((1u << s.na) - 1u) : 0u;
+    const uint32_t own = n_own ? rowstart[mask] : 0u;
+    for (uint32_t c = lane; c < n_own; c += 32) {
+      xo[c] = __ldg(x + own + c);
+      yo[c] = 0.f;
+    }
+    // (a unit without sets has no hole rows either)
+    if (lane < 24) {
+      const bool hole = n_s && ((holes >> lane) & 1u);
+      reinterpret_cast<uint32_t *>(sm + kOffStart)[warp * 24 + lane] = hole ? rowstart[mask | (1u << lane)] : 0u;
+    }
+    __syncwarp();
+    if (n_s) {
+      const uint4 *ta = tab_a + s.off[jp];
+      const uint2 *tb = tab_b + s.off[jp];
+      float v[32];
+      uint32_t at[P];  // this set's own-row cells (shared-memory addresses)
+      const uint32_t last = n_s - 1;
+      // the set's 32 values by orbital: column orbitals from the own row (the
+      // zero cell where the orbital is in the set), row-part holes from their
+      // rows (the table ends each set size with a full warp of zero cells)
+      auto gather = [&](uint32_t c0) {
+        const float *xl = x + min(c0 + lane, last);
+#pragma unroll
+        for (int b = 0; b < NR; b += 4) {
+          const uint4 r = lds128(ra + 4 * b);
+          v[P + b] = ldg_if(xl + r.x, holes & (1u << b));
+          v[P + b + 1] = ldg_if(xl + r.y, holes & (1u << (b + 1)));
+          if (b + 2 < NR) v[P + b + 2] = ldg_if(xl + r.z, holes & (1u << (b + 2)));
+          if (b + 3 < NR) v[P + b + 3] = ldg_if(xl + r.w, holes & (1u << (b + 3)));
+        }
+        uint32_t w[6];
+        const uint4 ea = __ldg(ta + c0 + lane);
+        w[0] = ea.x;
+        w[1] = ea.y;
+        w[2] = ea.z;
+        w[3] = ea.w;
+        if (P > 8) {
+          const uint2 eb = __ldg(tb + c0 + lane);
+          w[4] = eb.x;
+          w[5] = eb.y;
+        }
+#pragma unroll
+        for (int o = 0; o < P; ++o) {
+          at[o] = xa + (o & 1 ? w[o >> 1] >> 16 : w[o >> 1] & 0xffffu);
+          v[o] = lds(at[o]);
+        }
+      };
+      // v split into TF32 high and low parts in this lane's row of the tile
+      auto store = [&]() {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t r[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) r[i] = tf32_rna(v[16 * h + i]);
+          tst16(tw + 16 * h, r);
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            float a0 = v[16 * h + i], a1 = v[16 * h + i + 1];
+            add2(a0, a1, -__uint_as_float(r[i]), -__uint_as_float(r[i + 1]));
+            r[i] = __float_as_uint(a0);
+            r[i + 1] = __float_as_uint(a1);
+          }
+          tst16(tw + 32 + 16 * h, r);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      };
+      auto issue = [&]() {
+        if (w4 == 0 && lane == 0) {
+          fence_after();
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            if (ks < 2 || ks < nks) mma_ts(tg + 64, tg + 8 * ks, desc + 2 * ks, idesc(64), ks > 0);
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            if (ks < 2 || ks < nks) mma_ts(tg + 64, tg + 32 + 8 * ks, desc + 2 * ks, idesc(32), 1);
+          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+                       : "memory");
+        }
+        ++issued;
+        __syncwarp();
+      };
+      gather(0);
+      store();
+      fence_before();
+      stop = group_meet(wg, fail);
+      if (!stop) issue();
+      for (uint32_t c0 = 0; c0 < n_s && !stop; c0 += 32) {
+        const bool more = c0 + 32 < n_s;
+        uint32_t cur[P];
+#pragma unroll
+        for (int o = 0; o < P; ++o) cur[o] = at[o];
+        if (more) gather(c0 + 32);
+        bool done = false;
+        for (long k = 0; k < s.spin_limit && !done; ++k) done = mbar_try(bar, waited & 1u);
+        done = __all_sync(0xffffffffu, done);
+        ++waited;
+        if (!done) {
+          fail = true;
+          if (lane == 0) atomicCAS(err, 0, 21);
+        }
+        fence_after();
+        if (more) store();
+        float yv[32];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t r[16], l[16];
+          tld16(tw + 64 + 16 * h, r);
+          tld16(tw + 96 + 16 * h, l);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            yv[16 * h + i] = __uint_as_float(r[i]);
+            yv[16 * h + i + 1] = __uint_as_float(r[i + 1]);
+            add2(yv[16 * h + i], yv[16 * h + i + 1], __uint_as_float(l[i]), __uint_as_float(l[i + 1]));
+          }
+        }
+        fence_before();
+        stop = group_meet(wg, fail);
+        if (stop) break;
+        if (more) issue();
+        // own row: one orbital at a time no two sets meet (S -> S u o is one to
+        // one), and the warp alone adds to it
+#pragma unroll
+        for (int o = 0; o < P; ++o) {
+          sts(cur[o] + 4 * XC, lds(cur[o] + 4 * XC) + yv[o]);
+          __syncwarp();
+        }
+        float *yl = y + c0 + lane;
+        const uint32_t add = c0 + lane <= last ? holes : 0u;
+#pragma unroll
+        for (int b = 0; b < NR; b += 4) {
+          const uint4 r = lds128(ra + 4 * b);
+          red_if(yl + r.x, yv[P + b], add & (1u << b));
+          red_if(yl + r.y, yv[P + b + 1], add & (1u << (b + 1)));
+          if (b + 2 < NR) red_if(yl + r.z, yv[P + b + 2], add & (1u << (b + 2)));
+          if (b + 3 < NR) red_if(yl + r.w, yv[P + b + 3], add & (1u << (b + 3)));
+        }
+      }
+    }
+    __syncwarp();
+    if (!stop)
+      for (uint32_t c = lane; c < n_own; c += 32) atomicAdd(y + own + c, fmaf(diag[own + c], xo[c], yo[c]));
+    __syncwarp();
+  }
+  // after a wait that ran out: the MMAs in flight complete by themselves;
+  // wait for them (bounded) before the tensor memory is freed
+  if (stop && w4 == 0 && issued > 0) {
+    for (long i = 0; i < kTcSpinLimit && !mbar_try(bar, (issued - 1) & 1u); ++i) {
+    }
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+}
+
+__global__ void zero_kernel(float *__restrict__ y, uint32_t n) {
+  const uint32_t head = min(n, static_cast<uint32_t>((16 - (reinterpret_cast<uintptr_t>(y) & 15)) & 15) / 4);
+  const uint32_t n4 = (n - head) / 4, i0 = blockIdx.x * blockDim.x + threadIdx.x;
+  float4 *y4 = reinterpret_cast<float4 *>(y + head);
+  for (uint32_t i = i0; i < n4; i += gridDim.x * blockDim.x) y4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (i0 < head) y[i0] = 0.f;
+  if (i0 < n - head - 4 * n4) y[head + 4 * n4 + i0] = 0.f;
+}
+
+__global__ void build_starts_kernel(uint32_t *out, int P, int na, int N, uint32_t D, const uint32_t *binom) {
+  for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < (1u << na); m += gridDim.x * blockDim.x)
+    out[m] = pw::row_start(m, P, na, N, D, binom, kBinomCols);
+}
+__global__ void build_units_kernel(uint32_t *out, pw::Groups g, int na, const uint32_t *binom) {
+  const uint32_t total = g.first[g.n];
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    int k = 0;
+    while (k + 1 < g.n && g.first[k + 1] <= i) ++k;
+    const uint32_t j = i - g.first[k];
+    out[i] = j < g.count[k] ? dev::colex_unrank<kBinomCols>(j, na, g.kp[k], binom) : pw::kNone;
+  }
+}
+
+// the insertion tables, once per device and column-orbital count
+struct PwTables {
+  uint4 *a = nullptr;
+  uint2 *b = nullptr;
+};
+int pw_tables(int device, int P, PwTables *out) {
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, PwTables> cache;
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_pair(device, P);
+  auto it = cache.find(key);
+  if (it == cache.end()) {
+    std::vector<uint32_t> B(kBinomRows * kBinomCols), off;
+    std::vector<uint16_t> a, b;
+    fill_binom_table(B.data());
+    pw::build_tables(P, B.data(), kBinomCols, a, b, off);
+    PwTables t;
+    DOCI_CUDA(cudaMalloc(&t.a, a.size() * sizeof(uint16_t)));
+    DOCI_CUDA(cudaMalloc(&t.b, b.size() * sizeof(uint16_t)));
+    DOCI_CUDA(cudaMemcpy(t.a, a.data(), a.size() * sizeof(uint16_t), cudaMemcpyHostToDevice));
+    DOCI_CUDA(cudaMemcpy(t.b, b.data(), b.size() * sizeof(uint16_t), cudaMemcpyHostToDevice));
+    it = cache.emplace(key, t).first;
+  }
+  *out = it->second;
+  return DOCI_OK;
+}
+
+template <int P>
+int launch_p(const doci_ham *h, const PwShape &s, const float *x, float *y, cudaStream_t st) {
+  const size_t smem = std::max(kMinSmem, static_cast<size_t>(kOffRows) + 2 * 4 * pw::cells(P) * (kThreads / 32));
+  int per_sm = 1;
+  const int r = kernel_blocks(reinterpret_cast<const void *>(sigma_pair_warp_kernel<P>), kThreads, smem, &per_sm);
+  if (r != DOCI_OK) return r;
+  const int grid = std::min(device_sm_count(), (s.nquads + kWgs - 1) / kWgs);
+  sigma_pair_warp_kernel<P><<<grid, kThreads, smem, st>>>(s, h->d_wunits, h->d_wstart,
+                                                          static_cast<const uint4 *>(h->d_wtab_a),
+                                                          static_cast<const uint2 *>(h->d_wtab_b),
+                                                          reinterpret_cast<const float *>(h->d_kfrag), h->d_diag32, x,
+                                                          y, h->d_tc_err);
+  DOCI_CUDA(cudaGetLastError());
+  return DOCI_OK;
+}
+
+}  // namespace
+
+bool pair_warp_fits(const doci_ham *h) { return h->wsplit > 0; }
+
+int ham_build_pair_warp(doci_ham *h) {
+  h->wsplit = 0;
+  const int L = h->L, N = h->N;
+  if (L < 10 || N < 1) return DOCI_OK;
+  int major = 0, minor = 0;
+  cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, h->device);
+  cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, h->device);
+  if (major != 10 || minor != 3) return DOCI_OK;
+  std::vector<uint32_t> B(kBinomRows * kBinomCols);
+  fill_binom_table(B.data());
+  int P = 0;
+  pw::Groups g;
+  for (int p : {12, 10, 8}) {
+    if (L - p < 2 || L - p > 24) continue;
+    P = p;
+    g = pw::groups(P, L - P, N, B.data(), kBinomCols);
+    const uint32_t slots = static_cast<uint32_t>(kWgs * device_sm_count());
+    if (g.first[g.n] / 4 >= (p == 12 ? 4 : 1) * slots) break;
+  }
+  const int na = L - P;
+  const uint32_t total = g.first[g.n];
+  DOCI_CUDA(cudaMallocAsync(&h->d_wstart, sizeof(uint32_t) << na, h->stream));
+  DOCI_CUDA(cudaMallocAsync(&h->d_wunits, sizeof(uint32_t) * total, h->stream));
+  const int blocks = 4 * device_sm_count();
+  build_starts_kernel<<<std::min(blocks, ((1 << na) + 255) / 256), 256, 0, h->stream>>>(h->d_wstart, P, na, N, h->D,
+                                                                                       h->d_binom);
+  build_units_kernel<<<std::min<int>(blocks, (total + 255) / 256), 256, 0, h->stream>>>(h->d_wunits, g, na,
+                                                                                       h->d_binom);
+  DOCI_CUDA(cudaGetLastError());
+  h->nwquads = static_cast<int>(total / 4);
+  PwTables t;
+  const int r = pw_tables(h->device, P, &t);
+  if (r != DOCI_OK) return r;
+  h->d_wtab_a = t.a;
+  h->d_wtab_b = t.b;
+  h->wsplit = P;
+  return DOCI_OK;
+}
+
+int launch_pair_warp(const doci_ham *h, const float *x, float *y, cudaStream_t st) {
+  if (!pair_warp_fits(h)) return DOCI_ERR_INVALID;
+  const int P = h->wsplit;
+  PwShape s{};
+  s.D = h->D;
+  s.L = h->L;
+  s.N = h->N;
+  s.na = h->L - P;
+  s.nquads = h->nwquads;
+  s.spin_limit = tc_spin_limit();
+  uint32_t at = 0;
+  for (int j = 0; j <= P; ++j) {
+    s.n[j] = static_cast<uint32_t>(binom64(P, j));
+    s.off[j] = at;
+    at += pw::padded(s.n[j]);
+  }
+  zero_kernel<<<static_cast<unsigned>(std::min<uint64_t>((h->D / 4 + 256) / 256, 8ull * device_sm_count())), 256, 0,
+                st>>>(y, h->D);
+  DOCI_CUDA(cudaGetLastError());
+  if (P == 12) return launch_p<12>(h, s, x, y, st);
+  if (P == 10) return launch_p<10>(h, s, x, y, st);
+  return launch_p<8>(h, s, x, y, st);
+}
+
+}  // namespace doci

@@ -175,9 +175,10 @@ int doci_sigma_block(doci_ham *ham, const void *d_X, int64_t ldx, void *d_Y, int
  * with a row tiling kind 3 for FP32 and kind 4 for FP64; else kind 1),
  * 1 the per-determinant gather kernel, 3 the row pass doing all hops, 4 the
  * phase-ordered row pass (cross hops staged one source row at a time), 6 the
- * (N-1)-pair form on the warp-level tensor-core path (FP32 only: gather the
- * neighbours of every (N-1)-pair set, multiply by K, scatter with atomic
- * adds), 8 the (N-1)-pair form on the 5th-generation tensor cores (FP32
+ * (N-1)-pair form with one warp per group of sets (FP32 only: gather the
+ * neighbours of every (N-1)-pair set, multiply by K on the tensor cores,
+ * scatter, atomic adds between groups; below 10 orbitals and in
+ * doci_sigma_host the product runs on mma.sync), 8 the (N-1)-pair form on the 5th-generation tensor cores (FP32
  * only: the own row of a set's row part staged in shared memory, the other
  * rows streamed by TMA, the product in TMEM, each own row written once;
  * needs a 16-byte aligned x, else kind 6 runs), 9 the (N-1)-pair form in
@@ -189,7 +190,7 @@ int doci_sigma_block(doci_ham *ham, const void *d_X, int64_t ldx, void *d_Y, int
  * sigma with atomic adds, so their last bits vary between runs; FP64
  * requests for them use the automatic choice.  3-9 fall back to 1 when the
  * handle has no row tiling.  Other values: DOCI_ERR_INVALID.  A device wait
- * of kind 8 that runs out (it never should) is reported as
+ * of kind 6 or 8 that runs out (it never should) is reported as
  * DOCI_ERR_DEVICE_TIMEOUT by the handle's next synchronous call
  * (doci_sigma_host, doci_solve).  For tests and tuning. */
 int doci_ham_set_sigma_kernel(doci_ham *ham, int kind);

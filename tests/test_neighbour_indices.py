@@ -147,3 +147,29 @@ def test_host_schedule_orders_copies_and_groups(plan_exe, L, N, split):
 def test_host_schedule_check_catches_planted_mistakes(plan_exe, plant):
     r = subprocess.run([plan_exe, "32", "16", "16", plant], capture_output=True, text=True)
     assert r.returncode == 1 and "bad=0" not in r.stdout, r.stdout + r.stderr
+
+
+WARP_SRC = os.path.join(HERE, "host_checks", "pair_warp_check.cu")
+
+
+@pytest.fixture(scope="module")
+def warp_exe(tmp_path_factory):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not available")
+    out = str(tmp_path_factory.mktemp("pwarp") / "pair_warp_check")
+    subprocess.run([nvcc, "-O2", "-std=c++17", "-diag-suppress=20011", WARP_SRC, "-o", out], check=True)
+    return out
+
+
+@pytest.mark.parametrize("L,N,P,us,ss", [
+    # whole spaces: every determinant reached once per pair it holds, in one unit's own row
+    (10, 5, 8, 1, 1), (12, 1, 8, 1, 1), (12, 11, 8, 1, 1), (12, 12, 8, 1, 1), (16, 8, 10, 1, 1), (18, 9, 12, 1, 1),
+    (20, 10, 8, 1, 1), (22, 11, 10, 1, 1), (22, 8, 12, 1, 1), (32, 2, 12, 1, 1), (32, 30, 8, 1, 1), (32, 3, 8, 1, 1),
+    # sampled large spaces
+    (32, 16, 12, 5003, 101), (31, 15, 12, 4001, 29), (28, 14, 12, 97, 31), (27, 11, 12, 37, 31), (24, 12, 10, 17, 7),
+])
+def test_warp_pair_form_ranks(warp_exe, L, N, P, us, ss):
+    r = subprocess.run([warp_exe, str(L), str(N), str(P), str(us), str(ss)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert "bad=0" in r.stdout

@@ -370,3 +370,32 @@ def test_autotune_keeps_parity(synth, dg):
             for v in range(3):
                 ref = o.matvec(X[v].double().cpu().numpy())
                 assert np.abs(Y[v].double().cpu().numpy() - ref).max() <= tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("L,N,seed,off", [
+    (10, 1, 81, 0), (10, 5, 82, 1), (11, 10, 83, 2), (13, 13, 84, 3), (32, 2, 85, 1),  # 8 column orbitals
+    (22, 8, 86, 3), (23, 9, 87, 1), (24, 20, 88, 0),  # 10
+    (28, 6, 89, 1), (26, 19, 90, 3),  # 12
+])
+def test_sigma_pair_warp_edges(L, N, seed, off, synth, dg):
+    """The warp-per-unit pair form on each of its tilings (8, 10 and 12 column
+    orbitals), at the smallest and nearly full spaces, odd lengths and buffers
+    off 16-byte alignment, with y full of NaN before the call: the oracle's
+    matvec within the FP32 sigma tolerance, nothing written around y."""
+    torch = torch_cuda()
+    p = synth(L, N, seed)
+    o = oracle.Ham(p)
+    with dg.Hamiltonian.from_fcidump(p) as h:
+        h.set_sigma_kernel("pair")
+        assert h.sigma_plan(dg.FP32)[0] == 6
+        D = h.D
+        x = np.random.default_rng(seed).standard_normal(D).astype(np.float32)
+        xs = torch.zeros(D + 8, dtype=torch.float32, device="cuda")
+        xs[off:off + D] = torch.from_numpy(x)
+        ys = torch.full((D + 8,), float("nan"), dtype=torch.float32, device="cuda")
+        h.sigma_device(xs[off:].data_ptr(), ys[off:].data_ptr(), dg.FP32)
+        torch.cuda.synchronize()
+        yr = o.matvec(x.astype(np.float64))
+        y = ys.double().cpu().numpy()
+        assert np.abs(y[off:off + D] - yr).max() <= TOL32 * np.abs(yr).max()
+        assert np.isnan(y[:off]).all() and np.isnan(y[off + D:]).all()
