@@ -44,8 +44,12 @@ int grid_blocks() { return device_sm_count() * 4; }
 // reduction launch is needed.
 constexpr int kHeader = 1 + kMaxK;
 
+// With column groups (blockIdx.x; the rows are blockIdx.y) a block holds nk of
+// the row's `width` results, from column `first` on; the last block of all
+// groups sums them all.
 template <int K>
-__device__ __forceinline__ void block_reduce_store(double (&acc)[K], int nk, double *partials) {
+__device__ __forceinline__ void block_reduce_store(double (&acc)[K], int nk, double *partials, int width = 0,
+                                                   int first = 0) {
   __shared__ double red[32][kMaxK];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -60,21 +64,24 @@ __device__ __forceinline__ void block_reduce_store(double (&acc)[K], int nk, dou
   }
   __syncthreads();
   double *rows = partials + kHeader;
+  const bool groups = width > 0;
+  if (!groups) width = nk;
+  const unsigned row = groups ? blockIdx.y : blockIdx.x, nrows = groups ? gridDim.y : gridDim.x;
   if (threadIdx.x < nk) {
     double s = 0;
     for (int w = 0; w < nw; ++w) s += red[w][threadIdx.x];
-    rows[static_cast<size_t>(blockIdx.x) * nk + threadIdx.x] = s;
+    rows[static_cast<size_t>(row) * width + first + threadIdx.x] = s;
   }
   __threadfence();
   __syncthreads();
   unsigned int *counter = reinterpret_cast<unsigned int *>(partials);
-  if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x * gridDim.y - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
-  for (int k = warp; k < nk; k += nw) {
+  for (int k = warp; k < width; k += nw) {
     double s = 0;
-    for (unsigned b = lane; b < gridDim.x; b += 32) s += __ldcg(rows + static_cast<size_t>(b) * nk + k);
+    for (unsigned b = lane; b < nrows; b += 32) s += __ldcg(rows + static_cast<size_t>(b) * width + k);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (lane == 0) partials[1 + k] = s;
@@ -82,21 +89,121 @@ __device__ __forceinline__ void block_reduce_store(double (&acc)[K], int nk, dou
   if (threadIdx.x == 0) *counter = 0u;
 }
 
-// partials of V_i . w for i < m
-template <typename S, int K>
-__global__ void __launch_bounds__(kT)
-multidot_kernel(const S *__restrict__ V, size_t ld, int m, const S *__restrict__ w, size_t n,
+// partials of V_i . w for i < m, FP64.  The columns go in groups of four, one
+// per block (blockIdx.x, so that the groups of a stretch run together and w
+// comes from L2 after the first), with the loads of four elements in flight.
+// The FP64 units bound it from about ten columns on (one FMA per element:
+// 1.03 ms for 16 columns of 40.1M).  Each thread's and each column's order of
+// additions is that of a block holding all columns.
+constexpr int kAhead = 4, KG = 4;
+__global__ void __launch_bounds__(kT, 4)
+multidot_kernel(const double *__restrict__ V, size_t ld, int m, const double *__restrict__ w, size_t n,
                 double *__restrict__ partials) {
-  double acc[K];
+  const int k0 = blockIdx.x * KG, mk = min(KG, m - k0);
+  V += k0 * ld;
+  double acc[KG];
 #pragma unroll
-  for (int k = 0; k < K; ++k) acc[k] = 0;
-  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < n; j += (size_t)gridDim.x * blockDim.x) {
-    const double wj = static_cast<double>(w[j]);
+  for (int k = 0; k < KG; ++k) acc[k] = 0;
+  const size_t stride = (size_t)gridDim.y * blockDim.x;
+  size_t j = blockIdx.y * (size_t)blockDim.x + threadIdx.x;
+  for (; j + (kAhead - 1) * stride < n; j += kAhead * stride) {
+    double v[kAhead][KG], wj[kAhead];
 #pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (k < m) acc[k] += static_cast<double>(V[k * ld + j]) * wj;
+    for (int a = 0; a < kAhead; ++a) {
+      wj[a] = w[j + a * stride];
+#pragma unroll
+      for (int k = 0; k < KG; ++k) v[a][k] = k < mk ? V[k * ld + j + a * stride] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < KG; ++k)
+      if (k < mk) {
+#pragma unroll
+        for (int a = 0; a < kAhead; ++a) acc[k] += v[a][k] * wj[a];
+      }
   }
-  block_reduce_store<K>(acc, m, partials);
+  for (; j < n; j += stride) {
+    const double wj = w[j];
+#pragma unroll
+    for (int k = 0; k < KG; ++k)
+      if (k < mk) acc[k] += V[k * ld + j] * wj;
+  }
+  block_reduce_store<KG>(acc, mk, partials, m, k0);
+}
+
+// The same for FP32 vectors with exact products (doci_multidot), without the
+// FP64 units, whose rate (1/64 of FP32) and widening conversions held the
+// pass at 2.44 ms for 16 columns of 40.1M (1.1 TB/s).  A thread sums runs of
+// kRun products as pairs of floats: p = v w and its rounding error from an
+// FMA (v w = p + e exactly), s + p by Knuth's two-sum (exact), the errors in
+// c; then s and c go to an FP64 sum.  c's own rounding is 2^-24 of terms
+// already 2^-24 small.  That holds while the run's largest product is well
+// inside FP32's range; a run where it is not (all products tiny, an overflow,
+// an infinity, or all zero) is done again in FP64, skipping finite products
+// with a zero factor.
+// Columns go in groups of four, one per block (blockIdx.x, so that the groups
+// of a stretch run together and w comes from L2 after the first): 64 registers,
+// four blocks per SM, sixteen loads of V in flight per thread.  538 us there
+// (5.1 TB/s); groups of eight 568 us with two blocks per SM and 981 us with
+// three (spills), all sixteen columns in one block 770-850 us.
+constexpr int kRun = 64;
+__global__ void __launch_bounds__(kT, 4)
+multidot_exact_f32_kernel(const float *__restrict__ V, size_t ld, int m, const float *__restrict__ w, size_t n,
+                          double *__restrict__ partials) {
+  const int k0 = blockIdx.x * KG, mk = min(KG, m - k0);
+  V += k0 * ld;
+  double acc[KG];
+#pragma unroll
+  for (int k = 0; k < KG; ++k) acc[k] = 0;
+  const size_t stride = (size_t)gridDim.y * blockDim.x;
+  for (size_t j0 = blockIdx.y * (size_t)blockDim.x + threadIdx.x; j0 < n; j0 += stride * kRun) {
+    float s[KG], c[KG], big[KG];
+#pragma unroll
+    for (int k = 0; k < KG; ++k) s[k] = c[k] = big[k] = 0.f;
+    auto add = [&](int k, float v, float wj) {
+      const float p = __fmul_rn(v, wj), e = fmaf(v, wj, -p);
+      const float t = __fadd_rn(s[k], p), z = __fadd_rn(t, -s[k]);
+      const float d = __fadd_rn(__fadd_rn(s[k], -__fadd_rn(t, -z)), __fadd_rn(p, -z));
+      s[k] = t;
+      c[k] = __fadd_rn(c[k], __fadd_rn(e, d));
+      big[k] = fmaxf(big[k], fabsf(p));
+    };
+    const size_t left = (n - j0 + stride - 1) / stride;  // this thread's elements from j0 on
+    const int run = left < kRun ? static_cast<int>(left) : kRun;
+    const float *vp = V + j0, *wp = w + j0;
+    int u = 0;
+    for (; u + kAhead <= run; u += kAhead, vp += kAhead * stride, wp += kAhead * stride) {
+      float wj[kAhead], v[kAhead][KG];
+#pragma unroll
+      for (int a = 0; a < kAhead; ++a) {
+        wj[a] = wp[a * stride];
+#pragma unroll
+        for (int k = 0; k < KG; ++k) v[a][k] = k < mk ? vp[k * ld + a * stride] : 0.f;
+      }
+#pragma unroll
+      for (int a = 0; a < kAhead; ++a)
+#pragma unroll
+        for (int k = 0; k < KG; ++k) add(k, v[a][k], wj[a]);
+    }
+    for (; u < run; ++u, vp += stride, wp += stride)
+#pragma unroll
+      for (int k = 0; k < KG; ++k)
+        if (k < mk) add(k, vp[k * ld], wp[0]);
+#pragma unroll
+    for (int k = 0; k < KG; ++k)
+      if (k < mk) {
+        if (big[k] >= 0x1p-80f && big[k] <= 0x1p120f) {
+          acc[k] += static_cast<double>(s[k]) + static_cast<double>(c[k]);
+        } else {
+          for (int i = 0; i < run; ++i) {
+            const size_t j = j0 + i * stride;
+            const float v = V[k * ld + j], wj = w[j];
+            if (!((v == 0.f && fabsf(wj) < INFINITY) || (wj == 0.f && fabsf(v) < INFINITY)))
+              acc[k] += static_cast<double>(v) * static_cast<double>(wj);
+          }
+        }
+      }
+  }
+  block_reduce_store<KG>(acc, mk, partials, m, k0);
 }
 
 // Residual pass.  Outputs (per block): [0] ||r||^2, [1] ||t||^2, [2..2+m) V_i . t
@@ -772,10 +879,7 @@ int dispatch_k(int m, cudaStream_t st, Args... args) {
 template <typename S, int K>
 struct MultidotL {
   static void run(int g, cudaStream_t st, const S *V, size_t ld, int m, const S *w, size_t n, double *p) {
-    if constexpr (std::is_same<S, float>::value)
-      multidot_f32_kernel<K><<<wave_grid(multidot_f32_kernel<K>, f32_block<K>()), f32_block<K>(), 0, st>>>(V, ld, m, w, n, p);
-    else
-      multidot_kernel<S, K><<<g, kT, 0, st>>>(V, ld, m, w, n, p);
+    multidot_f32_kernel<K><<<wave_grid(multidot_f32_kernel<K>, f32_block<K>()), f32_block<K>(), 0, st>>>(V, ld, m, w, n, p);
   }
 };
 template <typename S, int K>
@@ -807,12 +911,6 @@ struct GsFinishMixL {
                   const S *t, S *out, double *p) {
     if constexpr (std::is_same<S, double>::value)
       gs_finish_mix_kernel<K><<<wave_grid(gs_finish_mix_kernel<K>, kT), kT, 0, st>>>(V, ld, m, c, sc, n, t, out, p);
-  }
-};
-template <typename S, int K>
-struct MultidotExactL {
-  static void run(int g, cudaStream_t st, const S *V, size_t ld, int m, const S *w, size_t n, double *p) {
-    multidot_kernel<S, K><<<g, kT, 0, st>>>(V, ld, m, w, n, p);
   }
 };
 template <typename S, int K>
@@ -948,8 +1046,17 @@ int vec_multidot(const S *V, size_t ld, int m, const S *w, size_t n, double *par
                  bool fp64_products, bool mixed) {
   if (m < 1 || m > 32) return DOCI_ERR_INVALID;
   if (mixed && std::is_same<S, double>::value) return dispatch_k<S, MultidotMixL>(m, st, V, ld, m, w, n, partials);
-  if (fp64_products) return dispatch_k<S, MultidotExactL>(m, st, V, ld, m, w, n, partials);
-  return dispatch_k<S, MultidotL>(m, st, V, ld, m, w, n, partials);
+  const int groups = (m + KG - 1) / KG;
+  if constexpr (std::is_same<S, double>::value) {
+    multidot_kernel<<<dim3(groups, grid_blocks()), kT, 0, st>>>(V, ld, m, w, n, partials);
+  } else if (fp64_products) {
+    // two rows of blocks per SM (at most grid_blocks(): the partial-sum buffers' sizes hold)
+    multidot_exact_f32_kernel<<<dim3(groups, 2 * device_sm_count()), kT, 0, st>>>(V, ld, m, w, n, partials);
+  } else {
+    return dispatch_k<S, MultidotL>(m, st, V, ld, m, w, n, partials);
+  }
+  DOCI_CUDA(cudaGetLastError());
+  return DOCI_OK;
 }
 template <typename S>
 int vec_residual(const S *V, const S *VA, size_t ld, int m, const double *y, double theta, const double *diag,
