@@ -26,6 +26,7 @@
 
 #include "internal.h"
 #include "vec.h"
+#include "warp_sums.cuh"
 
 namespace doci {
 namespace {
@@ -53,15 +54,7 @@ __device__ __forceinline__ void block_reduce_store(double (&acc)[K], int nk, dou
   __shared__ double red[32][kMaxK];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    if (k < nk) {
-      double v = acc[k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0) red[warp][k] = v;
-    }
-  }
+  warp_sums<K>(acc, red[warp]);
   __syncthreads();
   double *rows = partials + kHeader;
   const bool groups = width > 0;
