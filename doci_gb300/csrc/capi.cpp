@@ -298,26 +298,20 @@ int doci_sigma_host(doci_ham *h, const void *x, void *y, int precision) {
   void *dy = words ? const_cast<void *>(mapped_host(y)) : nullptr;
   const int kind = plan_sigma(h, precision).kind;
   const bool sched = h->d_pblocks_host && !h->host_steps.empty();
-  if (sched && ((precision == DOCI_FP32 && kind == 6 && pair_fits(h)) ||
-                (precision == DOCI_FP64 && kind == 9 && pair_ff_fits(h)))) {
-    // the pair forms overlap the copies with the sigma: pieces of x go up and
-    // pieces of y come down on the copy engines while the unit groups run (a
-    // pageable y is copied after the sigma: a copy into pageable memory can
-    // hold the calling thread until it is done)
-    const bool y_pinned = mapped_host(y) != nullptr;
-    if (precision == DOCI_FP32)
-      st = launch_pair_host(h, static_cast<const float *>(x), static_cast<float *>(h->d_stage_x),
-                            static_cast<float *>(h->d_stage_y), y_pinned ? static_cast<float *>(y) : nullptr,
-                            h->stream);
-    else
-      st = launch_pair_ff_host(h, static_cast<const double *>(x), static_cast<double *>(h->d_stage_x),
-                               static_cast<double *>(h->d_stage_y), y_pinned ? static_cast<double *>(y) : nullptr,
-                               h->stream);
+  // a large FP32 space between pinned buffers overlaps the copies with the
+  // mma.sync pair form, piece by piece (pieces of x go up and pieces of y come
+  // down on the copy engines while the unit groups run).  Measured against
+  // copy, warp-per-unit sigma, copy: 155M determinants 9.4 ms against 11.0,
+  // 601M 35.6 against 43.0; but 40M 4.4 against 2.9, and at every size in FP64
+  // (601M: 134 against 103 ms; 10M: 4.0 against 1.8) and into pageable y (601M
+  // FP32: 56 against 44 ms).
+  const bool y_pinned = mapped_host(y) != nullptr;
+  if (sched && precision == DOCI_FP32 && kind == 6 && pair_fits(h) && h->D >= (1u << 27) && y_pinned) {
+    st = launch_pair_host(h, static_cast<const float *>(x), static_cast<float *>(h->d_stage_x),
+                          static_cast<float *>(h->d_stage_y), static_cast<float *>(y), h->stream);
     if (st) return st;
-    if (y_pinned) {
-      DOCI_CUDA(cudaStreamSynchronize(h->stream));
-      return ham_device_error(h, h->stream);
-    }
+    DOCI_CUDA(cudaStreamSynchronize(h->stream));
+    return ham_device_error(h, h->stream);
   } else {
     if (dx) {
       if ((st = vec_copy(h->d_stage_x, dx, bytes, h->stream))) return st;

@@ -70,7 +70,7 @@ void ham_release(doci_ham *h) {
   cudaStream_t st = h->stream;
   void *bufs[] = {h->d_binom, h->d_Kmir64, h->d_Kmir32, h->d_tab64, h->d_diag, h->d_diag32, h->d_stage_x,
                   h->d_stage_y, h->d_rows, h->d_rowstart, h->d_pblocks, h->d_pblocks_host, h->d_kfrag, h->d_tc_err,
-                  h->d_wstart, h->d_wunits};  // d_rem/d_ins/d_ins_t/d_tab_off are shared (per-process cache)
+                  h->d_wstart, h->d_wunits, h->d_kdig};  // d_rem/d_ins/d_ins_t/d_tab_off are shared (per-process cache)
   for (void *p : bufs) release_async(p, st);
   if (h->h_diag) cudaFreeHost(h->h_diag);
   if (st) {
@@ -110,6 +110,7 @@ void ham_release(doci_ham *h) {
   h->d_pblocks = nullptr;
   h->d_kfrag = nullptr;
   h->d_wstart = h->d_wunits = nullptr;
+  h->d_kdig = nullptr;
   h->d_wtab_a = h->d_wtab_b = nullptr;
   h->wsplit = 0;
   h->d_tc_err = nullptr;

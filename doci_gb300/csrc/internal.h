@@ -106,6 +106,8 @@ struct doci_ham {
   // not fit), row starts by row-part mask and unit list (masks, four per tile)
   int wsplit = 0, nwquads = 0;
   uint32_t *d_wstart = nullptr, *d_wunits = nullptr;
+  uint16_t *d_kdig = nullptr;  // K in ten-bit digits (FP16) and their exponent
+  int kdig_exp = 0;
   const void *d_wtab_a = nullptr, *d_wtab_b = nullptr;  // insertion tables (per-process cache)
   // doci_sigma_host on the pair forms: x and sigma cross the host link in
   // pieces (chunk_off) on copy_stream while the pair units run in groups,
@@ -173,11 +175,11 @@ int launch_pair_host(doci_ham *h, const float *hx, float *dx, float *dy, float *
 int ham_build_pair_warp(doci_ham *h);
 bool pair_warp_fits(const doci_ham *h);
 int launch_pair_warp(const doci_ham *h, const float *x, float *y, cudaStream_t s);
-// FP64-accurate pair form in float-float arithmetic (sigma_pair.cu)
+// the same in FP64 accuracy (sigma_pair_warp64.cu)
+int launch_pair_warp64(const doci_ham *h, const double *x, double *y, cudaStream_t s);
+// FP64-accurate pair form in float-float arithmetic, one block per unit (sigma_pair.cu)
 bool pair_ff_fits(const doci_ham *h);
 int launch_pair_ff(const doci_ham *h, const double *x, double *y, cudaStream_t s);
-// its host-buffer form on the same piece and group schedule as launch_pair_host
-int launch_pair_ff_host(doci_ham *h, const double *hx, double *dx, double *dy, double *hy, cudaStream_t s);
 // tensor-core pair form (sigma_tc.cu), FP32 only, sm_103a; x 16-byte aligned.
 // A device wait that runs out writes a nonzero code to *d_err (spin_limit:
 // try_wait iterations per wait).

@@ -832,6 +832,15 @@ int tuned_choice(const doci_ham *h, int precision, int nv, bool allow_pair) {
   return it == g_tuned.end() ? 0 : it->second;
 }
 
+// Below this many determinants the automatic choice is the gather kernel: one
+// launch, and nothing to set up per unit.  Measured (us, gather / pair form):
+// FP32 12,870 determinants 13.0 / 16.7, 24,310 15.0 / 16.6, 48,620 16.8 / 16.8;
+// FP64 12,870 14.1 / 21.3, 24,310 20.9 / 21.4, 48,620 27.1 / 22.1; the row
+// passes are slower than both (14.8 and 23 us at the first two in FP32).
+constexpr uint32_t kGatherMaxD = 1u << 15;
+// the FP64 pair form is a candidate of the autotuning from here on
+constexpr uint32_t kTunedPairMinD = 1u << 18;
+
 // The path of kind `kind` (0 = the heuristics) for this handle; a kind that
 // does not fit falls back as described at doci_ham_set_sigma_kernel.
 SigmaPlan plan_kind(const doci_ham *h, int precision, bool allow_pair, int kind) {
@@ -840,9 +849,10 @@ SigmaPlan plan_kind(const doci_ham *h, int precision, bool allow_pair, int kind)
   if (allow_pair && precision == DOCI_FP32) {
     // tensor-core pair form with TMA-staged hole rows: on request (kind 8)
     if (kind == 8 && tc_fits(h)) return {8, tc_launches(h)};
-    // mma.sync pair form: the automatic FP32 choice where it fits and the
-    // space gives every SM blocks of work (measured fastest there)
-    const bool want_pair = kind == 6 || kind == 8 || (kind == 0 && h->npblocks >= device_sm_count());
+    // pair form: the automatic FP32 choice where it fits and the space gives
+    // every SM work
+    const bool want_pair =
+        kind == 6 || kind == 8 || (kind == 0 && h->npblocks >= device_sm_count() && h->D >= kGatherMaxD);
     if (want_pair && pair_fits(h)) return {6, 2};  // zero (or diag x) pass + pair pass
   }
   // float-float sigma (FP64 accuracy in FP32 arithmetic): the pair form, or
@@ -850,13 +860,13 @@ SigmaPlan plan_kind(const doci_ham *h, int precision, bool allow_pair, int kind)
   // conversion (with sigma = diag x for the pair form) and the pass
   if (kind == 9 && precision == DOCI_FP64 && (pair_ff_fits(h) || (h->nrows >= 1 && rowx_fits(h, sizeof(ff)))))
     return {9, 2};
-  // the automatic FP64 choice where the pair tiling gives every SM blocks of
-  // work: the float-float pair form (measured 3.2x faster than the row pass
-  // at L=32, N=16: 138.6 ms against 444.9 ms)
-  if (kind == 0 && allow_pair && precision == DOCI_FP64 && h->npblocks >= device_sm_count() && pair_ff_fits(h))
+  // the automatic FP64 choice where the pair tiling gives every SM work: the
+  // FP64-accurate pair form (L=32, N=16: 53.7 ms; the row pass 444.9 ms)
+  if (kind == 0 && allow_pair && precision == DOCI_FP64 && h->npblocks >= device_sm_count() &&
+      h->D >= kGatherMaxD && pair_ff_fits(h))
     return {9, 2};
   // row kernel when the row tiling exists, fits, and gives every SM work
-  bool row = kind >= 3 || (kind == 0 && h->nrows >= device_sm_count());
+  bool row = kind >= 3 || (kind == 0 && h->nrows >= device_sm_count() && h->D >= kGatherMaxD);
   if (row && !row_kernel_fits(h, elem)) row = false;
   if (!row) return {1, 1};
   // automatic: the phase-ordered pass for FP64 (measured faster there), the
@@ -910,6 +920,9 @@ int launch_sigma(const doci_ham *h, const void *x, void *y, int precision, cudaS
       return f64 ? launch_rowx<double>(h, x, y, st, 1) : launch_rowx<float>(h, x, y, st, 1);
     case 9:
       // the pair form where it fits, else the phase-ordered row pass, both in float-float
+      // from 10 orbitals on the warp-per-unit form
+      if (pair_warp_fits(h))
+        return launch_pair_warp64(h, static_cast<const double *>(x), static_cast<double *>(y), st);
       if (pair_ff_fits(h)) return launch_pair_ff(h, static_cast<const double *>(x), static_cast<double *>(y), st);
       return launch_rowx_ff(h, static_cast<const double *>(x), static_cast<double *>(y), st);
     default:  // 3
@@ -1011,7 +1024,10 @@ int autotune_sigma(doci_ham *h, int precision, int nv, cudaStream_t st, int *cho
       int pick = 0;
       for (int kind : {1, 3, 4, 6, 8, 9}) {
         if ((kind == 6 || kind == 8) && (!allow || precision != DOCI_FP32)) continue;
-        if (kind == 9 && precision != DOCI_FP64) continue;
+        // small tuned FP64 shapes keep to the kernels without atomic adds, whose
+        // results repeat bit for bit (they were the fastest there before kind 9
+        // ran on the tensor cores: 184,756 determinants, 60 us against 38 now)
+        if (kind == 9 && (precision != DOCI_FP64 || h->D < kTunedPairMinD)) continue;
         hm->sigma_kernel = kind;
         const SigmaPlan p = plan_sigma(h, precision, allow != 0);
         if (p.kind != kind) continue;  // the path does not fit this shape

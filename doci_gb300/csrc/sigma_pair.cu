@@ -1,7 +1,9 @@
-// sigma_pair.cu -- FP32 sigma in the (N-1)-pair intermediate form on the
-// warp-level mma.sync path (kind 6, the automatic FP32 choice once the
-// tiling gives every SM a unit), and the FP64-accurate float-float version
-// of the same form (kind 9).  The tcgen05 version of the FP32 form is
+// sigma_pair.cu -- the (N-1)-pair intermediate form with one block per unit:
+// FP32 on the warp-level mma.sync path (below 10 orbitals, and in
+// doci_sigma_host on large spaces, where its units run in groups between the
+// pieces of the copies) and FP64-accurate in float pairs (below 10 orbitals).
+// From 10 orbitals on kinds 6 and 9 run sigma_pair_warp.cu and
+// sigma_pair_warp64.cu; the tcgen05 version with one block per unit is
 // sigma_tc.cu (kind 8).
 //
 // Every off-diagonal element of the DOCI Hamiltonian is a pair hop
@@ -515,42 +517,6 @@ unsigned init_grid(uint64_t n) {
   return static_cast<unsigned>(std::min((n + 255) / 256, cap));
 }
 
-template <int NO>
-int launch_pair_ff_host_no(doci_ham *h, const double *hx, double *dx, double *dy, double *hy, cudaStream_t st) {
-  int per_sm = 1;
-  int r = kernel_blocks(reinterpret_cast<const void *>(sigma_pair_ff_kernel<NO>), kPairThreads, 0, &per_sm);
-  if (r != DOCI_OK) return r;
-  const int slots = device_sm_count() * per_sm;
-  ff *xf = nullptr;
-  DOCI_CUDA(cudaMallocAsync(&xf, sizeof(ff) * static_cast<size_t>(h->D), st));
-  const uint2 *blocks = reinterpret_cast<const uint2 *>(h->d_pblocks_host);
-  r = run_host_schedule<double>(
-      h, hx, dx, dy, hy, st,
-      [&](uint64_t a, uint64_t n, cudaStream_t s) {
-        pair_init64_kernel<<<init_grid(n), 256, 0, s>>>(static_cast<uint32_t>(n), h->d_diag + a, dx + a, dy + a,
-                                                         xf + a);
-        DOCI_CUDA(cudaGetLastError());
-        return static_cast<int>(DOCI_OK);
-      },
-      [&](int first, int count, cudaStream_t s) {
-        const PairShape ps{h->D, h->L, h->N, h->split, h->L - h->split, count};
-        sigma_pair_ff_kernel<NO><<<std::min(slots, count), kPairThreads, 0, s>>>(
-            ps, blocks + first, h->d_rowstart, h->d_binom, h->d_Kmir64, h->d_ins_t, h->d_tab_off, xf, dy);
-        DOCI_CUDA(cudaGetLastError());
-        return static_cast<int>(DOCI_OK);
-      });
-  // the side stream's groups read xf: st is ordered after them (the
-  // schedule's own join is skipped when it returns early with an error)
-  if (r != DOCI_OK && h->side_stream) {
-    cudaEventRecord(h->side_ev, h->side_stream);
-    cudaStreamWaitEvent(st, h->side_ev, 0);
-  }
-  const cudaError_t ef = cudaFreeAsync(xf, st);
-  if (r != DOCI_OK) return r;
-  DOCI_CUDA(ef);
-  return DOCI_OK;
-}
-
 }  // namespace
 
 int launch_pair_host(doci_ham *h, const float *hx, float *dx, float *dy, float *hy, cudaStream_t st) {
@@ -575,15 +541,6 @@ int launch_pair_host(doci_ham *h, const float *hx, float *dx, float *dy, float *
         DOCI_CUDA(cudaGetLastError());
         return static_cast<int>(DOCI_OK);
       });
-}
-
-int launch_pair_ff_host(doci_ham *h, const double *hx, double *dx, double *dy, double *hy, cudaStream_t st) {
-  if (!pair_ff_fits(h) || !h->d_pblocks_host || h->host_steps.empty()) return DOCI_ERR_INVALID;
-  const int no = h->L - h->N + 1;
-  if (no <= 8) return launch_pair_ff_host_no<8>(h, hx, dx, dy, hy, st);
-  if (no <= 17) return launch_pair_ff_host_no<17>(h, hx, dx, dy, hy, st);
-  if (no <= 24) return launch_pair_ff_host_no<24>(h, hx, dx, dy, hy, st);
-  return launch_pair_ff_host_no<32>(h, hx, dx, dy, hy, st);
 }
 
 bool pair_ff_fits(const doci_ham *h) { return pair_fits(h) && h->L - h->N + 1 <= 32; }

@@ -40,7 +40,9 @@
 
 #include "addressing.cuh"
 #include "internal.h"
+#include "pair_warp.h"
 #include "pair_warp_index.cuh"
+#include "tcgen.cuh"
 
 namespace doci {
 namespace {
@@ -57,105 +59,16 @@ constexpr int kOffStart = kOffBar + 128;    // row starts of a warp's hole rows,
 constexpr int kOffRows = kOffStart + 4 * 24 * (kThreads / 32);
 constexpr size_t kMinSmem = 120 * 1024;     // one block per SM: it allocates all of the tensor memory
 
-struct PwShape {
-  uint32_t D;
-  int L, N, na, nquads;
-  long spin_limit;
-  uint32_t n[16];    // C(P, j), 0 from j = P + 1
-  uint32_t off[16];  // first set of j elements in the tables
-};
-
-__device__ __forceinline__ uint32_t su32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ float lds(uint32_t a) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ void sts(uint32_t a, float v) {
-  asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
-  return v;
-}
-// *p where on, else 0; *p += v where on (predicated: `on` is the same in the whole warp or the lane is idle)
-__device__ __forceinline__ float ldg_if(const float *p, uint32_t on) {
-  float v;
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}\n"
-      : "=&f"(v)
-      : "l"(p), "r"(on));
-  return v;
-}
-__device__ __forceinline__ void red_if(float *p, float v, uint32_t on) {
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q red.global.add.f32 [%0], %1;\n\t}\n" ::"l"(p), "f"(v),
-               "r"(on)
-               : "memory");
-}
-// (a0, a1) + (b0, b1) and - in one instruction (FP32, round to nearest)
-__device__ __forceinline__ void add2(float &a0, float &a1, float b0, float b1) {
-  asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\tadd.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, "
-      "p;\n\t}\n"
-      : "+f"(a0), "+f"(a1)
-      : "f"(b0), "f"(b1));
-}
-__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(ok)
-      : "r"(a), "r"(parity), "r"(1000u)
-      : "memory");
-  return ok != 0;
-}
-// the four warps of a warpgroup meet; true when any of them failed
-__device__ __forceinline__ bool group_meet(int wg, bool fail) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, "
-      "q;\n\t}\n"
-      : "=r"(r)
-      : "r"(static_cast<uint32_t>(fail)), "r"(wg + 1)
-      : "memory");
-  return r != 0;
-}
-__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-  // K-major, 128-byte swizzle: leading offset unused (16 B), 8-row groups 1024 B apart, version 1
-  return static_cast<uint64_t>((addr >> 4) & 0x3FFFu) | (static_cast<uint64_t>(1) << 16) |
-         (static_cast<uint64_t>(1024 >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
-         (static_cast<uint64_t>(2) << 61);
-}
 __device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t id, uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d),
       "r"(a), "l"(b), "r"(id), "r"(acc));
 }
-__device__ __forceinline__ void tld16(uint32_t t, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(t));
-}
-__device__ __forceinline__ void tst16(uint32_t t, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(t),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
 // nearest TF32 (10-bit mantissa), ties away from zero: half a TF32 ulp added to
 // the magnitude, the low 13 bits cut (two integer instructions; cvt.rna.tf32
 // measured about five)
 __device__ __forceinline__ uint32_t tf32_rna(float f) { return (__float_as_uint(f) + 0x1000u) & 0xffffe000u; }
-// byte offset of element (row r, column k) of a 128-byte-swizzled K-major tile of 32 FP32 per row
-__host__ __device__ __forceinline__ uint32_t sw128(uint32_t r, uint32_t k) {
-  return (r >> 3) * 1024u + (r & 7u) * 128u + ((((k >> 2) ^ r) & 7u) << 4) + (k & 3u) * 4u;
-}
 
 template <int P>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -470,14 +383,14 @@ int ham_build_pair_warp(doci_ham *h) {
   PwTables t;
   const int r = pw_tables(h->device, P, &t);
   if (r != DOCI_OK) return r;
+  if (const int k = ham_build_kdigits(h)) return k;
   h->d_wtab_a = t.a;
   h->d_wtab_b = t.b;
   h->wsplit = P;
   return DOCI_OK;
 }
 
-int launch_pair_warp(const doci_ham *h, const float *x, float *y, cudaStream_t st) {
-  if (!pair_warp_fits(h)) return DOCI_ERR_INVALID;
+PwShape pair_warp_shape(const doci_ham *h) {
   const int P = h->wsplit;
   PwShape s{};
   s.D = h->D;
@@ -492,11 +405,17 @@ int launch_pair_warp(const doci_ham *h, const float *x, float *y, cudaStream_t s
     s.off[j] = at;
     at += pw::padded(s.n[j]);
   }
+  return s;
+}
+
+int launch_pair_warp(const doci_ham *h, const float *x, float *y, cudaStream_t st) {
+  if (!pair_warp_fits(h)) return DOCI_ERR_INVALID;
+  const PwShape s = pair_warp_shape(h);
   zero_kernel<<<static_cast<unsigned>(std::min<uint64_t>((h->D / 4 + 256) / 256, 8ull * device_sm_count())), 256, 0,
                 st>>>(y, h->D);
   DOCI_CUDA(cudaGetLastError());
-  if (P == 12) return launch_p<12>(h, s, x, y, st);
-  if (P == 10) return launch_p<10>(h, s, x, y, st);
+  if (h->wsplit == 12) return launch_p<12>(h, s, x, y, st);
+  if (h->wsplit == 10) return launch_p<10>(h, s, x, y, st);
   return launch_p<8>(h, s, x, y, st);
 }
 

@@ -170,27 +170,29 @@ int doci_sigma(doci_ham *ham, const void *d_x, void *d_y, int precision, void *s
 int doci_sigma_block(doci_ham *ham, const void *d_X, int64_t ldx, void *d_Y, int64_t ldy, int nv, int precision,
                      void *stream);
 
-/* Sigma kernel selection for a handle: 0 automatic (default: with a row
- * tiling that gives every SM work, kind 6 for FP32 and kind 9 for FP64; else
- * with a row tiling kind 3 for FP32 and kind 4 for FP64; else kind 1),
+/* Sigma kernel selection for a handle: 0 automatic (default: from 2^15
+ * determinants on, with a row tiling that gives every SM work, kind 6 for
+ * FP32 and kind 9 for FP64, or where these do not apply kind 3 for FP32 and
+ * kind 4 for FP64; else kind 1),
  * 1 the per-determinant gather kernel, 3 the row pass doing all hops, 4 the
  * phase-ordered row pass (cross hops staged one source row at a time), 6 the
- * (N-1)-pair form with one warp per group of sets (FP32 only: gather the
- * neighbours of every (N-1)-pair set, multiply by K on the tensor cores,
- * scatter, atomic adds between groups; below 10 orbitals and in
- * doci_sigma_host the product runs on mma.sync), 8 the (N-1)-pair form on the 5th-generation tensor cores (FP32
- * only: the own row of a set's row part staged in shared memory, the other
- * rows streamed by TMA, the product in TMEM, each own row written once;
- * needs a 16-byte aligned x, else kind 6 runs), 9 the (N-1)-pair form in
- * float-float arithmetic (FP64 only: FP64 accuracy from pairs of FP32
- * values on the FP32 units, x converted once per call into stream-ordered
- * scratch of D x 8 bytes, FP64 atomic adds into sigma; the phase-ordered row
- * pass in the same arithmetic where the pair tiling does not fit; FP32
+ * (N-1)-pair form (FP32 only: gather the neighbours of every (N-1)-pair set,
+ * multiply by K on the tensor cores, scatter; from 10 orbitals on one warp per
+ * group of sets, below and in doci_sigma_host on large spaces one block per
+ * group), 8 the (N-1)-pair form with one block per group on the 5th-generation
+ * tensor cores (FP32 only: the own row of a set's row part staged in shared
+ * memory, the other rows streamed by TMA, the product in TMEM, each own row
+ * written once; needs a 16-byte aligned x, else kind 6 runs), 9 the
+ * (N-1)-pair form in FP64 accuracy (FP64 only: x as pairs of FP32 values in
+ * stream-ordered scratch of D x 8 bytes, converted once per call, the products
+ * exact in digits on the tensor cores, or below 10 orbitals in float pairs on
+ * the FP32 units, FP64 atomic adds into sigma; the phase-ordered row
+ * pass in float pairs where the pair tiling does not fit; FP32
  * requests for it use the automatic choice).  Kinds 6, 8 and 9 reduce into
  * sigma with atomic adds, so their last bits vary between runs; FP64
- * requests for them use the automatic choice.  3-9 fall back to 1 when the
+ * requests for 6 and 8 use the automatic choice.  3-9 fall back to 1 when the
  * handle has no row tiling.  Other values: DOCI_ERR_INVALID.  A device wait
- * of kind 6 or 8 that runs out (it never should) is reported as
+ * of kind 6, 8 or 9 that runs out (it never should) is reported as
  * DOCI_ERR_DEVICE_TIMEOUT by the handle's next synchronous call
  * (doci_sigma_host, doci_solve).  For tests and tuning. */
 int doci_ham_set_sigma_kernel(doci_ham *ham, int kind);
@@ -202,7 +204,8 @@ int doci_ham_set_sigma_kernel(doci_ham *ham, int kind);
  * pair form allowed) and the pair-free path of the block solves; nvec = 2..4
  * tunes the block sigma of nvec vectors (doci_sigma_block, doci_solve_roots
  * with that many roots; *choice = 1 row pass in groups, 2 gather, 3 one
- * vector at a time).  Synchronous; a few sigma calls per candidate.  The
+ * vector at a time).  FP64 shapes below 2^18 determinants keep to the paths
+ * without atomic adds (kinds 1, 3, 4).  Synchronous; a few sigma calls per candidate.  The
  * choices change which kernels run, so results computed before and after a
  * tuning may differ in their last bits; tune before a batch whose results
  * are compared to single solves.  No counterpart in the reference. */
@@ -213,13 +216,13 @@ int doci_ham_autotune(doci_ham *ham, int precision, int nvec, int *choice);
  * *launches, the number of kernel launches of one call.  Host-only query. */
 int doci_sigma_plan(const doci_ham *ham, int precision, int *kind, int *launches);
 
-/* Same on host buffers; copies in and out inside the call, synchronous.  On
- * the pair forms (kinds 6 and 9) x is uploaded, and a pinned (page-locked) y
- * downloaded, in pieces on the handle's own copy stream, overlapped with the
- * sigma (whose unit groups alternate between the handle's stream and a
- * second stream of its own).  The staging buffers and these streams belong
- * to the handle: calls on one handle from several host threads must be
- * serialised by the caller. */
+/* Same on host buffers; copies in and out inside the call, synchronous.  In
+ * FP32 from 2^27 determinants on (kind 6), with a pinned (page-locked) y, x is
+ * uploaded and y downloaded in pieces on the handle's own copy stream,
+ * overlapped with the sigma (whose unit groups alternate between the handle's
+ * stream and a second stream of its own); else copy, sigma, copy in turn.  The
+ * staging buffers and these streams belong to the handle: calls on one handle
+ * from several host threads must be serialised by the caller. */
 int doci_sigma_host(doci_ham *ham, const void *x, void *y, int precision);
 
 /* Lexical addressing on the device: bitstrings of determinants

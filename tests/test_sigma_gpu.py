@@ -399,3 +399,58 @@ def test_sigma_pair_warp_edges(L, N, seed, off, synth, dg):
         y = ys.double().cpu().numpy()
         assert np.abs(y[off:off + D] - yr).max() <= TOL32 * np.abs(yr).max()
         assert np.isnan(y[:off]).all() and np.isnan(y[off + D:]).all()
+
+
+@pytest.mark.parametrize("L,N,seed", [
+    (10, 1, 91), (10, 5, 92), (11, 10, 93), (13, 13, 94), (32, 2, 95), (32, 30, 96),  # 8 column orbitals
+    (22, 8, 97), (24, 20, 98),  # 10
+    (28, 6, 99), (26, 19, 100),  # 12
+])
+def test_sigma_fp64_warp_edges(L, N, seed, synth, dg):
+    """The FP64-accurate pair form on each of its tilings, with values over
+    many orders of magnitude: random vectors, one-hot, all equal, falling off
+    over 2^-60, and small and large overall scales, each against the oracle's
+    matvec of the same vector within 1e-12 of its largest element."""
+    torch = torch_cuda()
+    p = synth(L, N, seed)
+    o = oracle.Ham(p)
+    rng = np.random.default_rng(seed)
+    with dg.Hamiltonian.from_fcidump(p) as h:
+        h.set_sigma_kernel("rowff")
+        assert h.sigma_plan(dg.FP64) == (9, 2)
+        D = h.D
+        base = rng.standard_normal(D)
+        hot = np.zeros(D)
+        hot[D // 2] = -3.0
+        vecs = [base, hot, np.ones(D), np.full(D, 1 / 3), base * np.exp2(-60 * rng.random(D)), base * 1e-20,
+                base * 1e25, np.where(rng.random(D) < 0.5, 1.0, -1.0)]
+        y = torch.empty(D, dtype=torch.float64, device="cuda")
+        for i, x in enumerate(vecs):
+            xd = torch.from_numpy(x).cuda()
+            y.fill_(float("nan"))
+            h.sigma_device(xd.data_ptr(), y.data_ptr(), dg.FP64)
+            torch.cuda.synchronize()
+            ref = o.matvec(x)
+            assert np.abs(y.cpu().numpy() - ref).max() <= TOL64 * np.abs(ref).max(), i
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("prec_name,kernel", [("FP32", "pair"), ("FP64", "rowff")])
+@pytest.mark.parametrize("L,N,seed", [(12, 6, 101), (22, 8, 102)])
+def test_sigma_pair_warp_nonfinite(L, N, seed, prec_name, kernel, bad, synth, dg):
+    """An infinity or a NaN in x reaches the same elements of sigma (its own and
+    its neighbours') as in the gather kernel, and no others."""
+    torch = torch_cuda()
+    prec = getattr(dg, prec_name)
+    tdt = torch.float64 if prec == dg.FP64 else torch.float32
+    with dg.Hamiltonian.from_fcidump(synth(L, N, seed)) as h:
+        x = torch.randn(h.D, dtype=tdt, device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed))
+        x[h.D // 3] = bad
+        out = []
+        for k in ("gather", kernel):
+            h.set_sigma_kernel(k)
+            y = torch.empty_like(x)
+            h.sigma_device(x.data_ptr(), y.data_ptr(), prec)
+            torch.cuda.synchronize()
+            out.append(torch.isfinite(y))
+        assert torch.equal(out[0], out[1]) and int((~out[0]).sum()) == N * (L - N) + 1
