@@ -3,34 +3,42 @@
 // Y_S = X_S K), one warp per unit, the product with K on the 5th-generation
 // tensor cores.  This is what kind 6 runs from 10 orbitals on.
 //
-// A warp walks the sets of one unit (pair_warp_index.cuh), 32 at a time, one
-// set per lane, which is also the set's lane in tensor memory.  The unit's own
-// row, at most C(12,6) = 924 elements, has its x and its sums in shared memory
-// private to the warp: the random accesses of the column orbitals stay on
-// chip, and since S -> S u o is one to one the sums are plain
-// read-modify-writes, one orbital after the other, with no atomics.  The rows
-// of the row-part holes are read and added to at the set's own column, 32
-// consecutive elements at a time.  The orbital axis is not compacted, so K
-// (high and low TF32 parts, 64 x 32, the B operand) is the same for every unit
-// and four warps with units of their own share one 128-row MMA tile.
+// A unit (pair_warp_index.cuh) belongs to two warps, which walk its sets 32 at
+// a time, one set per lane, which is also the set's lane in tensor memory: one
+// gathers a set's values and splits them into the A operand, the other reads
+// the product back and scatters it, while the first is at the next 32 sets.
+// The unit's own row, at most C(12,6) = 924 elements, is private to them in
+// shared memory, its x with the one and its sums with the other: the random
+// accesses of the column orbitals stay on chip, and since S -> S u o is one to
+// one the sums are plain read-modify-writes, one orbital after the other, with
+// no atomics.  The rows of the row-part holes are read and added to at the
+// set's own column, 32 consecutive elements at a time.  The orbital axis is
+// not compacted, so K (high and low TF32 parts, 64 x 32, the B operand) is the
+// same for every unit and four warps with units of their own share one
+// 128-row MMA tile; tensor memory holds four tiles.
 //
 // TF32 three ways (x high x K high, x high x K low, x low x K high): the first
 // two as one MMA of 64 columns, since an MMA of 128 rows takes the same 51
 // cycles for 32 and for 64 columns on GB300 (24.6 ns in a run of 96; 72 cycles
 // at 128 columns).  The two halves are added when they are read back.
 //
-// Column orbitals: 12 as long as that leaves four units per resident warp,
-// else 10 as long as each has one, else 8.  Larger rows mean fewer set-ups
-// and fewer row-part orbitals to look at, smaller ones more units to spread.
-// Measured (us, 12 / 10 / 8): L=32 N=16 19,120 / 22,940 / 38,470;
-// L=26 N=13 347 / 362 / 562; L=24 N=12 107 / 103 / 138;
-// L=22 N=11 70 / 38 / 46; L=21 N=9 70 / 27.6 / 25.1; L=18 N=9 69 / 27 / 16.8.
+// Column orbitals: 12 as long as that leaves four units per tile row in
+// flight, else 10 as long as each has one, else 8.  Larger rows mean fewer
+// set-ups and fewer row-part orbitals to look at, smaller ones more units to
+// spread.  Measured with one warp doing both jobs (us, 12 / 10 / 8): L=32 N=16
+// 19,120 / 22,940 / 38,470; L=26 N=13 347 / 362 / 562; L=24 N=12
+// 107 / 103 / 138; L=22 N=11 70 / 38 / 46; L=21 N=9 70 / 27.6 / 25.1;
+// L=18 N=9 69 / 27 / 16.8.
 //
 // Measured against the one-block-per-unit mma.sync kernel of sigma_pair.cu:
-// L=32 N=16 33.9 -> 19.1 ms, L=28 N=14 1.82 -> 1.23 ms, L=27 N=11 524 -> 331 us,
-// L=20 N=10 28.0 -> 20.9 us.  Bound by instruction issue and the latency of the
-// hole rows (about 600 warp instructions per 32 sets; 16 warps per SM by the
-// 128 tensor-memory columns of a tile).
+// L=32 N=16 33.9 -> 16.9 ms (one warp for both jobs 19.1), L=28 N=14 1.82 ->
+// 1.11 ms (1.23), L=27 N=11 524 -> 303 us (331), L=20 N=10 28.0 -> 20.4 us
+// (20.9).  Bound by instruction issue (65 % of the slots, 690 warp instructions
+// per 32 sets), the shared-memory pipe (60 %) and the latency of the hole rows.
+// Two sets per lane, two tiles per warp pair: fewer instructions (628), but
+// half the warps, 1.33 ms at L=28; only the live row-part orbitals, at
+// tensor-memory columns known at run time: 1.77 ms (their addresses go
+// through uniform registers one by one).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -47,9 +55,9 @@
 namespace doci {
 namespace {
 
-constexpr int kWgs = 4;                     // warpgroups: tiles in flight
-constexpr int kThreads = 128 * kWgs;
-constexpr uint32_t kTmemCols = 512;         // per warpgroup: A high 32 | A low 32 | D 64
+constexpr int kSlots = 4;                   // tiles in flight
+constexpr int kThreads = 2 * 128 * kSlots;  // a gathering and a scattering warpgroup per tile
+constexpr uint32_t kTmemCols = 512;         // per tile: A high 32 | A low 32 | D 64
 // tcgen05 instruction descriptor: D FP32, A and B TF32, both K-major, M = 128
 __host__ __device__ constexpr uint32_t idesc(uint32_t n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
@@ -80,27 +88,33 @@ sigma_pair_warp_kernel(const __grid_constant__ PwShape s, const uint32_t *__rest
   constexpr int NR = 32 - P;
   constexpr int XC = pw::cells(P);
   extern __shared__ __align__(1024) uint8_t sm[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = warp >> 2, w4 = warp & 3;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, slot = (warp >> 2) & (kSlots - 1), w4 = warp & 3;
+  const bool gatherer = warp < 4 * kSlots;
   const uint32_t base = su32(sm);
   if (base & 1023u) {  // the swizzled K tile needs a 1024-byte aligned base
     if (tid == 0) atomicCAS(err, 0, 3);
     return;
   }
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + kOffBar + 64);
-  const uint32_t bar = base + kOffBar + 8 * wg;
-  float *xo = reinterpret_cast<float *>(sm + kOffRows) + warp * 2 * XC, *yo = xo + XC;
-  const uint32_t xa = su32(xo), ra = base + kOffStart + warp * 96;
+  const uint32_t bar_done = base + kOffBar + 8 * slot, bar_free = bar_done + 8 * kSlots;
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + kOffBar + 16 * kSlots) + slot;
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + kOffBar + 20 * kSlots);
+  // the own row's x (gathering warps) or sums (scattering warps)
+  float *cells = reinterpret_cast<float *>(sm + kOffRows) + warp * XC;
+  const uint32_t ca = su32(cells), ra = base + kOffStart + warp * 96;
 
   for (int e = tid; e < 64 * 32; e += kThreads) {
     const int r = e >> 5, k = e & 31;
     *reinterpret_cast<float *>(sm + sw128(r, k)) = g_ksplit[(r >> 5) * 1024 + (r & 31) * 32 + k];
   }
   if (tid == 0) {
-    for (int i = 0; i < kWgs; ++i)
+    for (int i = 0; i < kSlots; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(base + kOffBar + 8 * i));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(base + kOffBar + 8 * (kSlots + i)));
+      reinterpret_cast<volatile int *>(sm + kOffBar + 16 * kSlots)[i] = 0;
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (lane == 0) xo[XC - 1] = 0.f;
+  if (lane == 0) cells[XC - 1] = 0.f;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tslot)),
                  "r"(kTmemCols));
@@ -111,13 +125,12 @@ sigma_pair_warp_kernel(const __grid_constant__ PwShape s, const uint32_t *__rest
   __syncthreads();
   fence_after();
   const uint32_t tmem = *tslot;
-  const uint32_t tg = tmem + 128u * wg, tw = tg + (static_cast<uint32_t>(32 * w4) << 16);
+  const uint32_t tg = tmem + 128u * slot, tw = tg + (static_cast<uint32_t>(32 * w4) << 16);
   const int nks = (s.L + 7) >> 3;  // >= 2 (L >= 10)
-  const uint64_t desc = smem_desc(base);
 
-  uint32_t waited = 0, issued = 0;
-  bool fail = false, stop = false;
-  for (int q = blockIdx.x * kWgs + wg; q < s.nquads && !stop; q += gridDim.x * kWgs) {
+  uint32_t n = 0;  // tiles of this slot so far
+  bool ok = true, fail = false;
+  for (int q = blockIdx.x * kSlots + slot; q < s.nquads && ok; q += gridDim.x * kSlots) {
     const uint32_t mask = units[4 * q + w4];
     const int jp = s.N - 1 - __popc(units[4 * q]);
     const uint32_t n_s = jp >= 0 ? s.n[jp] : 0u;
@@ -125,26 +138,23 @@ sigma_pair_warp_kernel(const __grid_constant__ PwShape s, const uint32_t *__rest
     const uint32_t n_own = real ? s.n[jp + 1] : 0u;
     const uint32_t holes = real ? ~mask & ((1u << s.na) - 1u) : 0u;
     const uint32_t own = n_own ? rowstart[mask] : 0u;
-    for (uint32_t c = lane; c < n_own; c += 32) {
-      xo[c] = __ldg(x + own + c);
-      yo[c] = 0.f;
-    }
+    for (uint32_t c = lane; c < n_own; c += 32) cells[c] = gatherer ? __ldg(x + own + c) : 0.f;
     // (a unit without sets has no hole rows either)
     if (lane < 24) {
       const bool hole = n_s && ((holes >> lane) & 1u);
       reinterpret_cast<uint32_t *>(sm + kOffStart)[warp * 24 + lane] = hole ? rowstart[mask | (1u << lane)] : 0u;
     }
     __syncwarp();
-    if (n_s) {
-      const uint4 *ta = tab_a + s.off[jp];
-      const uint2 *tb = tab_b + s.off[jp];
-      float v[32];
-      uint32_t at[P];  // this set's own-row cells (shared-memory addresses)
-      const uint32_t last = n_s - 1;
-      // the set's 32 values by orbital: column orbitals from the own row (the
-      // zero cell where the orbital is in the set), row-part holes from their
-      // rows (the table ends each set size with a full warp of zero cells)
-      auto gather = [&](uint32_t c0) {
+    const uint4 *ta = tab_a + (n_s ? s.off[jp] : 0u) + lane;
+    const uint2 *tb = tab_b + (n_s ? s.off[jp] : 0u) + lane;
+    const uint32_t last = n_s - 1;
+
+    if (gatherer) {
+      for (uint32_t c0 = 0; c0 < n_s; c0 += 32, ++n) {
+        // the set's 32 values by orbital: row-part holes from their rows, column
+        // orbitals from the own row (the zero cell where the orbital is in the
+        // set; the table ends each set size with a full warp of zero cells)
+        float v[32];
         const float *xl = x + min(c0 + lane, last);
 #pragma unroll
         for (int b = 0; b < NR; b += 4) {
@@ -155,102 +165,78 @@ sigma_pair_warp_kernel(const __grid_constant__ PwShape s, const uint32_t *__rest
           if (b + 3 < NR) v[P + b + 3] = ldg_if(xl + r.w, holes & (1u << (b + 3)));
         }
         uint32_t w[6];
-        const uint4 ea = __ldg(ta + c0 + lane);
-        w[0] = ea.x;
-        w[1] = ea.y;
-        w[2] = ea.z;
-        w[3] = ea.w;
+        const uint4 ea = __ldg(ta + c0);
+        w[0] = ea.x, w[1] = ea.y, w[2] = ea.z, w[3] = ea.w;
         if (P > 8) {
-          const uint2 eb = __ldg(tb + c0 + lane);
-          w[4] = eb.x;
-          w[5] = eb.y;
+          const uint2 eb = __ldg(tb + c0);
+          w[4] = eb.x, w[5] = eb.y;
         }
 #pragma unroll
-        for (int o = 0; o < P; ++o) {
-          at[o] = xa + (o & 1 ? w[o >> 1] >> 16 : w[o >> 1] & 0xffffu);
-          v[o] = lds(at[o]);
-        }
-      };
-      // v split into TF32 high and low parts in this lane's row of the tile
-      auto store = [&]() {
+        for (int o = 0; o < P; ++o) v[o] = lds(ca + (o & 1 ? w[o >> 1] >> 16 : w[o >> 1] & 0xffffu));
+        if (n > 0 && !warp_wait(bar_done, (n - 1) & 1u, s.spin_limit, abort_flag, err, 21)) fail = true;
+        fence_after();
+        // split into TF32 high and low parts in this lane's row of the tile
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t r[16];
+        for (int h = 0; h < 4; ++h) {
+          uint32_t r[8];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) r[i] = tf32_rna(v[16 * h + i]);
-          tst16(tw + 16 * h, r);
+          for (int i = 0; i < 8; ++i) r[i] = tf32_rna(v[8 * h + i]);
+          tst8(tw + 8 * h, r);
 #pragma unroll
-          for (int i = 0; i < 16; i += 2) {
-            float a0 = v[16 * h + i], a1 = v[16 * h + i + 1];
-            add2(a0, a1, -__uint_as_float(r[i]), -__uint_as_float(r[i + 1]));
-            r[i] = __float_as_uint(a0);
-            r[i + 1] = __float_as_uint(a1);
-          }
-          tst16(tw + 32 + 16 * h, r);
+          for (int i = 0; i < 8; ++i) r[i] = __float_as_uint(v[8 * h + i] - __uint_as_float(r[i]));
+          tst8(tw + 32 + 8 * h, r);
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      };
-      auto issue = [&]() {
-        if (w4 == 0 && lane == 0) {
-          fence_after();
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            if (ks < 2 || ks < nks) mma_ts(tg + 64, tg + 8 * ks, desc + 2 * ks, idesc(64), ks > 0);
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            if (ks < 2 || ks < nks) mma_ts(tg + 64, tg + 32 + 8 * ks, desc + 2 * ks, idesc(32), 1);
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                       : "memory");
-        }
-        ++issued;
-        __syncwarp();
-      };
-      gather(0);
-      store();
-      fence_before();
-      stop = group_meet(wg, fail);
-      if (!stop) issue();
-      for (uint32_t c0 = 0; c0 < n_s && !stop; c0 += 32) {
-        const bool more = c0 + 32 < n_s;
-        uint32_t cur[P];
-#pragma unroll
-        for (int o = 0; o < P; ++o) cur[o] = at[o];
-        if (more) gather(c0 + 32);
-        bool done = false;
-        for (long k = 0; k < s.spin_limit && !done; ++k) done = mbar_try(bar, waited & 1u);
-        done = __all_sync(0xffffffffu, done);
-        ++waited;
-        if (!done) {
-          fail = true;
-          if (lane == 0) atomicCAS(err, 0, 21);
-        }
-        fence_after();
-        if (more) store();
-        float yv[32];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t r[16], l[16];
-          tld16(tw + 64 + 16 * h, r);
-          tld16(tw + 96 + 16 * h, l);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int i = 0; i < 16; i += 2) {
-            yv[16 * h + i] = __uint_as_float(r[i]);
-            yv[16 * h + i + 1] = __uint_as_float(r[i + 1]);
-            add2(yv[16 * h + i], yv[16 * h + i + 1], __uint_as_float(l[i]), __uint_as_float(l[i + 1]));
-          }
-        }
         fence_before();
-        stop = group_meet(wg, fail);
-        if (stop) break;
-        if (more) issue();
-        // own row: one orbital at a time no two sets meet (S -> S u o is one to
-        // one), and the warp alone adds to it
+        if (group_meet(slot, fail)) {
+          ok = false;
+          break;
+        }
+        if (w4 == 0) {
+          // the sums of the tile before have to be read
+          if (n > 0 && !warp_wait(bar_free, (n - 1) & 1u, s.spin_limit, abort_flag, err, 22)) fail = true;
+          if (!fail && lane == 0) {
+            fence_after();
+            const uint64_t desc = smem_desc(base);
 #pragma unroll
-        for (int o = 0; o < P; ++o) {
-          sts(cur[o] + 4 * XC, lds(cur[o] + 4 * XC) + yv[o]);
+            for (int ks = 0; ks < 4; ++ks)
+              if (ks < 2 || ks < nks) mma_ts(tg + 64, tg + 8 * ks, desc + 2 * ks, idesc(64), ks > 0);
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks)
+              if (ks < 2 || ks < nks) mma_ts(tg + 64, tg + 32 + 8 * ks, desc + 2 * ks, idesc(32), 1);
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_done)
+                         : "memory");
+          }
           __syncwarp();
         }
+      }
+    } else {
+      for (uint32_t c0 = 0; c0 < n_s; c0 += 32, ++n) {
+        uint32_t w[6];
+        const uint4 ea = __ldg(ta + c0);
+        w[0] = ea.x, w[1] = ea.y, w[2] = ea.z, w[3] = ea.w;
+        if (P > 8) {
+          const uint2 eb = __ldg(tb + c0);
+          w[4] = eb.x, w[5] = eb.y;
+        }
+        if (!warp_wait(bar_done, n & 1u, s.spin_limit, abort_flag, err, 23)) {
+          ok = false;
+          break;
+        }
+        fence_after();
+        float yv[32];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          float r[8], l[8];
+          tld8(tw + 64 + 8 * h, r);
+          tld8(tw + 96 + 8 * h, l);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 8; ++i) yv[8 * h + i] = r[i] + l[i];
+        }
+        fence_before();
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_free) : "memory");
         float *yl = y + c0 + lane;
         const uint32_t add = c0 + lane <= last ? holes : 0u;
 #pragma unroll
@@ -261,19 +247,27 @@ sigma_pair_warp_kernel(const __grid_constant__ PwShape s, const uint32_t *__rest
           if (b + 2 < NR) red_if(yl + r.z, yv[P + b + 2], add & (1u << (b + 2)));
           if (b + 3 < NR) red_if(yl + r.w, yv[P + b + 3], add & (1u << (b + 3)));
         }
+        // own row: one orbital at a time no two sets meet (S -> S u o is one to
+        // one), and the warp alone adds to it
+#pragma unroll
+        for (int o = 0; o < P; ++o) {
+          const uint32_t a = ca + (o & 1 ? w[o >> 1] >> 16 : w[o >> 1] & 0xffffu);
+          sts(a, lds(a) + yv[o]);
+          __syncwarp();
+        }
       }
-    }
-    __syncwarp();
-    if (!stop)
-      for (uint32_t c = lane; c < n_own; c += 32) atomicAdd(y + own + c, fmaf(diag[own + c], xo[c], yo[c]));
-    __syncwarp();
-  }
-  // after a wait that ran out: the MMAs in flight complete by themselves;
-  // wait for them (bounded) before the tensor memory is freed
-  if (stop && w4 == 0 && issued > 0) {
-    for (long i = 0; i < kTcSpinLimit && !mbar_try(bar, (issued - 1) & 1u); ++i) {
+      __syncwarp();
+      if (ok)
+        for (uint32_t c = lane; c < n_own; c += 32)
+          atomicAdd(y + own + c, fmaf(diag[own + c], __ldg(x + own + c), cells[c]));
+      __syncwarp();
     }
   }
+  // after a wait that ran out: the MMAs in flight complete by themselves; wait
+  // for them (bounded) before the tensor memory is freed
+  if (gatherer && w4 == 0 && !ok && n > 0)
+    for (long i = 0; i < kTcSpinLimit && !mbar_try(bar_done, (n - 1) & 1u); ++i) {
+    }
   fence_before();
   __syncthreads();
   fence_after();
@@ -332,11 +326,11 @@ int pw_tables(int device, int P, PwTables *out) {
 
 template <int P>
 int launch_p(const doci_ham *h, const PwShape &s, const float *x, float *y, cudaStream_t st) {
-  const size_t smem = std::max(kMinSmem, static_cast<size_t>(kOffRows) + 2 * 4 * pw::cells(P) * (kThreads / 32));
+  const size_t smem = std::max(kMinSmem, static_cast<size_t>(kOffRows) + 4 * pw::cells(P) * (kThreads / 32));
   int per_sm = 1;
   const int r = kernel_blocks(reinterpret_cast<const void *>(sigma_pair_warp_kernel<P>), kThreads, smem, &per_sm);
   if (r != DOCI_OK) return r;
-  const int grid = std::min(device_sm_count(), (s.nquads + kWgs - 1) / kWgs);
+  const int grid = std::min(device_sm_count(), (s.nquads + kSlots - 1) / kSlots);
   sigma_pair_warp_kernel<P><<<grid, kThreads, smem, st>>>(s, h->d_wunits, h->d_wstart,
                                                           static_cast<const uint4 *>(h->d_wtab_a),
                                                           static_cast<const uint2 *>(h->d_wtab_b),
@@ -366,7 +360,7 @@ int ham_build_pair_warp(doci_ham *h) {
     if (L - p < 2 || L - p > 24) continue;
     P = p;
     g = pw::groups(P, L - P, N, B.data(), kBinomCols);
-    const uint32_t slots = static_cast<uint32_t>(kWgs * device_sm_count());
+    const uint32_t slots = static_cast<uint32_t>(kSlots * device_sm_count());
     if (g.first[g.n] / 4 >= (p == 12 ? 4 : 1) * slots) break;
   }
   const int na = L - P;

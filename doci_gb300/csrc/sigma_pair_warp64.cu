@@ -119,24 +119,6 @@ __device__ __forceinline__ void mma_f16(uint32_t d, uint32_t a, uint64_t b, uint
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d),
       "r"(a), "l"(b), "r"(id), "r"(acc));
 }
-__device__ __forceinline__ void tst8(uint32_t t, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(t), "r"(r[0]), "r"(r[1]),
-               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
-__device__ __forceinline__ void tst1(uint32_t t, uint32_t r) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(t), "r"(r) : "memory");
-}
-__device__ __forceinline__ uint32_t tld1(uint32_t t) {
-  uint32_t r;
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(t));
-  return r;
-}
-__device__ __forceinline__ void tld8(uint32_t t, float (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
-               : "r"(t));
-}
 // (h + l) 2^e as a double by integer operations, |l| at most an ulp of h, h 0
 // or of magnitude 2^-74 .. 2^120 (the FP64 units convert one lane in 64
 // cycles per quarter SM); nan: or-ed into the high word
@@ -151,21 +133,6 @@ __device__ __forceinline__ double widen(float h, float l, int e, uint32_t nan) {
   uint32_t lo = static_cast<uint32_t>(m);
   if (mag == 0) hi = lo = 0;
   return __hiloint2double(static_cast<int>(hi | (u & 0x80000000u) | nan), static_cast<int>(lo));
-}
-
-// bounded wait by a whole warp; false when it ran out or the slot was given up
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, long limit, volatile int *abort_flag, int *err) {
-  bool done = false;
-  for (long k = 0; k < limit && !done; ++k) {
-    done = mbar_try(bar, parity);
-    if (!done && (k & 63) == 63 && *abort_flag) break;
-  }
-  done = __all_sync(0xffffffffu, done);
-  if (!done && (threadIdx.x & 31) == 0) {
-    *abort_flag = 1;
-    atomicCAS(err, 0, 22);
-  }
-  return done;
 }
 
 template <int P>
@@ -283,7 +250,7 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
         const bool inf = eb == 255u;
         const float f1 = inf ? __uint_as_float(0x7fc00000u) : __uint_as_float((262u - eb) << 23);  // 2^(135 - eb)
         const float f3 = __uint_as_float((284u - (inf ? 30u : eb)) << 23);                         // 2^(157 - eb)
-        if (n > 0 && !warp_wait(bar_done, (n - 1) & 1u, s.spin_limit, abort_flag, err)) fail = true;
+        if (n > 0 && !warp_wait(bar_done, (n - 1) & 1u, s.spin_limit, abort_flag, err, 31)) fail = true;
         fence_after();
         // five signed digits of eleven bits, most significant first:
         // X 2^(124 - eb) = sum_i d_i 2^(-11 i), below 1/4, d_i the nearest
@@ -327,7 +294,7 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
         }
         if (w4 == 0) {
           // D of the tile before has to be read
-          if (n > 0 && !warp_wait(bar_free, (n - 1) & 1u, s.spin_limit, abort_flag, err)) fail = true;
+          if (n > 0 && !warp_wait(bar_free, (n - 1) & 1u, s.spin_limit, abort_flag, err, 32)) fail = true;
           if (!fail && lane == 0) {
             fence_after();
             // digit i of X times digits 1..6-i of K (128-byte rows, 32 rows per
@@ -353,7 +320,7 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
           const uint2 eb = __ldg(tb + c0 + lane);
           w[4] = eb.x, w[5] = eb.y;
         }
-        if (!warp_wait(bar_done, n & 1u, s.spin_limit, abort_flag, err)) {
+        if (!warp_wait(bar_done, n & 1u, s.spin_limit, abort_flag, err, 33)) {
           ok = false;
           break;
         }

@@ -38,13 +38,6 @@ __device__ __forceinline__ void red_if(float *p, float v, uint32_t on) {
                "r"(on)
                : "memory");
 }
-// (a0, a1) + (b0, b1) and - in one instruction (FP32, round to nearest)
-__device__ __forceinline__ void add2(float &a0, float &a1, float b0, float b1) {
-  asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\tadd.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, "
-      "p;\n\t}\n"
-      : "+f"(a0), "+f"(a1)
-      : "f"(b0), "f"(b1));
-}
 __device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -73,19 +66,38 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
          (static_cast<uint64_t>(1024 >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
          (static_cast<uint64_t>(2) << 61);
 }
-__device__ __forceinline__ void tld16(uint32_t t, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(t));
+__device__ __forceinline__ void tst8(uint32_t t, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(t), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
 }
-__device__ __forceinline__ void tst16(uint32_t t, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(t),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
+__device__ __forceinline__ void tld8(uint32_t t, float (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
+               : "r"(t));
+}
+__device__ __forceinline__ void tst1(uint32_t t, uint32_t r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(t), "r"(r) : "memory");
+}
+__device__ __forceinline__ uint32_t tld1(uint32_t t) {
+  uint32_t r;
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(t));
+  return r;
+}
+// bounded wait by a whole warp; false when it ran out or the slot was given up
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, long limit, volatile int *abort_flag, int *err,
+                                          int code) {
+  bool done = false;
+  for (long k = 0; k < limit && !done; ++k) {
+    done = mbar_try(bar, parity);
+    if (!done && (k & 63) == 63 && *abort_flag) break;
+  }
+  done = __all_sync(0xffffffffu, done);
+  if (!done && (threadIdx.x & 31) == 0) {
+    *abort_flag = 1;
+    atomicCAS(err, 0, code);
+  }
+  return done;
 }
 // byte offset of element (row r, column k) of a 128-byte-swizzled K-major tile of 32 FP32 per row
 __host__ __device__ __forceinline__ uint32_t sw128(uint32_t r, uint32_t k) {
