@@ -177,6 +177,11 @@ bool pair_warp_fits(const doci_ham *h);
 int launch_pair_warp(const doci_ham *h, const float *x, float *y, cudaStream_t s);
 // the same in FP64 accuracy (sigma_pair_warp64.cu)
 int launch_pair_warp64(const doci_ham *h, const double *x, double *y, cudaStream_t s);
+// the reproducible forms: no atomic adds, pair_warp_slabs(h) vectors of D
+// elements of scratch
+int pair_warp_slabs(const doci_ham *h);
+int launch_pair_warp_det(const doci_ham *h, const float *x, float *y, float *slab, cudaStream_t s);
+int launch_pair_warp64_det(const doci_ham *h, const double *x, double *y, double *slab, cudaStream_t s);
 // FP64-accurate pair form in float-float arithmetic, one block per unit (sigma_pair.cu)
 bool pair_ff_fits(const doci_ham *h);
 int launch_pair_ff(const doci_ham *h, const double *x, double *y, cudaStream_t s);

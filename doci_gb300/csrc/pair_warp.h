@@ -17,6 +17,9 @@ struct PwShape {
 };
 PwShape pair_warp_shape(const doci_ham *h);
 int ham_build_kdigits(doci_ham *h);
+// the last pass of the reproducible form (sigma_pair_warp.cu)
+template <typename T>
+int launch_sum_slabs(const doci_ham *h, const T *slab, T *y, cudaStream_t st);
 
 inline int cuda_ok(const char *what) {
   const cudaError_t e = cudaGetLastError();

@@ -952,6 +952,45 @@ int multi_method_auto(const doci_ham *h, int precision) {
   return kMultiSingle;
 }
 
+// One vector at a time through the reproducible pair form: the pair kernels
+// with every contribution stored in a place of its own and summed in a fixed
+// order, up to kDetMaxBytes of scratch (40.1M determinants in FP64: 4.2 GiB).
+// Measured against the multi-vector row and gather kernels (us, nv = 2 / 4):
+// FP32 L=24 N=12 1,256 / 1,455 -> 247 / 490; L=20 N=10 140 / 155 -> 52 / 101;
+// L=18 N=9 72 / 79 -> 44 / 81, so from 2^16 determinants for three vectors or
+// more, 2^15 for fewer.  FP64 L=24 2,915 / 3,113 -> 725 / 1,444; L=18 102 / 110
+// -> 64 / 125.
+constexpr size_t kDetMaxBytes = size_t(5) << 30;
+bool det_fits(const doci_ham *h, size_t elem, int nv) {
+  return h->sigma_kernel == 0 && pair_warp_fits(h) && h->D >= (nv >= 3 ? 1u << 16 : 1u << 15) &&
+         static_cast<size_t>(pair_warp_slabs(h)) * h->D * elem <= kDetMaxBytes;
+}
+// *done = false: there is no memory for the scratch
+int run_det(const doci_ham *h, const char *x, size_t ldx, char *y, size_t ldy, int nv, int precision, cudaStream_t st,
+            bool *done) {
+  const size_t elem = precision == DOCI_FP64 ? 8 : 4;
+  *done = false;
+  void *slab = nullptr;
+  if (cudaMallocAsync(&slab, static_cast<size_t>(pair_warp_slabs(h)) * h->D * elem, st) != cudaSuccess) {
+    cudaGetLastError();
+    return DOCI_OK;
+  }
+  *done = true;
+  int r = DOCI_OK;
+  for (int v = 0; v < nv && r == DOCI_OK; ++v) {
+    const char *xv = x + v * ldx * elem;
+    char *yv = y + v * ldy * elem;
+    r = precision == DOCI_FP64
+            ? launch_pair_warp64_det(h, reinterpret_cast<const double *>(xv), reinterpret_cast<double *>(yv),
+                                     static_cast<double *>(slab), st)
+            : launch_pair_warp_det(h, reinterpret_cast<const float *>(xv), reinterpret_cast<float *>(yv),
+                                   static_cast<float *>(slab), st);
+  }
+  const cudaError_t e = cudaFreeAsync(slab, st);
+  if (r == DOCI_OK) DOCI_CUDA(e);
+  return r;
+}
+
 int run_multi(const doci_ham *h, int method, const void *x, size_t ldx, void *y, size_t ldy, int nv, int precision,
               cudaStream_t st) {
   const size_t elem = precision == DOCI_FP64 ? 8 : 4;
@@ -974,6 +1013,11 @@ int run_multi(const doci_ham *h, int method, const void *x, size_t ldx, void *y,
   if (method == kMultiGather)
     return precision == DOCI_FP64 ? launch_gather_multi_typed<double>(h, x, ldx, y, ldy, nv, st)
                                   : launch_gather_multi_typed<float>(h, x, ldx, y, ldy, nv, st);
+  if (det_fits(h, elem, nv)) {
+    bool done;
+    const int r = run_det(h, xc, ldx, yc, ldy, nv, precision, st, &done);
+    if (done || r != DOCI_OK) return r;
+  }
   for (int v = 0; v < nv; ++v) {  // one vector at a time
     const int r = launch_sigma(h, xc + v * ldx * elem, yc + v * ldy * elem, precision, st, false);
     if (r) return r;
@@ -987,9 +1031,14 @@ int launch_sigma_multi(const doci_ham *h, const void *x, size_t ldx, void *y, si
                        cudaStream_t st) {
   if (nv < 1 || nv > 4 || ldx < h->D || ldy < h->D) return DOCI_ERR_INVALID;
   if (precision != DOCI_FP64 && precision != DOCI_FP32) return DOCI_ERR_INVALID;
-  // the block solves stay run-to-run reproducible: no pair form here
-  if (nv == 1) return launch_sigma(h, x, y, precision, st, false);
+  // block sigmas are reproducible from run to run: no atomic adds here
   int method = h->sigma_kernel == 0 ? tuned_choice(h, precision, nv, false) : 0;
+  if (method == 0 && det_fits(h, precision == DOCI_FP64 ? 8 : 4, nv)) {
+    bool done;
+    const int r = run_det(h, static_cast<const char *>(x), ldx, static_cast<char *>(y), ldy, nv, precision, st, &done);
+    if (done || r != DOCI_OK) return r;
+  }
+  if (nv == 1) return launch_sigma(h, x, y, precision, st, false);
   if (method == 0) method = multi_method_auto(h, precision);
   return run_multi(h, method, x, ldx, y, ldy, nv, precision, st);
 }

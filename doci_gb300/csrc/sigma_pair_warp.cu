@@ -78,13 +78,17 @@ __device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint3
 // measured about five)
 __device__ __forceinline__ uint32_t tf32_rna(float f) { return (__float_as_uint(f) + 0x1000u) & 0xffffe000u; }
 
-template <int P>
+// DET: what is added to hole rows is stored instead, each contribution in a
+// place of its own (`slab`: the sum that element e of the target's row part
+// contributes to determinant T at e D + T), and the own row is stored; the
+// sums then have a fixed order (sum_slabs_kernel).
+template <int P, bool DET>
 __global__ void __launch_bounds__(kThreads, 1)
 sigma_pair_warp_kernel(const __grid_constant__ PwShape s, const uint32_t *__restrict__ units,
                        const uint32_t *__restrict__ rowstart, const uint4 *__restrict__ tab_a,
                        const uint2 *__restrict__ tab_b, const float *__restrict__ g_ksplit,
                        const float *__restrict__ diag, const float *__restrict__ x, float *__restrict__ y,
-                       int *__restrict__ err) {
+                       float *__restrict__ slab, int *__restrict__ err) {
   constexpr int NR = 32 - P;
   constexpr int XC = pw::cells(P);
   extern __shared__ __align__(1024) uint8_t sm[];
@@ -142,7 +146,9 @@ sigma_pair_warp_kernel(const __grid_constant__ PwShape s, const uint32_t *__rest
     // (a unit without sets has no hole rows either)
     if (lane < 24) {
       const bool hole = n_s && ((holes >> lane) & 1u);
-      reinterpret_cast<uint32_t *>(sm + kOffStart)[warp * 24 + lane] = hole ? rowstart[mask | (1u << lane)] : 0u;
+      uint32_t r = hole ? rowstart[mask | (1u << lane)] : 0u;
+      if (DET && hole && !gatherer) r += s.D * static_cast<uint32_t>(__popc(mask & ((1u << lane) - 1u)));
+      reinterpret_cast<uint32_t *>(sm + kOffStart)[warp * 24 + lane] = r;
     }
     __syncwarp();
     const uint4 *ta = tab_a + (n_s ? s.off[jp] : 0u) + lane;
@@ -237,15 +243,19 @@ sigma_pair_warp_kernel(const __grid_constant__ PwShape s, const uint32_t *__rest
         fence_before();
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_free) : "memory");
-        float *yl = y + c0 + lane;
+        float *yl = (DET ? slab : y) + c0 + lane;
         const uint32_t add = c0 + lane <= last ? holes : 0u;
+        auto put = [](float *p, float v, uint32_t on) {
+          if (DET) st_if(p, v, on);
+          else red_if(p, v, on);
+        };
 #pragma unroll
         for (int b = 0; b < NR; b += 4) {
           const uint4 r = lds128(ra + 4 * b);
-          red_if(yl + r.x, yv[P + b], add & (1u << b));
-          red_if(yl + r.y, yv[P + b + 1], add & (1u << (b + 1)));
-          if (b + 2 < NR) red_if(yl + r.z, yv[P + b + 2], add & (1u << (b + 2)));
-          if (b + 3 < NR) red_if(yl + r.w, yv[P + b + 3], add & (1u << (b + 3)));
+          put(yl + r.x, yv[P + b], add & (1u << b));
+          put(yl + r.y, yv[P + b + 1], add & (1u << (b + 1)));
+          if (b + 2 < NR) put(yl + r.z, yv[P + b + 2], add & (1u << (b + 2)));
+          if (b + 3 < NR) put(yl + r.w, yv[P + b + 3], add & (1u << (b + 3)));
         }
         // own row: one orbital at a time no two sets meet (S -> S u o is one to
         // one), and the warp alone adds to it
@@ -258,8 +268,11 @@ sigma_pair_warp_kernel(const __grid_constant__ PwShape s, const uint32_t *__rest
       }
       __syncwarp();
       if (ok)
-        for (uint32_t c = lane; c < n_own; c += 32)
-          atomicAdd(y + own + c, fmaf(diag[own + c], __ldg(x + own + c), cells[c]));
+        for (uint32_t c = lane; c < n_own; c += 32) {
+          const float v = fmaf(diag[own + c], __ldg(x + own + c), cells[c]);
+          if (DET) y[own + c] = v;
+          else atomicAdd(y + own + c, v);
+        }
       __syncwarp();
     }
   }
@@ -281,6 +294,28 @@ __global__ void zero_kernel(float *__restrict__ y, uint32_t n) {
   for (uint32_t i = i0; i < n4; i += gridDim.x * blockDim.x) y4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   if (i0 < head) y[i0] = 0.f;
   if (i0 < n - head - 4 * n4) y[head + 4 * n4 + i0] = 0.f;
+}
+
+// sigma[T] += the slabs of the elements of T's row part, in ascending order; a
+// warp per row
+template <typename T>
+__global__ void __launch_bounds__(256)
+sum_slabs_kernel(const __grid_constant__ PwShape s, const uint32_t *__restrict__ units,
+                 const uint32_t *__restrict__ rowstart, const T *__restrict__ slab, T *__restrict__ y) {
+  const int lane = threadIdx.x & 31;
+  for (int u = (blockIdx.x * 256 + threadIdx.x) >> 5; u < 4 * s.nquads; u += gridDim.x * 8) {
+    const uint32_t mask = units[u];
+    if (mask == pw::kNone) continue;
+    const int k = __popc(mask);
+    const uint32_t n = s.n[s.N - k], r = n ? rowstart[mask] : 0u;
+    for (uint32_t c = lane; c < n; c += 32) {
+      T v = y[r + c];
+      const T *p = slab + r + c;
+#pragma unroll 4
+      for (int e = 0; e < k; ++e) v += p[static_cast<size_t>(e) * s.D];
+      y[r + c] = v;
+    }
+  }
 }
 
 __global__ void build_starts_kernel(uint32_t *out, int P, int na, int N, uint32_t D, const uint32_t *binom) {
@@ -324,18 +359,18 @@ int pw_tables(int device, int P, PwTables *out) {
   return DOCI_OK;
 }
 
-template <int P>
-int launch_p(const doci_ham *h, const PwShape &s, const float *x, float *y, cudaStream_t st) {
+template <int P, bool DET>
+int launch_p(const doci_ham *h, const PwShape &s, const float *x, float *y, float *slab, cudaStream_t st) {
   const size_t smem = std::max(kMinSmem, static_cast<size_t>(kOffRows) + 4 * pw::cells(P) * (kThreads / 32));
   int per_sm = 1;
-  const int r = kernel_blocks(reinterpret_cast<const void *>(sigma_pair_warp_kernel<P>), kThreads, smem, &per_sm);
+  const int r = kernel_blocks(reinterpret_cast<const void *>(sigma_pair_warp_kernel<P, DET>), kThreads, smem, &per_sm);
   if (r != DOCI_OK) return r;
   const int grid = std::min(device_sm_count(), (s.nquads + kSlots - 1) / kSlots);
-  sigma_pair_warp_kernel<P><<<grid, kThreads, smem, st>>>(s, h->d_wunits, h->d_wstart,
+  sigma_pair_warp_kernel<P, DET><<<grid, kThreads, smem, st>>>(s, h->d_wunits, h->d_wstart,
                                                           static_cast<const uint4 *>(h->d_wtab_a),
                                                           static_cast<const uint2 *>(h->d_wtab_b),
                                                           reinterpret_cast<const float *>(h->d_kfrag), h->d_diag32, x,
-                                                          y, h->d_tc_err);
+                                                          y, slab, h->d_tc_err);
   DOCI_CUDA(cudaGetLastError());
   return DOCI_OK;
 }
@@ -408,9 +443,31 @@ int launch_pair_warp(const doci_ham *h, const float *x, float *y, cudaStream_t s
   zero_kernel<<<static_cast<unsigned>(std::min<uint64_t>((h->D / 4 + 256) / 256, 8ull * device_sm_count())), 256, 0,
                 st>>>(y, h->D);
   DOCI_CUDA(cudaGetLastError());
-  if (h->wsplit == 12) return launch_p<12>(h, s, x, y, st);
-  if (h->wsplit == 10) return launch_p<10>(h, s, x, y, st);
-  return launch_p<8>(h, s, x, y, st);
+  if (h->wsplit == 12) return launch_p<12, false>(h, s, x, y, nullptr, st);
+  if (h->wsplit == 10) return launch_p<10, false>(h, s, x, y, nullptr, st);
+  return launch_p<8, false>(h, s, x, y, nullptr, st);
 }
+
+// slabs of the reproducible form: the largest row part
+int pair_warp_slabs(const doci_ham *h) { return std::min(h->L - h->wsplit, h->N); }
+
+int launch_pair_warp_det(const doci_ham *h, const float *x, float *y, float *slab, cudaStream_t st) {
+  if (!pair_warp_fits(h)) return DOCI_ERR_INVALID;
+  const PwShape s = pair_warp_shape(h);
+  const int r = h->wsplit == 12   ? launch_p<12, true>(h, s, x, y, slab, st)
+                : h->wsplit == 10 ? launch_p<10, true>(h, s, x, y, slab, st)
+                                  : launch_p<8, true>(h, s, x, y, slab, st);
+  return r == DOCI_OK ? launch_sum_slabs(h, slab, y, st) : r;
+}
+
+template <typename T>
+int launch_sum_slabs(const doci_ham *h, const T *slab, T *y, cudaStream_t st) {
+  const PwShape s = pair_warp_shape(h);
+  sum_slabs_kernel<T><<<std::min(16 * device_sm_count(), (4 * s.nquads + 7) / 8), 256, 0, st>>>(s, h->d_wunits,
+                                                                                              h->d_wstart, slab, y);
+  return cuda_ok("sum_slabs_kernel");
+}
+template int launch_sum_slabs<float>(const doci_ham *, const float *, float *, cudaStream_t);
+template int launch_sum_slabs<double>(const doci_ham *, const double *, double *, cudaStream_t);
 
 }  // namespace doci

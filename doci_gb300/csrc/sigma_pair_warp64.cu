@@ -135,12 +135,14 @@ __device__ __forceinline__ double widen(float h, float l, int e, uint32_t nan) {
   return __hiloint2double(static_cast<int>(hi | (u & 0x80000000u) | nan), static_cast<int>(lo));
 }
 
-template <int P>
+// DET: as in sigma_pair_warp.cu, contributions stored in slabs instead of added
+template <int P, bool DET>
 __global__ void __launch_bounds__(kThreads64, 1)
 sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__restrict__ units,
                          const uint32_t *__restrict__ rowstart, const uint4 *__restrict__ tab_a,
                          const uint2 *__restrict__ tab_b, const uint16_t *__restrict__ g_kdig, int kexp,
-                         const ff *__restrict__ x, double *__restrict__ y, int *__restrict__ err) {
+                         const ff *__restrict__ x, double *__restrict__ y, double *__restrict__ slab,
+                         int *__restrict__ err) {
   constexpr int NR = 32 - P;
   constexpr int XC = pw::cells(P);
   extern __shared__ __align__(1024) uint8_t sm[];
@@ -202,7 +204,9 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
     }
     if (lane < 24) {
       const bool hole = n_s && ((holes >> lane) & 1u);
-      reinterpret_cast<uint32_t *>(sm + kOffStart)[warp * 24 + lane] = hole ? rowstart[mask | (1u << lane)] : 0u;
+      uint32_t r = hole ? rowstart[mask | (1u << lane)] : 0u;
+      if (DET && hole && !gatherer) r += s.D * static_cast<uint32_t>(__popc(mask & ((1u << lane) - 1u)));
+      reinterpret_cast<uint32_t *>(sm + kOffStart)[warp * 24 + lane] = r;
     }
     __syncwarp();
     if (n_s == 0) continue;
@@ -366,7 +370,7 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
             __syncwarp();
           }
         }
-        double *yr = y + c0 + lane;
+        double *yr = (DET ? slab : y) + c0 + lane;
         const uint32_t add = c0 + lane <= last ? holes : 0u;
         // a NaN or an infinity among the set's values makes every product NaN
         const uint32_t nan = yh[0] == yh[0] ? 0u : 0x7ff80000u;
@@ -376,8 +380,11 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
           const uint32_t st[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
           for (int i = 0; i < 4; ++i)
-            if (b + i < NR && (holes & (1u << (b + i))))
-              red64_if(yr + st[i], widen(yh[P + b + i], yl[P + b + i], e, nan), add & (1u << (b + i)));
+            if (b + i < NR && (holes & (1u << (b + i)))) {
+              const double v = widen(yh[P + b + i], yl[P + b + i], e, nan);
+              if (!DET) red64_if(yr + st[i], v, add & (1u << (b + i)));
+              else if (add) yr[st[i]] = v;
+            }
         }
       }
       __syncwarp();
@@ -389,7 +396,9 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
           const float h = v.x + v.y, l = v.y - (h - v.x);
           const uint32_t mh = __float_as_uint(h) & 0x7fffffffu;
           const bool plain = mag < 0x7b800000u && (mh == 0 || mh > 0x1a800000u);
-          atomicAdd(y + own + c, plain ? widen(h, l, 0, 0u) : static_cast<double>(v.x) + static_cast<double>(v.y));
+          const double t = plain ? widen(h, l, 0, 0u) : static_cast<double>(v.x) + static_cast<double>(v.y);
+          if (DET) y[own + c] += t;
+          else atomicAdd(y + own + c, t);
         }
       __syncwarp();
     }
@@ -415,16 +424,16 @@ __global__ void init64_kernel(uint32_t D, const double *__restrict__ diag, const
   }
 }
 
-template <int P>
-int launch_p(const doci_ham *h, const PwShape &s, const ff *x, double *y, cudaStream_t st) {
+template <int P, bool DET>
+int launch_p(const doci_ham *h, const PwShape &s, const ff *x, double *y, double *slab, cudaStream_t st) {
   const size_t smem = std::max(kMinSmem, static_cast<size_t>(kOffCells) + 8 * pw::cells(P) * (kThreads64 / 32));
   int per_sm = 1;
-  const int r = kernel_blocks(reinterpret_cast<const void *>(sigma_pair_warp64_kernel<P>), kThreads64, smem, &per_sm);
+  const int r = kernel_blocks(reinterpret_cast<const void *>(sigma_pair_warp64_kernel<P, DET>), kThreads64, smem, &per_sm);
   if (r != DOCI_OK) return r;
   const int grid = std::min(device_sm_count(), (s.nquads + kSlots - 1) / kSlots);
-  sigma_pair_warp64_kernel<P><<<grid, kThreads64, smem, st>>>(
+  sigma_pair_warp64_kernel<P, DET><<<grid, kThreads64, smem, st>>>(
       s, h->d_wunits, h->d_wstart, static_cast<const uint4 *>(h->d_wtab_a), static_cast<const uint2 *>(h->d_wtab_b),
-      h->d_kdig, h->kdig_exp, x, y, h->d_tc_err);
+      h->d_kdig, h->kdig_exp, x, y, slab, h->d_tc_err);
   DOCI_CUDA(cudaGetLastError());
   return DOCI_OK;
 }
@@ -471,7 +480,9 @@ int ham_build_kdigits(doci_ham *h) {
   return DOCI_OK;
 }
 
-int launch_pair_warp64(const doci_ham *h, const double *x, double *y, cudaStream_t st) {
+namespace {
+template <bool DET>
+int launch64(const doci_ham *h, const double *x, double *y, double *slab, cudaStream_t st) {
   if (!pair_warp_fits(h)) return DOCI_ERR_INVALID;
   ff *xf = nullptr;
   DOCI_CUDA(cudaMallocAsync(&xf, sizeof(ff) * static_cast<size_t>(h->D), st));
@@ -481,14 +492,24 @@ int launch_pair_warp64(const doci_ham *h, const double *x, double *y, cudaStream
   int r = cuda_ok("init64_kernel");
   if (r == DOCI_OK) {
     const PwShape s = pair_warp_shape(h);
-    r = h->wsplit == 12 ? launch_p<12>(h, s, xf, y, st)
-        : h->wsplit == 10 ? launch_p<10>(h, s, xf, y, st)
-                          : launch_p<8>(h, s, xf, y, st);
+    r = h->wsplit == 12   ? launch_p<12, DET>(h, s, xf, y, slab, st)
+        : h->wsplit == 10 ? launch_p<10, DET>(h, s, xf, y, slab, st)
+                          : launch_p<8, DET>(h, s, xf, y, slab, st);
   }
   const cudaError_t ef = cudaFreeAsync(xf, st);
   if (r != DOCI_OK) return r;
   DOCI_CUDA(ef);
   return DOCI_OK;
+}
+}  // namespace
+
+int launch_pair_warp64(const doci_ham *h, const double *x, double *y, cudaStream_t st) {
+  return launch64<false>(h, x, y, nullptr, st);
+}
+
+int launch_pair_warp64_det(const doci_ham *h, const double *x, double *y, double *slab, cudaStream_t st) {
+  const int r = launch64<true>(h, x, y, slab, st);
+  return r == DOCI_OK ? launch_sum_slabs(h, slab, y, st) : r;
 }
 
 }  // namespace doci

@@ -38,6 +38,11 @@ __device__ __forceinline__ void red_if(float *p, float v, uint32_t on) {
                "r"(on)
                : "memory");
 }
+__device__ __forceinline__ void st_if(float *p, float v, uint32_t on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.global.f32 [%0], %1;\n\t}\n" ::"l"(p), "f"(v),
+               "r"(on)
+               : "memory");
+}
 __device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
   uint32_t ok;
   asm volatile(

@@ -159,13 +159,16 @@ const double *doci_ham_diagonal_device(const doci_ham *ham);
 int doci_sigma(doci_ham *ham, const void *d_x, void *d_y, int precision, void *stream);
 
 /* Block sigma Y_v = H X_v for v < nv on device buffers: X and Y column-major
- * with leading dimensions ldx, ldy >= D (elements).  The neighbour ranks and
- * hop weights of each determinant are computed once per launch for up to
- * four vectors (larger nv runs in groups of four), so a block of vectors
- * costs much less than nv doci_sigma calls.  Results agree with doci_sigma to
+ * with leading dimensions ldx, ldy >= D (elements).  Without atomic adds:
+ * results repeat bit for bit.  On large spaces one vector after the other in
+ * the pair form with every contribution in a place of its own (stream-ordered
+ * scratch of at most min(N, L - 8) x D elements, up to 5 GiB); else, and when
+ * there is no memory for that, the neighbour ranks and hop weights of each
+ * determinant are computed once per launch for up to four vectors (larger nv
+ * runs in groups of four).  Results agree with doci_sigma to
  * rounding (identical when both use the same kernel).  No counterpart in the
- * reference, whose matvec (doci.c:164-238) takes one vector; used by the
- * block Davidson of doci_solve_roots.  Asynchronous on stream (NULL = the
+ * reference, whose matvec (doci.c:164-238) takes one vector; for callers with
+ * block methods.  Asynchronous on stream (NULL = the
  * default stream). */
 int doci_sigma_block(doci_ham *ham, const void *d_X, int64_t ldx, void *d_Y, int64_t ldy, int nv, int precision,
                      void *stream);

@@ -454,3 +454,30 @@ def test_sigma_pair_warp_nonfinite(L, N, seed, prec_name, kernel, bad, synth, dg
             torch.cuda.synchronize()
             out.append(torch.isfinite(y))
         assert torch.equal(out[0], out[1]) and int((~out[0]).sum()) == N * (L - N) + 1
+
+
+@pytest.mark.parametrize("L,N,seed,nv", [(18, 9, 111, 2), (20, 13, 112, 3), (22, 8, 113, 5), (23, 17, 114, 1),
+                                         (28, 6, 115, 2), (32, 4, 116, 3)])
+def test_sigma_block_reproducible(L, N, seed, nv, synth, dg):
+    """The automatic block sigma (the pair form with contributions stored apart
+    on these sizes: 8, 10 and 12 column orbitals, many and few pairs) gives the
+    oracle's matvec of each column and the same bits when called again."""
+    torch = torch_cuda()
+    p = synth(L, N, seed)
+    o = oracle.Ham(p)
+    with dg.Hamiltonian.from_fcidump(p) as h:
+        D = h.D
+        X = np.random.default_rng(seed).standard_normal((nv, D))
+        refs = [o.matvec(x) for x in X]
+        for prec, dt, tol in ((dg.FP64, torch.float64, TOL64), (dg.FP32, torch.float32, TOL32)):
+            xb = torch.from_numpy(X).to(dt).cuda()
+            outs = []
+            for _ in range(2):
+                y = torch.full((nv, D + 1), float("nan"), dtype=dt, device="cuda")
+                h.sigma_block_device(xb.data_ptr(), D, y.data_ptr(), D + 1, nv, prec)
+                torch.cuda.synchronize()
+                outs.append(y[:, :D].clone())
+                assert bool(torch.isnan(y[:, D]).all())
+            assert torch.equal(outs[0], outs[1])
+            for v in range(nv):
+                assert np.abs(outs[0][v].double().cpu().numpy() - refs[v]).max() <= tol * np.abs(refs[v]).max()
