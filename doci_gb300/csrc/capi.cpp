@@ -387,7 +387,8 @@ int64_t doci_solve_footprint(int L, int n_pairs, const doci_solve_opts *o, int n
   (void)nroots;
   const int64_t D = static_cast<int64_t>(binom64(L, n_pairs));
   const int64_t mv = o->davidson_max_vec;
-  const int64_t ham = D * 12;  // FP64 + FP32 diagonal
+  // FP64 + FP32 diagonal, neighbour table
+  const int64_t ham = D * 12 + static_cast<int64_t>(nbr_table_bytes(L, n_pairs, D));
   int64_t solver;
   if (o->solver != DOCI_SOLVER_D) {
     solver = D * 8 * 7;  // x, p, Ax, Ap, g, pinv + start

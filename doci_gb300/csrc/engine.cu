@@ -67,6 +67,7 @@ constexpr int kMaxV = 32;               // basis vectors
 struct EProb {
   uint32_t D;
   int L, N, nh;
+  const uint32_t *nbr;  // neighbour table (small spaces; sigma.cu), or null
   const void *K;        // mirrored K (32 x 32) in the phase's type
   const void *diag_s;   // the sigma's diagonal in the phase's type (FP32 phase: diag - shift)
   const double *diag;   // FP64 diagonal (preconditioner)
@@ -186,10 +187,6 @@ __global__ void __launch_bounds__(kET) eng_sigma(EArgs a) {
   for (int e = 0; e < pb.dpt; ++e) {
   const uint32_t r = tile_first + e * kET;
   if (r >= pb.D) return;
-  const uint32_t Dm1 = pb.D - 1, R = Dm1 - r;
-  const uint32_t M = dev::colex_unrank<kBinomCols>(R, pb.L, pb.N, B);
-  dev::Neighbours<NH, kBinomCols> nb;
-  nb.precompute(M, R, pb.L, pb.nh, B);
   struct Acc {
     const S *K, *x;
     uint32_t D;
@@ -208,7 +205,29 @@ __global__ void __launch_bounds__(kET) eng_sigma(EArgs a) {
 #pragma unroll
   for (int v = 0; v < kMaxR; ++v)
     if (v < nv) f.acc[v] = d * x[static_cast<size_t>(v) * pb.D + r];
-  nb.visit(M, R, Dm1, pb.N, pb.nh, B, f);
+  if (pb.nbr) {  // the same hops in the same order, from the table
+    const int hops = pb.N * pb.nh;
+    const uint32_t *t = pb.nbr + r;
+    constexpr int kB = 4;
+    for (int h = 0; h < hops; h += kB, t += static_cast<size_t>(kB) * pb.D) {
+      uint32_t en[kB];
+#pragma unroll
+      for (int i = 0; i < kB; ++i) en[i] = h + i < hops ? __ldg(t + static_cast<size_t>(i) * pb.D) : 0u;
+#pragma unroll
+      for (int i = 0; i < kB; ++i)
+        if (h + i < hops) {
+          const uint32_t at = en[i] >> 21, m = (at * 1986u) >> 16;  // 33 m + q
+          f.Krow = K + 32 * m;
+          f.hop(0, static_cast<int>(at - 33 * m), en[i] & 0x1fffffu);
+        }
+    }
+  } else {
+    const uint32_t Dm1 = pb.D - 1, R = Dm1 - r;
+    const uint32_t M = dev::colex_unrank<kBinomCols>(R, pb.L, pb.N, B);
+    dev::Neighbours<NH, kBinomCols> nb;
+    nb.precompute(M, R, pb.L, pb.nh, B);
+    nb.visit(M, R, Dm1, pb.N, pb.nh, B, f);
+  }
 #pragma unroll
   for (int v = 0; v < kMaxR; ++v)
     if (v < nv) y[static_cast<size_t>(v) * pb.D + r] = f.acc[v];
@@ -1059,6 +1078,7 @@ int engine_tune(doci_ham *h, int nv, int *dpt_out) {
   pb.L = h->L;
   pb.N = h->N;
   pb.nh = h->nh;
+  pb.nbr = h->d_nbr;
   pb.K = h->d_Kmir32;
   pb.diag_s = h->d_diag32;
   pb.diag = h->d_diag;
@@ -1137,7 +1157,8 @@ int64_t engine_footprint(int L, int N, const doci_batch_opts &o) {
   const int64_t D = static_cast<int64_t>(binom64(L, N));
   const int64_t R = std::max(1, std::min(o.nroots, kMaxR));
   const int64_t mv = std::min(kMaxV, std::max(o.max_vec, 2 * o.nroots));
-  const int64_t ham = D * 12 + (16ll << 20);  // the handle's diagonals and tables
+  // the handle's diagonals and tables
+  const int64_t ham = D * 12 + (16ll << 20) + static_cast<int64_t>(nbr_table_bytes(L, N, D));
   const int64_t x = D * R * 8;                 // Ritz vectors
   const int64_t p64 = 2 * mv * D * 8 + R * D * 8 + 2 * R * D * 8;  // + staging of a large problem
   const int64_t p32 = o.mode == DOCI_MODE_MIXED ? 2 * mv * D * 4 + R * D * 4 + D * 4 + 2 * R * D * 4 : 0;
@@ -1215,6 +1236,7 @@ int engine_solve(int n, doci_ham *const *hams, const doci_batch_opts &o, cudaStr
       pb.L = h->L;
       pb.N = h->N;
       pb.nh = h->nh;
+      pb.nbr = h->d_nbr;
       pb.diag = h->d_diag;
       pb.V = static_cast<char *>(V) + off * a.maxv * elem;
       pb.VA = static_cast<char *>(VA) + off * a.maxv * elem;

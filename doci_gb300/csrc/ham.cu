@@ -70,7 +70,7 @@ void ham_release(doci_ham *h) {
   cudaStream_t st = h->stream;
   void *bufs[] = {h->d_binom, h->d_Kmir64, h->d_Kmir32, h->d_tab64, h->d_diag, h->d_diag32, h->d_stage_x,
                   h->d_stage_y, h->d_rows, h->d_rowstart, h->d_pblocks, h->d_pblocks_host, h->d_kfrag, h->d_tc_err,
-                  h->d_wstart, h->d_wunits, h->d_kdig};  // d_rem/d_ins/d_ins_t/d_tab_off are shared (per-process cache)
+                  h->d_wstart, h->d_wunits, h->d_kdig, h->d_nbr};  // d_rem/d_ins/d_ins_t/d_tab_off are shared (per-process cache)
   for (void *p : bufs) release_async(p, st);
   if (h->h_diag) cudaFreeHost(h->h_diag);
   if (st) {
@@ -111,6 +111,7 @@ void ham_release(doci_ham *h) {
   h->d_kfrag = nullptr;
   h->d_wstart = h->d_wunits = nullptr;
   h->d_kdig = nullptr;
+  h->d_nbr = nullptr;
   h->d_wtab_a = h->d_wtab_b = nullptr;
   h->wsplit = 0;
   h->d_tc_err = nullptr;
@@ -215,6 +216,8 @@ int ham_build(doci_ham *h, const Integrals &in) {
   st = ham_build_rows(h);
   if (st) return st;
   st = ham_build_pair_warp(h);
+  if (st) return st;
+  st = ham_build_nbr(h);
   if (st) return st;
   DOCI_CUDA(cudaStreamSynchronize(h->stream));
   return DOCI_OK;

@@ -95,6 +95,9 @@ struct doci_ham {
   // size j at tab_off[j] + 4 (q C(split, j) + c)): a warp's 16-byte loads of
   // one quad are consecutive (the pair kernels)
   uint32_t *d_ins_t = nullptr;
+  // small spaces: every neighbour's rank and hop weight (sigma.cu,
+  // nbr_table_kernel); null where the table would be too large
+  uint32_t *d_nbr = nullptr;
   // pair form (sigma_pair.cu): one block per (N-1)-pair set's row part R',
   // {own row start or ~0, mask | k' << 24}, largest first; the K matrix split
   // into TF32 high and low parts (2 x 32 x 32 floats, mirrored orbitals; also
@@ -198,4 +201,7 @@ int launch_bitstrings(const doci_ham *h, int64_t first, int64_t count, uint32_t 
 int launch_ranks(const doci_ham *h, const uint32_t *bits, int64_t count, int64_t *out, cudaStream_t s);
 int launch_diagonal(doci_ham *h, cudaStream_t s);
 int ham_build_rows(doci_ham *h);
+int ham_build_nbr(doci_ham *h);
+// bytes of the neighbour table of an (L, N) handle, 0 when it has none
+size_t nbr_table_bytes(int L, int N, uint64_t D);
 }  // namespace doci

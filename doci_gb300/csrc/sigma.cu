@@ -137,7 +137,11 @@ int launch_nh(const doci_ham *h, const void *x, void *y, cudaStream_t st) {
 }
 
 template <typename Real>
+int launch_nbr(const doci_ham *h, const void *x, size_t ldx, void *y, size_t ldy, int nv, cudaStream_t st);
+
+template <typename Real>
 int launch_typed(const doci_ham *h, const void *x, void *y, cudaStream_t st) {
+  if (h->d_nbr) return launch_nbr<Real>(h, x, 0, y, 0, 1, st);
   const int nh = h->nh;
   if (nh <= 4) return launch_nh<Real, 4>(h, x, y, st);
   if (nh <= 8) return launch_nh<Real, 8>(h, x, y, st);
@@ -147,6 +151,115 @@ int launch_typed(const doci_ham *h, const void *x, void *y, cudaStream_t st) {
   if (nh <= 24) return launch_nh<Real, 24>(h, x, y, st);
   if (nh <= 28) return launch_nh<Real, 28>(h, x, y, st);
   return launch_nh<Real, 32>(h, x, y, st);
+}
+
+// ---------------------------------------------------------------------------
+// Small spaces: the ranks of all N (L - N) neighbours of every determinant, with
+// the hop's place in K, are laid out once per handle, hop by hop (entry of hop
+// t and determinant r at t D + r: rank | (33 m + q) << 21; rows of 33, so that
+// lanes at the same hole and different pairs are in different banks), so that
+// a sigma is one pass of independent coalesced entry loads and gathers.
+// Unranking and the neighbour ranks' dependent steps were most of a small
+// sigma.  The hops are summed before diag x is added (in two sums, even and
+// odd hops), which keeps their rounding errors at their own size.
+// Measured per call against the gather kernel and the pair form (us): FP64
+// 1,287 determinants 7.8 (what a call costs the host) against 10.5; 12,870 8.5
+// against 13.7; 48,620 14.6 against 26.8 / 22.3; 92,378 24.7 against 33.0 /
+// 27.0.  FP32 12,870 8.5 against 12.5 / 16.6; 48,620 12.4 against 16.5 / 16.6;
+// 92,378 16.6 against 18.6 / 16.8.  The table is at most 32 MiB: from there on
+// the pair form is the faster.  Error against 64 bits in FP32 3.5e-8 to 4e-8
+// (gather kernel 1.4e-7 to 2.5e-7, pair form 6.6e-8 to 8.8e-8), in FP64 against
+// 128-bit sums 4.5e-17 to 1.3e-16 (gather kernel 1.5e-16 to 4e-15).
+// ---------------------------------------------------------------------------
+constexpr size_t kNbrMaxEntries = size_t(1) << 23;  // 32 MiB
+
+__global__ void __launch_bounds__(kThreads)
+nbr_table_kernel(SigmaShape s, const uint32_t *__restrict__ g_binom, uint32_t *__restrict__ out) {
+  __shared__ uint32_t B[kBinomRows * kBinomCols];
+  for (int t = threadIdx.x; t < kBinomRows * kBinomCols; t += blockDim.x) B[t] = g_binom[t];
+  __syncthreads();
+  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < s.D; r += gridDim.x * blockDim.x) {
+    const uint32_t R = s.D - 1 - r, M = dev::colex_unrank<kBinomCols>(R, s.L, s.N, B);
+    dev::Neighbours<32, kBinomCols> nb;
+    nb.precompute(M, R, s.L, s.nh, B);
+    struct Put {
+      uint32_t *p;
+      uint32_t D;
+      __device__ __forceinline__ void begin(int) {}
+      __device__ __forceinline__ void hop(int m, int q, uint32_t idx) {
+        *p = idx | static_cast<uint32_t>(33 * m + q) << 21;
+        p += D;
+      }
+    } f{out + r, s.D};
+    nb.visit(M, R, s.D - 1, s.N, s.nh, B, f);
+  }
+}
+
+// one determinant per thread and NV vectors (x_v = x + v ldx, y_v = y + v ldy, v < nv <= NV)
+template <typename Real, int NV>
+__global__ void __launch_bounds__(kThreads)
+sigma_nbr_kernel(uint32_t D, int L, int hops, const uint32_t *__restrict__ nbr, const Real *__restrict__ g_K,
+                 const Real *__restrict__ diag, const Real *__restrict__ x, size_t ldx, Real *__restrict__ y,
+                 size_t ldy, int nv) {
+  __shared__ Real K[32 * 33];
+  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x, rr = r < D ? r : D - 1;
+  constexpr int kB = NV == 1 ? 16 : 8;  // hops whose loads are in flight together
+  uint32_t e[kB];
+  const uint32_t *p = nbr + rr;
+#pragma unroll
+  for (int i = 0; i < kB; ++i) e[i] = i < hops ? __ldg(p + static_cast<size_t>(i) * D) : 0u;
+  for (int t = threadIdx.x; t < 32 * L; t += blockDim.x) K[t + (t >> 5)] = g_K[t];
+  const Real d = diag[rr];
+  Real acc[2][NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) acc[0][v] = acc[1][v] = Real(0);
+  __syncthreads();
+  for (int t = 0; t < hops; t += kB) {
+    uint32_t c[kB];
+#pragma unroll
+    for (int i = 0; i < kB; ++i) {
+      c[i] = e[i];
+      e[i] = t + kB + i < hops ? __ldg(p + static_cast<size_t>(t + kB + i) * D) : 0u;
+    }
+    Real xv[kB][NV];
+#pragma unroll
+    for (int i = 0; i < kB; ++i)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) xv[i][v] = (t + i < hops && v < nv) ? __ldg(x + v * ldx + (c[i] & 0x1fffffu)) : Real(0);
+#pragma unroll
+    for (int i = 0; i < kB; ++i)
+      if (t + i < hops) {
+        const Real kv = K[c[i] >> 21];
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+          if (v < nv) acc[i & 1][v] += kv * xv[i][v];
+      }
+  }
+  if (r < D) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+      if (v < nv) y[v * ldy + r] = d * x[v * ldx + r] + (acc[0][v] + acc[1][v]);
+  }
+}
+
+template <typename Real>
+int launch_nbr(const doci_ham *h, const void *x, size_t ldx, void *y, size_t ldy, int nv, cudaStream_t st) {
+  const Real *K = std::is_same<Real, double>::value ? reinterpret_cast<const Real *>(h->d_Kmir64)
+                                                   : reinterpret_cast<const Real *>(h->d_Kmir32);
+  const Real *dg = std::is_same<Real, double>::value ? reinterpret_cast<const Real *>(h->d_diag)
+                                                    : reinterpret_cast<const Real *>(h->d_diag32);
+  // small blocks while they leave SMs idle
+  const int threads = h->D <= 64u * device_sm_count() ? 64 : h->D <= 512u * device_sm_count() ? 128 : 256;
+  const unsigned grid = (h->D + threads - 1) / threads;
+  const int hops = h->N * h->nh;
+  const Real *xr = static_cast<const Real *>(x);
+  Real *yr = static_cast<Real *>(y);
+  if (nv == 1)
+    sigma_nbr_kernel<Real, 1><<<grid, threads, 0, st>>>(h->D, h->L, hops, h->d_nbr, K, dg, xr, ldx, yr, ldy, 1);
+  else
+    sigma_nbr_kernel<Real, 4><<<grid, threads, 0, st>>>(h->D, h->L, hops, h->d_nbr, K, dg, xr, ldx, yr, ldy, nv);
+  DOCI_CUDA(cudaGetLastError());
+  return DOCI_OK;
 }
 
 // Several vectors at once (block methods): x_v = x + v ldx, y_v = y + v ldy,
@@ -215,6 +328,7 @@ int launch_gather_multi(const doci_ham *h, const void *x, size_t ldx, void *y, s
 template <typename Real>
 int launch_gather_multi_typed(const doci_ham *h, const void *x, size_t ldx, void *y, size_t ldy, int nv,
                               cudaStream_t st) {
+  if (h->d_nbr) return launch_nbr<Real>(h, x, ldx, y, ldy, nv, st);
   const int nh = h->nh;
   if (nh <= 8) return launch_gather_multi<Real, 8>(h, x, ldx, y, ldy, nv, st);
   if (nh <= 16) return launch_gather_multi<Real, 16>(h, x, ldx, y, ldy, nv, st);
@@ -832,12 +946,6 @@ int tuned_choice(const doci_ham *h, int precision, int nv, bool allow_pair) {
   return it == g_tuned.end() ? 0 : it->second;
 }
 
-// Below this many determinants the automatic choice is the gather kernel: one
-// launch, and nothing to set up per unit.  Measured (us, gather / pair form):
-// FP32 12,870 determinants 13.0 / 16.7, 24,310 15.0 / 16.6, 48,620 16.8 / 16.8;
-// FP64 12,870 14.1 / 21.3, 24,310 20.9 / 21.4, 48,620 27.1 / 22.1; the row
-// passes are slower than both (14.8 and 23 us at the first two in FP32).
-constexpr uint32_t kGatherMaxD = 1u << 15;
 // the FP64 pair form is a candidate of the autotuning from here on
 constexpr uint32_t kTunedPairMinD = 1u << 18;
 
@@ -852,7 +960,7 @@ SigmaPlan plan_kind(const doci_ham *h, int precision, bool allow_pair, int kind)
     // pair form: the automatic FP32 choice where it fits and the space gives
     // every SM work
     const bool want_pair =
-        kind == 6 || kind == 8 || (kind == 0 && h->npblocks >= device_sm_count() && h->D >= kGatherMaxD);
+        kind == 6 || kind == 8 || (kind == 0 && !h->d_nbr && h->npblocks >= device_sm_count());
     if (want_pair && pair_fits(h)) return {6, 2};  // zero (or diag x) pass + pair pass
   }
   // float-float sigma (FP64 accuracy in FP32 arithmetic): the pair form, or
@@ -862,11 +970,12 @@ SigmaPlan plan_kind(const doci_ham *h, int precision, bool allow_pair, int kind)
     return {9, 2};
   // the automatic FP64 choice where the pair tiling gives every SM work: the
   // FP64-accurate pair form (L=32, N=16: 53.7 ms; the row pass 444.9 ms)
-  if (kind == 0 && allow_pair && precision == DOCI_FP64 && h->npblocks >= device_sm_count() &&
-      h->D >= kGatherMaxD && pair_ff_fits(h))
+  if (kind == 0 && !h->d_nbr && allow_pair && precision == DOCI_FP64 && h->npblocks >= device_sm_count() &&
+      pair_ff_fits(h))
     return {9, 2};
   // row kernel when the row tiling exists, fits, and gives every SM work
-  bool row = kind >= 3 || (kind == 0 && h->nrows >= device_sm_count() && h->D >= kGatherMaxD);
+  // (small spaces have their neighbour table: the gather kernel reads it)
+  bool row = kind >= 3 || (kind == 0 && !h->d_nbr && h->nrows >= device_sm_count());
   if (row && !row_kernel_fits(h, elem)) row = false;
   if (!row) return {1, 1};
   // automatic: the phase-ordered pass for FP64 (measured faster there), the
@@ -945,6 +1054,7 @@ int multi_row_group(const doci_ham *h, size_t elem) {
 
 int multi_method_auto(const doci_ham *h, int precision) {
   const size_t elem = precision == DOCI_FP64 ? 8 : 4;
+  if (h->d_nbr && h->sigma_kernel == 0) return kMultiGather;
   // same choice of family as the single-vector dispatch
   const bool want_row = h->sigma_kernel >= 2 || (h->sigma_kernel == 0 && h->nrows >= device_sm_count());
   if (want_row && multi_row_group(h, elem) >= 2) return kMultiRow;
@@ -957,12 +1067,11 @@ int multi_method_auto(const doci_ham *h, int precision) {
 // order, up to kDetMaxBytes of scratch (40.1M determinants in FP64: 4.2 GiB).
 // Measured against the multi-vector row and gather kernels (us, nv = 2 / 4):
 // FP32 L=24 N=12 1,256 / 1,455 -> 247 / 490; L=20 N=10 140 / 155 -> 52 / 101;
-// L=18 N=9 72 / 79 -> 44 / 81, so from 2^16 determinants for three vectors or
-// more, 2^15 for fewer.  FP64 L=24 2,915 / 3,113 -> 725 / 1,444; L=18 102 / 110
-// -> 64 / 125.
+// FP64 L=24 2,915 / 3,113 -> 725 / 1,444.  (Spaces with a neighbour table take
+// the gather kernel.)
 constexpr size_t kDetMaxBytes = size_t(5) << 30;
-bool det_fits(const doci_ham *h, size_t elem, int nv) {
-  return h->sigma_kernel == 0 && pair_warp_fits(h) && h->D >= (nv >= 3 ? 1u << 16 : 1u << 15) &&
+bool det_fits(const doci_ham *h, size_t elem) {
+  return h->sigma_kernel == 0 && !h->d_nbr && pair_warp_fits(h) &&
          static_cast<size_t>(pair_warp_slabs(h)) * h->D * elem <= kDetMaxBytes;
 }
 // *done = false: there is no memory for the scratch
@@ -1013,7 +1122,7 @@ int run_multi(const doci_ham *h, int method, const void *x, size_t ldx, void *y,
   if (method == kMultiGather)
     return precision == DOCI_FP64 ? launch_gather_multi_typed<double>(h, x, ldx, y, ldy, nv, st)
                                   : launch_gather_multi_typed<float>(h, x, ldx, y, ldy, nv, st);
-  if (det_fits(h, elem, nv)) {
+  if (det_fits(h, elem)) {
     bool done;
     const int r = run_det(h, xc, ldx, yc, ldy, nv, precision, st, &done);
     if (done || r != DOCI_OK) return r;
@@ -1033,7 +1142,7 @@ int launch_sigma_multi(const doci_ham *h, const void *x, size_t ldx, void *y, si
   if (precision != DOCI_FP64 && precision != DOCI_FP32) return DOCI_ERR_INVALID;
   // block sigmas are reproducible from run to run: no atomic adds here
   int method = h->sigma_kernel == 0 ? tuned_choice(h, precision, nv, false) : 0;
-  if (method == 0 && det_fits(h, precision == DOCI_FP64 ? 8 : 4, nv)) {
+  if (method == 0 && det_fits(h, precision == DOCI_FP64 ? 8 : 4)) {
     bool done;
     const int r = run_det(h, static_cast<const char *>(x), ldx, static_cast<char *>(y), ldy, nv, precision, st, &done);
     if (done || r != DOCI_OK) return r;
@@ -1119,6 +1228,21 @@ int autotune_sigma(doci_ham *h, int precision, int nv, cudaStream_t st, int *cho
 }
 
 bool sigma_tuned(const doci_ham *h, int precision, int nv) { return tuned_choice(h, precision, nv, false) != 0; }
+
+size_t nbr_table_bytes(int L, int N, uint64_t D) {
+  const uint64_t n = D * static_cast<uint64_t>(N) * static_cast<uint64_t>(L - N);
+  return n > 0 && n <= kNbrMaxEntries && D < (1u << 21) ? n * sizeof(uint32_t) : 0;
+}
+
+int ham_build_nbr(doci_ham *h) {
+  const size_t bytes = nbr_table_bytes(h->L, h->N, h->D);
+  if (bytes == 0) return DOCI_OK;
+  DOCI_CUDA(cudaMallocAsync(&h->d_nbr, bytes, h->stream));
+  nbr_table_kernel<<<grid_for(h->D), kThreads, 0, h->stream>>>(SigmaShape{h->D, h->L, h->N, h->nh}, h->d_binom,
+                                                               h->d_nbr);
+  DOCI_CUDA(cudaGetLastError());
+  return DOCI_OK;
+}
 
 int launch_diagonal(doci_ham *h, cudaStream_t st) {
   const SigmaShape s{h->D, h->L, h->N, h->nh};

@@ -173,11 +173,12 @@ int doci_sigma(doci_ham *ham, const void *d_x, void *d_y, int precision, void *s
 int doci_sigma_block(doci_ham *ham, const void *d_X, int64_t ldx, void *d_Y, int64_t ldy, int nv, int precision,
                      void *stream);
 
-/* Sigma kernel selection for a handle: 0 automatic (default: from 2^15
- * determinants on, with a row tiling that gives every SM work, kind 6 for
- * FP32 and kind 9 for FP64, or where these do not apply kind 3 for FP32 and
- * kind 4 for FP64; else kind 1),
- * 1 the per-determinant gather kernel, 3 the row pass doing all hops, 4 the
+/* Sigma kernel selection for a handle: 0 automatic (default: kind 1 on small
+ * spaces, where the handle holds a table of every determinant's neighbours (D
+ * N (L - N) entries of 4 bytes, at most 32 MiB); on larger ones, with a row
+ * tiling that gives every SM work, kind 6 for FP32 and kind 9 for FP64, or
+ * where these do not apply kind 3 for FP32 and kind 4 for FP64; else kind 1),
+ * 1 the per-determinant gather kernel (from the table on small spaces), 3 the row pass doing all hops, 4 the
  * phase-ordered row pass (cross hops staged one source row at a time), 6 the
  * (N-1)-pair form (FP32 only: gather the neighbours of every (N-1)-pair set,
  * multiply by K on the tensor cores, scatter; from 10 orbitals on one warp per

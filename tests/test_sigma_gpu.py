@@ -481,3 +481,31 @@ def test_sigma_block_reproducible(L, N, seed, nv, synth, dg):
             assert torch.equal(outs[0], outs[1])
             for v in range(nv):
                 assert np.abs(outs[0][v].double().cpu().numpy() - refs[v]).max() <= tol * np.abs(refs[v]).max()
+
+
+@pytest.mark.parametrize("L,N,seed,nv", [(1, 1, 121, 1), (2, 1, 122, 2), (3, 1, 123, 4), (7, 6, 124, 3), (9, 4, 125, 5),
+                                         (13, 5, 126, 2), (32, 1, 127, 3), (32, 31, 128, 4), (32, 3, 129, 2),
+                                         (19, 9, 130, 1), (20, 7, 131, 4)])
+def test_sigma_neighbour_table(L, N, seed, nv, synth, dg):
+    """The gather kernel from the neighbour table (small spaces, the automatic
+    choice there), on spaces of one determinant up to nearly the largest with
+    a table (92,378 determinants of 90 hops): the oracle's matvec, single and block calls bit for bit alike, y
+    written nowhere else."""
+    torch = torch_cuda()
+    p = synth(L, N, seed)
+    o = oracle.Ham(p)
+    with dg.Hamiltonian.from_fcidump(p) as h:
+        D = h.D
+        X = np.random.default_rng(seed).standard_normal((nv, D))
+        for prec, dt, tol in ((dg.FP64, torch.float64, TOL64), (dg.FP32, torch.float32, TOL32)):
+            assert h.sigma_plan(prec) == (1, 1)
+            xb = torch.from_numpy(X).to(dt).cuda()
+            yb = torch.full((nv, D + 3), 7.0, dtype=dt, device="cuda")
+            h.sigma_block_device(xb.data_ptr(), D, yb.data_ptr(), D + 3, nv, prec)
+            y1 = torch.full((D + 3,), 7.0, dtype=dt, device="cuda")
+            for v in range(nv):
+                h.sigma_device(xb[v].data_ptr(), y1.data_ptr(), prec)
+                torch.cuda.synchronize()
+                ref = o.matvec(X[v])
+                assert torch.equal(y1[:D], yb[v, :D]) and bool((yb[v, D:] == 7.0).all() and (y1[D:] == 7.0).all())
+                assert np.abs(y1[:D].double().cpu().numpy() - ref).max() <= tol * max(np.abs(ref).max(), 1e-300)
