@@ -380,29 +380,35 @@ int ham_build_pairs(doci_ham *h, const std::vector<uint32_t> &start) {
     flat.push_back(e.second.second);
   }
   h->npblocks = static_cast<int>(bl.size());
-  // host-buffer path: pieces of the vector, units by the pieces their rows
-  // reach, the group schedule and its launch steps (host_plan.h)
-  hostplan::pieces(h->D, h->chunk_off);
-  std::vector<hostplan::Unit> hu;
-  hu.reserve(bl.size());
-  for (auto &e : bl) {
-    const uint32_t mask = e.second.second & 0xffffffu;
-    const int kp = static_cast<int>(e.second.second >> 24), jp = N - 1 - kp;
-    uint32_t touched = 0;
-    if (e.second.first != kNone) touched |= hostplan::row_pieces(h->chunk_off, e.second.first, binom64(sp, jp + 1));
-    for (int b = 0; b < na; ++b)
-      if (!(mask >> b & 1u)) touched |= hostplan::row_pieces(h->chunk_off, start[mask | (1u << b)], binom64(sp, jp));
-    hu.push_back({e.second.first, e.second.second, binom64(sp, jp), touched});
-  }
+  // host-buffer path, for the spaces that it overlaps: pieces of the vector,
+  // units by the pieces their rows reach, the group schedule and its launch
+  // steps (host_plan.h).  The search for the schedule is serial host work, 6.3
+  // of a Hamiltonian's 8.7 ms at 2.7M determinants, so nobody else pays for it.
   std::vector<uint32_t> flat_host;
-  hostplan::schedule(hu, h->D, h->host_groups, flat_host);
-  h->host_steps = hostplan::steps(h->host_groups);
+  if (h->D >= kHostOverlapMinD) {
+    hostplan::pieces(h->D, h->chunk_off);
+    std::vector<hostplan::Unit> hu;
+    hu.reserve(bl.size());
+    for (auto &e : bl) {
+      const uint32_t mask = e.second.second & 0xffffffu;
+      const int kp = static_cast<int>(e.second.second >> 24), jp = N - 1 - kp;
+      uint32_t touched = 0;
+      if (e.second.first != kNone) touched |= hostplan::row_pieces(h->chunk_off, e.second.first, binom64(sp, jp + 1));
+      for (int b = 0; b < na; ++b)
+        if (!(mask >> b & 1u)) touched |= hostplan::row_pieces(h->chunk_off, start[mask | (1u << b)], binom64(sp, jp));
+      hu.push_back({e.second.first, e.second.second, binom64(sp, jp), touched});
+    }
+    hostplan::schedule(hu, h->D, h->host_groups, flat_host);
+    h->host_steps = hostplan::steps(h->host_groups);
+  }
   DOCI_CUDA(cudaMallocAsync(&h->d_kfrag, ks.size() * sizeof(float), h->stream));
   DOCI_CUDA(cudaMemcpyAsync(h->d_kfrag, ks.data(), ks.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
   if (!flat.empty()) {
     DOCI_CUDA(cudaMallocAsync(&h->d_pblocks, flat.size() * sizeof(uint32_t), h->stream));
     DOCI_CUDA(cudaMemcpyAsync(h->d_pblocks, flat.data(), flat.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
                               h->stream));
+  }
+  if (!flat_host.empty()) {
     DOCI_CUDA(cudaMallocAsync(&h->d_pblocks_host, flat_host.size() * sizeof(uint32_t), h->stream));
     DOCI_CUDA(cudaMemcpyAsync(h->d_pblocks_host, flat_host.data(), flat_host.size() * sizeof(uint32_t),
                               cudaMemcpyHostToDevice, h->stream));
