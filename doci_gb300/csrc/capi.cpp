@@ -471,6 +471,7 @@ int doci_solve_trace(doci_ham *h, const doci_solve_opts *opts, double *vec, doci
       op32.n = D;
       op32.enable_timing();
       s = davidson_run<float>(op32, D, h->d_diag, static_cast<float *>(t32.p), a32, st, &out, d_x);
+      op32.collect_time();
       op.sigma_seconds += op32.sigma_seconds;
       if (s) return s;
       res->iterations_fp32 = out.iterations;
@@ -554,6 +555,7 @@ int doci_solve_trace(doci_ham *h, const doci_solve_opts *opts, double *vec, doci
     return DOCI_ERR_UNKNOWN_SOLVER;
   }
   res->seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+  op.collect_time();
   res->sigma_seconds = op.sigma_seconds;
   if (vec) DOCI_CUDA(cudaMemcpyAsync(vec, d_x, sizeof(double) * D, cudaMemcpyDeviceToHost, st));
   DOCI_CUDA(cudaStreamSynchronize(st));

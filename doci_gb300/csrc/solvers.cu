@@ -80,6 +80,7 @@ ShiftedView::~ShiftedView() {
 
 int MatvecOp::apply(const void *d_x, void *d_y, int precision, cudaStream_t st) {
   if (ham) {
+    collect_time();
     if (events_on) cudaEventRecord(ev0, st);
     int s;
     if (ham32 && precision == DOCI_FP64 && !anchor_next) {
@@ -95,10 +96,7 @@ int MatvecOp::apply(const void *d_x, void *d_y, int precision, cudaStream_t st) 
     anchor_next = false;
     if (events_on) {
       cudaEventRecord(ev1, st);
-      cudaEventSynchronize(ev1);
-      float ms = 0;
-      cudaEventElapsedTime(&ms, ev0, ev1);
-      sigma_seconds += ms * 1e-3;
+      timed = true;
     }
     return s;
   }
@@ -111,6 +109,14 @@ int MatvecOp::apply(const void *d_x, void *d_y, int precision, cudaStream_t st) 
   DOCI_CUDA(cudaMemcpyAsync(d_y, hy.data(), n * sizeof(double), cudaMemcpyHostToDevice, st));
   DOCI_CUDA(cudaStreamSynchronize(st));
   return DOCI_OK;
+}
+
+void MatvecOp::collect_time() {
+  if (!timed) return;
+  float ms = 0;
+  if (cudaEventSynchronize(ev1) == cudaSuccess && cudaEventElapsedTime(&ms, ev0, ev1) == cudaSuccess)
+    sigma_seconds += ms * 1e-3;
+  timed = false;
 }
 
 void MatvecOp::enable_timing() {
@@ -194,6 +200,13 @@ int davidson_run(MatvecOp &op, size_t D, const double *d_diag, S *d_t, const Dav
       // Kaufman-Stewart criterion); the residual pass already gave V^T t
       DOCI_CUDA(cudaMemcpyAsync(d_vec, c.data(), sizeof(double) * m, cudaMemcpyHostToDevice, st));
       DOCI_TRY(vec_gs_finish<S>(Vp, D, m, d_vec, 1.0 / std::sqrt(t_norm2 - proj2), D, d_t, Vm, dp, st, mixed_sigmas));
+    } else if (sizeof(S) == 8 && !mixed_sigmas) {
+      // both passes take their coefficients from the device's results of the
+      // pass before: V^T t lies behind ||r||^2 and ||t||^2
+      if constexpr (sizeof(S) == 8) {
+        DOCI_TRY(vec_gs_update<S>(Vp, D, m, vec_results(dp) + 2, D, d_t, dp, st));
+        DOCI_TRY(vec_gs_finish_sums(Vp, D, m, dp, D, d_t, Vm, st));
+      }
     } else {
       DOCI_CUDA(cudaMemcpyAsync(d_vec, c.data(), sizeof(double) * m, cudaMemcpyHostToDevice, st));
       DOCI_TRY(vec_gs_update<S>(Vp, D, m, d_vec, D, d_t, dp, st, mixed_sigmas));

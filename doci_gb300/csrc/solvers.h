@@ -18,8 +18,8 @@ struct MatvecOp {
   void *host_dat = nullptr;
   size_t n = 0;
   std::vector<double> hx, hy;
-  double sigma_seconds = 0;
-  bool events_on = false;
+  double sigma_seconds = 0;  // of the sigmas up to the last collect_time()
+  bool events_on = false, timed = false;
   cudaEvent_t ev0{}, ev1{};
   // FP64 phase of the mixed mode: the first FP64 sigma after `anchor_next`
   // is a true FP64 sigma (the anchor vector); the later ones (correction
@@ -37,6 +37,9 @@ struct MatvecOp {
   bool anchor_next = true;
   int apply(const void *d_x, void *d_y, int precision, cudaStream_t st);
   void enable_timing();
+  // adds the last sigma's time, waiting for it if it still runs (apply calls it
+  // for the sigma before, which the solver has waited for)
+  void collect_time();
   ~MatvecOp();
 };
 

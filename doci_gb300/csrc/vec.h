@@ -43,6 +43,9 @@ int vec_gs_update(const S *V, size_t ld, int m, const double *c, size_t n, S *t,
 template <typename S>
 int vec_gs_finish(const S *V, size_t ld, int m, const double *c, double scale, size_t n, const S *t, S *out,
                   double *partials, cudaStream_t st, bool mixed = false);
+// the same, with c and the norm from the results of vec_gs_update on `partials`
+int vec_gs_finish_sums(const double *V, size_t ld, int m, const double *partials, size_t n, const double *t, double *out,
+                       cudaStream_t st);
 template <typename S>
 int vec_deflate(S *V, size_t ld, int mv, int keep, const double *Y, int ldy, size_t n, cudaStream_t st);
 template <typename S>

@@ -71,3 +71,43 @@ def test_multidot_f32_exact_products(n, m):
         assert L.doci_multidot(V.data_ptr(), n, m, w.data_ptr(), n, 1, out.data_ptr(), None) == 0
         exact = (V.double() * w.double()).sum(1)
         assert torch.equal(torch.isnan(out), torch.isnan(exact)) and torch.equal(torch.isinf(out), torch.isinf(exact))
+
+
+@pytest.mark.parametrize("n,m", [(1, 1), (33, 3), (1023, 4), (1025, 5), (4097, 32), (155649, 17), (319770, 16),
+                                 (622593, 2)])
+def test_multidot_fp64_grid_edges(n, m):
+    """FP64 columns at the edges of the grid (one block, one more than a block's
+    four elements per thread, more elements than one wave takes at once): the
+    sums to n roundings of the sum of magnitudes."""
+    import torch
+    import doci_gb300
+    g = torch.Generator(device="cuda").manual_seed(n + m)
+    V = torch.randn(m, n, device="cuda", generator=g, dtype=torch.float64)
+    w = torch.randn(n, device="cuda", generator=g, dtype=torch.float64)
+    out = torch.empty(m, dtype=torch.float64, device="cuda")
+    assert doci_gb300.lib().doci_multidot(V.data_ptr(), n, m, w.data_ptr(), n, 0, out.data_ptr(), None) == 0
+    prod = V * w
+    assert bool(((out - prod.sum(1)).abs() <= 2 * n * 2.0 ** -53 * prod.abs().sum(1)).all())
+
+
+@pytest.mark.parametrize("L,N,max_vec", [(1, 1, 2), (3, 1, 9), (8, 4, 2), (8, 4, 8), (10, 5, 9), (10, 4, 16),
+                                         (10, 5, 17), (12, 6, 32)])
+def test_fp64_davidson_basis_sizes(L, N, max_vec, synth):
+    """FP64 Davidson with bases at the edges of its passes' column counts (8, 16,
+    32) on spaces of less than a warp to several blocks: a normalised vector
+    whose residual, formed by the oracle, is the reported one, and the energy
+    of an eigenvalue.  Residuals below 1e-10 bound the energy's error; the
+    oracle's own sums are good to about 1e-12 here."""
+    import doci_gb300 as dg
+    import oracle
+    p = synth(L, N, 300 + L + max_vec)
+    o = oracle.Ham(p)
+    with dg.Hamiltonian.from_fcidump(p) as h:
+        H = np.stack([np.asarray(o.matvec(e)) for e in np.eye(h.D)])
+        res, v = h.solve(solver="D", mode="fp64", tol=1e-10, max_its=400, davidson_max_vec=max_vec,
+                          davidson_keep=1)
+    v = np.asarray(v)
+    e = res["energy"]
+    assert res["converged"] and abs(np.linalg.norm(v) - 1) < 1e-12
+    assert np.linalg.norm(H @ v - (v @ H @ v) * v) < 1e-9
+    assert np.abs(np.linalg.eigvalsh(H) - e).min() < 1e-9
