@@ -627,40 +627,97 @@ __global__ void eng_init_state(EArgs a) {
 // part is below 1e-30 of the whole; ascending eigenvalues; then the restart
 // decision.
 //
-// One thread computes each rotation, all threads apply them, first to the
-// columns of A and of the eigenvectors, then to the rows of A.  The FP64 units
-// (two lanes per clock and SM) and the latency of FP64 divisions and square
-// roots bound it: the tangent, which only steers the convergence, is computed
-// in FP32 from FP64 differences, the cosine in FP64 (an FP32 reciprocal square
-// root and two Newton steps), so that the rotations stay orthogonal to FP64
-// accuracy; and a pair whose square is below 1e-34 of the whole, which cannot
-// keep the off-diagonal part above its limit, is left alone.  Measured on 12
-// problems of up to 32 vectors (average over a solve): 1,609 us with one warp
-// and FP64 tangents, 468 us so.
+// The FP64 units (two lanes per clock and SM) bound it, so most of the way is
+// gone in FP32: Jacobi on the matrix rounded to FP32, its vectors V made
+// orthogonal to FP64 accuracy (with V^T V = 1 + E, E about 1e-6, V (1 - E/2 +
+// 3 E^2 / 8) is orthogonal to E^3), and the FP64 Jacobi then starts from V^T A V,
+// whose off-diagonal part is about 1e-6 of the whole: two sweeps instead of six
+// or seven, with fewer FP64 roundings than those (vectors orthogonal to 5e-15
+// instead of 1e-14 at n = 32).  A round rotates the 2 x 2 blocks of A, one
+// thread per block of the upper triangle (their columns and rows at once, the
+// mirror written along) while the free warps turn 7/16 of the vectors; then warp
+// 0 computes the next round's rotations while the others turn the rest (so that
+// the SM's four quarters have about the same FP64 work in both steps).  A rotation's tangent, which only steers the
+// convergence, is computed in FP32 from differences in the matrix's type, the
+// cosine in that type (an FP32 reciprocal square root and one third-order
+// step for FP64), so that the rotations stay orthogonal to its accuracy; and a
+// pair whose square is below `skip`, which cannot keep the off-diagonal part
+// above its limit, is left alone.
+// Measured on 12 problems of up to 32 vectors (average over a solve): 1,609 us
+// with one warp and FP64 tangents, 468 us with 256 threads in FP64 alone, 198
+// us so.
 constexpr int kEigT = 256;
 constexpr int kLdA = kMaxV + 1;
-__global__ void __launch_bounds__(kEigT) eng_eig(EArgs a) {
-  const int p = blockIdx.x;
-  EState &st = a.St[p];
-  if (st.done) return;
-  __shared__ double A[kMaxV * kLdA], Vv[kMaxV * kLdA];
-  __shared__ double rc[kMaxV / 2], rs[kMaxV / 2], part[2][kEigT / 32];
-  __shared__ int rp[kMaxV / 2], rq[kMaxV / 2];
-  __shared__ double wv[kMaxV];
-  __shared__ int idx[kMaxV];
-  const int n = st.m, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int n2 = n + (n & 1), half = n2 / 2;
-  for (int i = tid; i < kMaxV * kMaxV; i += kEigT) {
-    const int r = i % kMaxV, c = i / kMaxV;
-    A[c * kLdA + r] = (r < n && c < n) ? st.S[i] : 0.0;
-    Vv[c * kLdA + r] = (r == c) ? 1.0 : 0.0;
+constexpr int kHalfV = kMaxV / 2;
+constexpr int kPreMinN = 8;  // below, six FP64 sweeps cost less than the way through FP32
+
+template <typename Real>
+struct Rotations {  // one round's pairs (twice: this round's and the next one's)
+  Real c[2][kHalfV], s[2][kHalfV];
+  int p[2][kHalfV], q[2][kHalfV];
+};
+
+// rotation of pair `k` of a round (n2 = n rounded up to even; with n odd one
+// pair a round is idle)
+template <typename Real>
+__device__ __forceinline__ void eig_rotation(const Real *A, int n, int n2, int round, int k, Real skip,
+                                             Rotations<Real> &rot, int buf) {
+  auto player = [&](int i) {  // i - 1 + round modulo n2 - 1, plus one
+    const int j = i + round;
+    return i == 0 ? 0 : j > n2 - 1 ? j - (n2 - 1) : j;
+  };
+  const int pl = player(k), ql = player(n2 - 1 - k);
+  const int pp = min(pl, ql), qq = max(pl, ql);
+  Real cs = 1, sn = 0;
+  if (qq < n) {
+    const Real apq = A[qq * kLdA + pp];
+    if (apq * apq > skip) {
+      // t = sign(d) b / (|d| + sqrt(d^2 + b^2)), d = aqq - app, b = 2 apq (A is
+      // scaled to about 1 and apq not below `skip`: no under- or overflow)
+      const float d = static_cast<float>(A[qq * kLdA + qq] - A[pp * kLdA + pp]), b = 2 * static_cast<float>(apq);
+      const float h = d * d + b * b, tf = __fdividef(d >= 0 ? b : -b, fabsf(d) + h * rsqrtf(h));
+      const Real t = tf, u = 1 + t * t;
+      Real y = rsqrtf(static_cast<float>(u));
+      if constexpr (sizeof(Real) == 8) {  // y has 22 bits; 1/sqrt(u) = y / sqrt(1 - e), e = 1 - u y^2, to e^3
+        const Real e = 1 - u * (y * y);
+        y += y * (e * (0.5 + 0.375 * e));
+      }
+      cs = y;
+      sn = t * y;
+    }
   }
-  __syncthreads();
-  for (int sweep = 0; sweep < 100 && n > 1; ++sweep) {
+  rot.p[buf][k] = pp;
+  rot.q[buf][k] = qq;
+  rot.c[buf][k] = cs;
+  rot.s[buf][k] = sn;
+}
+
+// sweeps on A (symmetric, full) with the vectors V until the off-diagonal
+// squares are below `stop` of the whole (at most `sweeps`)
+template <typename Real>
+__device__ void eig_jacobi(Real *A, Real *V, int n, Real stop, Real skip_rel, int sweeps, Rotations<Real> &rot,
+                           double (*part)[kEigT / 32]) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n2 = n + (n & 1), half = n2 / 2;
+  int bi = tid, bj = 1;  // this thread's block of the upper triangle (threads 0 to 127)
+  while (bi >= bj && bj < half) bi -= bj++;
+  const bool off_block = tid < half * (half - 1) / 2;
+  auto turn = [&](int b, int first, int step, int end) {  // the vectors by the pairs first, first + step, ...
+    if (lane >= n) return;
+    for (int k = first; k < end; k += step) {
+      const int pp = rot.p[b][k], qq = rot.q[b][k];
+      const Real c = rot.c[b][k], s = rot.s[b][k];
+      if (s == 0) continue;
+      const Real vp = V[pp * kLdA + lane], vq = V[qq * kLdA + lane];
+      V[pp * kLdA + lane] = c * vp - s * vq;
+      V[qq * kLdA + lane] = s * vp + c * vq;
+    }
+  };
+  for (int sweep = 0; sweep < sweeps && n > 1; ++sweep) {
     double off = 0, tot = 0;
     for (int i = tid; i < n * n; i += kEigT) {
       const int r = i % n, c = i / n;
-      const double e = A[c * kLdA + r] * A[c * kLdA + r];
+      const double e = static_cast<double>(A[c * kLdA + r] * A[c * kLdA + r]);
       tot += e;
       if (r != c) off += e;
     }
@@ -679,65 +736,141 @@ __global__ void __launch_bounds__(kEigT) eng_eig(EArgs a) {
       off += part[0][w];
       tot += part[1][w];
     }
-    if (off == 0 || off <= 1e-30 * tot) break;
-    const double skip = 1e-34 * tot;
+    if (off == 0 || off <= stop * tot) break;
+    const Real skip = static_cast<Real>(skip_rel * tot);
+    if (tid < half) eig_rotation<Real>(A, n, n2, 0, tid, skip, rot, 0);
+    __syncthreads();
     for (int round = 0; round < n2 - 1; ++round) {
-      if (tid < half) {
-        auto player = [&](int k) { return k == 0 ? 0 : ((k - 1 + round) % (n2 - 1)) + 1; };
-        int pp = player(tid), qq = player(n2 - 1 - tid);
-        if (pp > qq) {
-          const int t = pp;
-          pp = qq;
-          qq = t;
+      const int b = round & 1;
+      if (off_block) {  // rows (p, q) of pair i, columns (p, q) of pair j
+        const int pi = rot.p[b][bi], qi = rot.q[b][bi], pj = rot.p[b][bj], qj = rot.q[b][bj];
+        const Real ci = rot.c[b][bi], si = rot.s[b][bi], cj = rot.c[b][bj], sj = rot.s[b][bj];
+        if (si != 0 || sj != 0) {
+          const Real a00 = A[pj * kLdA + pi], a01 = A[qj * kLdA + pi], a10 = A[pj * kLdA + qi], a11 = A[qj * kLdA + qi];
+          const Real x0 = cj * a00 - sj * a01, x1 = sj * a00 + cj * a01;
+          const Real y0 = cj * a10 - sj * a11, y1 = sj * a10 + cj * a11;
+          const Real r00 = ci * x0 - si * y0, r10 = si * x0 + ci * y0;
+          const Real r01 = ci * x1 - si * y1, r11 = si * x1 + ci * y1;
+          A[pj * kLdA + pi] = A[pi * kLdA + pj] = r00;
+          A[pj * kLdA + qi] = A[qi * kLdA + pj] = r10;
+          A[qj * kLdA + pi] = A[pi * kLdA + qj] = r01;
+          A[qj * kLdA + qi] = A[qi * kLdA + qj] = r11;
         }
-        double cs = 1.0, sn = 0.0;
-        if (qq < n) {
-          const double apq = A[qq * kLdA + pp];
-          if (apq * apq > skip) {
-            // t = sign(d) b / (|d| + sqrt(d^2 + b^2)), d = aqq - app, b = 2 apq, scaled to the larger
-            const double d = A[qq * kLdA + qq] - A[pp * kLdA + pp], b = 2 * apq;
-            const double big = fabs(d) > fabs(b) ? fabs(d) : fabs(b);
-            const int ex = ilogb(big);
-            const float df = static_cast<float>(scalbn(d, -ex)), bf = static_cast<float>(scalbn(b, -ex));
-            const float tf = (df >= 0 ? bf : -bf) / (fabsf(df) + sqrtf(df * df + bf * bf));
-            const double t = static_cast<double>(tf), u = 1 + t * t;
-            double y = static_cast<double>(rsqrtf(static_cast<float>(u)));
-            y = y * (1.5 - 0.5 * u * y * y);
-            y = y * (1.5 - 0.5 * u * y * y);
-            cs = y;
-            sn = t * y;
-          }
+      } else if (tid >= 128 && tid < 128 + half) {  // a pair's own block: app + e, aqq - e
+        const int k = tid - 128, pp = rot.p[b][k], qq = rot.q[b][k];
+        const Real c = rot.c[b][k], s = rot.s[b][k];
+        if (s != 0) {
+          const Real app = A[pp * kLdA + pp], apq = A[qq * kLdA + pp], aqq = A[qq * kLdA + qq];
+          const Real d = aqq - app, g = c * apq, f = g - s * d, e = -s * (f + g);
+          A[pp * kLdA + pp] = app + e;
+          A[qq * kLdA + pp] = A[pp * kLdA + qq] = c * f - s * (s * apq);
+          A[qq * kLdA + qq] = aqq - e;
         }
-        rp[tid] = pp;
-        rq[tid] = qq;
-        rc[tid] = cs;
-        rs[tid] = sn;
       }
+      const int early = half * 7 / 16;
+      if (warp > 4) turn(b, warp - 5, 3, early);
       __syncthreads();
-      for (int i = warp; i < half; i += kEigT / 32) {  // columns p, q of row `lane`
-        const int pp = rp[i], qq = rq[i];
-        const double cs = rc[i], sn = rs[i];
-        if (sn == 0.0 || lane >= n) continue;
-        const double akp = A[pp * kLdA + lane], akq = A[qq * kLdA + lane];
-        A[pp * kLdA + lane] = cs * akp - sn * akq;
-        A[qq * kLdA + lane] = sn * akp + cs * akq;
-        const double vkp = Vv[pp * kLdA + lane], vkq = Vv[qq * kLdA + lane];
-        Vv[pp * kLdA + lane] = cs * vkp - sn * vkq;
-        Vv[qq * kLdA + lane] = sn * vkp + cs * vkq;
-      }
-      __syncthreads();
-      for (int i = warp; i < half; i += kEigT / 32) {  // rows p, q of column `lane`
-        const int pp = rp[i], qq = rq[i];
-        const double cs = rc[i], sn = rs[i];
-        if (sn == 0.0 || lane >= n) continue;
-        const double apk = A[lane * kLdA + pp], aqk = A[lane * kLdA + qq];
-        A[lane * kLdA + pp] = cs * apk - sn * aqk;
-        A[lane * kLdA + qq] = sn * apk + cs * aqk;
+      if (warp == 0) {
+        if (lane < half && round + 1 < n2 - 1) eig_rotation<Real>(A, n, n2, round + 1, lane, skip, rot, 1 - b);
+      } else if (warp != 4) {
+        turn(b, early + (warp < 4 ? warp - 1 : warp - 2), 6, half);
       }
       __syncthreads();
     }
   }
   __syncthreads();
+}
+
+// C = op(A) B for n x n matrices, columns of length kLdA (op: transpose)
+template <bool TRANS, typename TA, typename TB, typename Out>
+__device__ __forceinline__ void eig_matmul(const TA *A, const TB *B, int n, Out out) {
+  const int r0 = threadIdx.x % kHalfV, c0 = threadIdx.x / kHalfV;  // elements (r0 + 0/16, c0 + 0/16)
+  double s[2][2] = {{0, 0}, {0, 0}};
+  for (int k = 0; k < n; ++k) {
+    double a[2], b[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = r0 + i * kHalfV, c = c0 + i * kHalfV;
+      a[i] = static_cast<double>(TRANS ? A[r * kLdA + k] : A[k * kLdA + r]);
+      b[i] = static_cast<double>(B[c * kLdA + k]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if (r0 + i * kHalfV < n && c0 + j * kHalfV < n) s[i][j] += a[i] * b[j];
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (r0 + i * kHalfV < n && c0 + j * kHalfV < n) out(r0 + i * kHalfV, c0 + j * kHalfV, s[i][j]);
+}
+
+__global__ void __launch_bounds__(kEigT) eng_eig(EArgs a) {
+  const int p = blockIdx.x;
+  EState &st = a.St[p];
+  if (st.done) return;
+  __shared__ double A[kMaxV * kLdA], Vv[kMaxV * kLdA], T[kMaxV * kLdA];
+  __shared__ float A32[kMaxV * kLdA], V32[kMaxV * kLdA];
+  __shared__ Rotations<double> rot;
+  __shared__ Rotations<float> rot32;
+  __shared__ double part[2][kEigT / 32];
+  __shared__ double wv[kMaxV];
+  __shared__ int idx[kMaxV];
+  const int n = st.m, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double big = 0;
+  for (int i = tid; i < kMaxV * kMaxV; i += kEigT) {
+    const int r = i % kMaxV, c = i / kMaxV;
+    const double v = (r < n && c < n) ? st.S[i] : 0.0;
+    A[c * kLdA + r] = v;
+    Vv[c * kLdA + r] = (r == c) ? 1.0 : 0.0;
+    V32[c * kLdA + r] = (r == c) ? 1.f : 0.f;
+    big += fabs(v);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) big += __shfl_xor_sync(0xffffffffu, big, o);
+  if (lane == 0) part[0][warp] = big;
+  __syncthreads();
+  big = 0;
+  for (int w = 0; w < kEigT / 32; ++w) big += part[0][w];
+  __syncthreads();
+  const int ex = big > 0 && big < 1e300 ? ilogb(big) : 0;  // A is scaled to about 1
+  for (int i = tid; i < kMaxV * kMaxV; i += kEigT) {
+    const int at = i / kMaxV * kLdA + i % kMaxV;
+    const double v = scalbn(A[at], -ex);
+    A[at] = v;
+    A32[at] = static_cast<float>(v);
+  }
+  __syncthreads();
+  if (n >= kPreMinN && big > 0 && big < 1e300) {
+    eig_jacobi<float>(A32, V32, n, 1e-10f, 1e-18f, 12, rot32, part);
+    float *E = A32;
+    eig_matmul<true>(V32, V32, n, [&](int r, int c, double v) {
+      const double e = r == c ? v - 1.0 : v;
+      T[c * kLdA + r] = e;
+      E[c * kLdA + r] = static_cast<float>(e);
+    });
+    __syncthreads();
+    for (int i = tid; i < n * n; i += kEigT) {  // (E^2 is 1e-12: FP32 does for it)
+      const int r = i % n, c = i / n;
+      float e2 = 0;
+      for (int k = 0; k < n; ++k) e2 += E[k * kLdA + r] * E[c * kLdA + k];
+      T[c * kLdA + r] = 0.5 * T[c * kLdA + r] - 0.375 * static_cast<double>(e2);
+    }
+    __syncthreads();
+    eig_matmul<false>(V32, T, n, [&](int r, int c, double v) {
+      Vv[c * kLdA + r] = static_cast<double>(V32[c * kLdA + r]) - v;
+    });
+    __syncthreads();
+    eig_matmul<false>(A, Vv, n, [&](int r, int c, double v) { T[c * kLdA + r] = v; });
+    __syncthreads();
+    eig_matmul<true>(Vv, T, n, [&](int r, int c, double v) {
+      if (r <= c) A[c * kLdA + r] = A[r * kLdA + c] = v;
+    });
+    __syncthreads();
+  }
+  eig_jacobi<double>(A, Vv, n, 1e-30, 1e-34, 100, rot, part);
   if (tid < n) {  // rank of each eigenvalue (ties by index)
     const double w = A[tid * (kLdA + 1)];
     int rank = 0;
@@ -746,7 +879,7 @@ __global__ void __launch_bounds__(kEigT) eng_eig(EArgs a) {
       rank += (wj < w || (wj == w && j < tid)) ? 1 : 0;
     }
     idx[rank] = tid;
-    wv[rank] = w;
+    wv[rank] = scalbn(w, ex);
   }
   __syncthreads();
   for (int i = warp; i < n; i += kEigT / 32) {

@@ -129,3 +129,18 @@ def test_engine_tile_autotune(synth, dg):
         after = dg.solve_roots(h, nroots=2, tol=1e-6, mode="mixed")
     assert before["converged"] == after["converged"] == 1
     assert np.allclose(before["energies"], after["energies"], rtol=0, atol=1e-9)
+
+
+@pytest.mark.parametrize("nroots,max_vec", [(1, 7), (1, 8), (1, 9), (2, 15), (3, 31), (4, 17), (4, 32)])
+def test_subspace_eigenproblem_sizes(nroots, max_vec, synth, dg):
+    """Bases around the size from which the subspace eigenproblem goes through
+    FP32 first (8), odd and even, up to the largest: every energy is an
+    eigenvalue, to the square of the residual bound over the gap and FP64's
+    rounding of the solve (1e-9, as above)."""
+    p = synth(10, 5, 140 + max_vec)
+    ref = dense_eigs(p, 252)
+    with dg.Hamiltonian.from_fcidump(p) as h:
+        r = dg.solve_roots(h, nroots=nroots, tol=1e-7, mode="fp64", max_vec=max_vec, max_its=400)
+    assert r["status"] == 0 and r["converged"] == 1
+    for e in r["energies"][:nroots]:
+        assert np.abs(ref - e).min() < 1e-9
