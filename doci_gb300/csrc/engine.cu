@@ -81,9 +81,9 @@ struct EProb {
 };
 
 struct EState {
-  int m, m0, its, done, converged, stall, restart, kk, nact, added, sigmas, idx0, need2;
+  int m, m0, its, done, converged, stall, restart, kk, nact, pend, sigmas, idx0, need2;
   int act[kMaxR];
-  double best, n0, n1, scale;
+  double best, n0, scale;
   double res[kMaxR];
   double w[kMaxV];
   double c[kMaxV];
@@ -127,8 +127,8 @@ __device__ __forceinline__ S *colp(void *base, uint32_t D, int c) {
 // problem's last block to arrive sums the rows in chunk order into
 // out[0..width) and returns true (in every thread of that block).  Results do
 // not depend on timing or on the other problems.
-template <int NK>
-__device__ bool chunk_reduce(double (&acc)[NK], int width, const EArgs &a, const EProb &pb, int p, uint32_t chunk,
+template <int NK, typename S>
+__device__ bool chunk_reduce(S (&acc)[NK], int width, const EArgs &a, const EProb &pb, int p, uint32_t chunk,
                              double *out, int first = 0, int groups = 1) {
   __shared__ double red[kET / 32][NK];
   __shared__ bool last;
@@ -147,15 +147,27 @@ __device__ bool chunk_reduce(double (&acc)[NK], int width, const EArgs &a, const
   __syncthreads();
   if (!last) return false;
   __threadfence();
-  // one warp per output, lanes over the rows (stride 32), then a fixed
-  // shuffle tree: the order depends only on the problem's chunk count
+  // up to 16 threads per output, each over every such row, then over the
+  // threads in order: the order depends only on the problem's chunk count and
+  // the width.  (One warp per output and a shuffle tree took seven of the
+  // Gram-Schmidt step's 25 us: nine outputs per warp, one after the other.)
+  __shared__ double part[kET];
   const double *r0 = a.part + static_cast<size_t>(pb.chunk0) * a.ldp;
-  for (int k = warp; k < width; k += kET / 32) {
+  const int fit = width < kET ? kET / width : 1, per = fit < 16 ? fit : 16;
+  for (int k0 = 0; k0 < width; k0 += kET) {
+    const int w = width - k0 < kET ? width - k0 : kET, k = threadIdx.x % w, g = threadIdx.x / w;
     double s = 0;
-    for (uint32_t c = lane; c < pb.nchunks; c += 32) s += __ldcg(r0 + static_cast<size_t>(c) * a.ldp + k);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) out[k] = s;
+    if (g < per) {
+#pragma unroll 8
+      for (uint32_t c = g; c < pb.nchunks; c += per) s += __ldcg(r0 + static_cast<size_t>(c) * a.ldp + k0 + k);
+    }
+    part[threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.x < w) {
+      for (int i = 1; i < per; ++i) s += part[i * w + threadIdx.x];
+      out[k0 + threadIdx.x] = s;
+    }
+    __syncthreads();
   }
   if (threadIdx.x == 0) a.cnt[p] = 0;
   __syncthreads();
@@ -253,7 +265,8 @@ constexpr int eng_minb() { return sizeof(S) == 4 ? 3 : 1; }
 // The new columns of the subspace matrix, V_k . VA_i for the i = m0 + j new
 // vectors (j < R) and all k <= i: a block takes eight k (blockIdx.y) and four
 // j (blockIdx.z), so that a basis vector is read once for four columns;
-// products summed over the thread's elements in S, then in FP64
+// products summed over the thread's elements in S, then in FP64 (FP32 ones over
+// the warp as pairs of floats: 17 us against 37 with FP64 adds)
 constexpr int kCk = 8, kCj = 4;
 template <typename S>
 __global__ void __launch_bounds__(kET) eng_subcol(EArgs a) {
@@ -285,11 +298,11 @@ __global__ void __launch_bounds__(kET) eng_subcol(EArgs a) {
         }
     }
   }
-  double acc[kCj * kCk];
+  S acc[kCj * kCk];
 #pragma unroll
   for (int j = 0; j < kCj; ++j)
 #pragma unroll
-    for (int k = 0; k < kCk; ++k) acc[j * kCk + k] = static_cast<double>(f[j][k]);
+    for (int k = 0; k < kCk; ++k) acc[j * kCk + k] = f[j][k];
   const int kg = gridDim.y, first = (blockIdx.z * kg + blockIdx.y) * kCj * kCk;
   __shared__ double out[kMaxR * kMaxV];
   if (chunk_reduce<kCj * kCk>(acc, gridDim.z * kg * kCj * kCk, a, pb, p, chunk, out, first, kg * gridDim.z)) {
@@ -350,86 +363,127 @@ __global__ void __launch_bounds__(kET) eng_residual(EArgs a) {
         colp<S>(pb.T, pb.D, q0 + q)[jj] = dd > S(1e-12) ? r / dd : r / S(1e-12);
       }
   }
-  double acc[kRq];
-#pragma unroll
-  for (int q = 0; q < kRq; ++q) acc[q] = static_cast<double>(f[q]);
   __shared__ double out[kMaxR];
-  if (chunk_reduce<kRq>(acc, gridDim.y * kRq, a, pb, p, chunk, out, q0, gridDim.y))
+  if (chunk_reduce<kRq>(f, gridDim.y * kRq, a, pb, p, chunk, out, q0, gridDim.y))
     if (static_cast<int>(threadIdx.x) < nr) st.res[threadIdx.x] = sqrt(out[threadIdx.x]);
 }
 
-// projections of correction act[q]: [t.t, V_k.t]; with `update` (1: first
-// pass, 2: second pass) first t -= sum_k c_k V_k (c from the previous
-// projection).  The second pass runs only when the first left less than half
-// of the correction's norm (the Daniel-Gragg-Kaufman-Stewart test).
+// One step of the Gram-Schmidt orthogonalisation of the corrections t_q =
+// T[:, act[q]], in one read of the basis: t_q -= sum_k c_k V_k with the
+// projections c of the step before, then the sums t_q.t_q and V_k.t_q, and for
+// the next correction t_{q+1}.t_{q+1}, V_k.t_{q+1} and t_q.t_{q+1} (q = -1: only
+// those of t_0).  When t_q keeps more than half of its norm (the Daniel-Gragg-
+// Kaufman-Stewart test) it becomes the basis vector V_m = t_q / |t_q|, whose
+// projection on t_{q+1} is t_q.t_{q+1} / |t_q|: the next step starts from these
+// and writes V_m on its way.  Otherwise the step runs a second time (`pass` 2)
+// with the new projections.
+// A step is bound by its latency (launch, one round of loads, the block's sums,
+// the last block's), so it does all that the data in its registers allow: a
+// projection and an update pass per correction, a pass writing the vector and
+// one counting it took 12 problems of up to 32 vectors 52 us per correction, 32
+// so (FP32 phase).
 template <typename S, int KM>
-__global__ void __launch_bounds__(kET, eng_minb<S>()) eng_gs(EArgs a, int q, int update) {
+__global__ void __launch_bounds__(kET, sizeof(S) == 4 ? 2 : 1) eng_gs(EArgs a, int q, int pass) {
   ENG_CHUNK_PROLOGUE
   if (st.done || q >= st.nact) return;
-  if (update == 2 && !st.need2) return;
-  const int m = st.m;
+  if (pass == 2 && !st.need2) return;
+  const int m = st.m, pend = pass == 1 ? st.pend : -1;
+  const bool own = q >= 0, next = q + 1 < st.nact;
   __shared__ S cs[KM];
-  if (threadIdx.x < KM) cs[threadIdx.x] = (update && threadIdx.x < m) ? static_cast<S>(st.c[threadIdx.x]) : S(0);
+  if (threadIdx.x < KM) cs[threadIdx.x] = (own && threadIdx.x < m) ? static_cast<S>(st.c[threadIdx.x]) : S(0);
   __syncthreads();
-  const S *V = static_cast<const S *>(pb.V);
-  S *t = colp<S>(pb.T, pb.D, st.act[q]);
-  S f[KM + 1];
+  S *V = static_cast<S *>(pb.V);
+  S *t = colp<S>(pb.T, pb.D, own ? st.act[q] : 0);
+  const S *tn = colp<S>(pb.T, pb.D, next ? st.act[q + 1] : 0), *tp = colp<S>(pb.T, pb.D, pend >= 0 ? st.act[pend] : 0);
+  const S psc = pend >= 0 ? static_cast<S>(st.scale) : S(0);
+  constexpr int NK = 3 + 2 * KM;  // t.t, tn.tn, t.tn, then per column V.t, V.tn
+  S f[NK];
 #pragma unroll
-  for (int k = 0; k < KM + 1; ++k) f[k] = S(0);
+  for (int k = 0; k < NK; ++k) f[k] = S(0);
   for (int e = 0; e < eper; ++e) {
     const uint32_t jj = jbase + e * kET;
     if (jj >= pb.D) break;
-    S tv = t[jj];
+    S tv = own ? t[jj] : S(0);
+    const S nv = next ? tn[jj] : S(0);
+    const S pv = pend >= 0 ? tp[jj] * psc : S(0);
     S v[KM];
 #pragma unroll
     for (int k = 0; k < KM; ++k)
-      if (k < m) v[k] = V[static_cast<size_t>(k) * pb.D + jj];
-    if (update) {
+      if (k < m) v[k] = (pend >= 0 && k == m - 1) ? pv : V[static_cast<size_t>(k) * pb.D + jj];
+    if (pend >= 0) V[static_cast<size_t>(m - 1) * pb.D + jj] = pv;
+    if (own) {
 #pragma unroll
       for (int k = 0; k < KM; ++k)
         if (k < m) tv -= cs[k] * v[k];
       t[jj] = tv;
     }
     f[0] += tv * tv;
+    f[1] += nv * nv;
+    f[2] += tv * nv;
 #pragma unroll
     for (int k = 0; k < KM; ++k)
-      if (k < m) f[1 + k] += v[k] * tv;
-  }
-  double acc[KM + 1];
-#pragma unroll
-  for (int k = 0; k < KM + 1; ++k) acc[k] = static_cast<double>(f[k]);
-  __shared__ double out[KM + 1];
-  if (chunk_reduce<KM + 1>(acc, m + 1, a, pb, p, chunk, out)) {
-    if (threadIdx.x < m) st.c[threadIdx.x] = out[1 + threadIdx.x];
-    if (threadIdx.x == 0) {
-      if (!update) {
-        st.n0 = out[0];
-      } else {
-        st.n1 = out[0];
-        if (update == 1) st.need2 = !(out[0] > 0.25 * st.n0);
-        if (update == 2 || !st.need2) {
-          // keep the correction if an independent direction is left
-          const double n0 = st.n0, n1 = st.n1;
-          st.added = (n0 > 0) && (n1 > 0) && (n1 > 1e-20 * n0) && m < a.maxv;
-          st.scale = st.added ? 1.0 / sqrt(n1) : 0.0;
-        }
+      if (k < m) {
+        f[3 + 2 * k] += v[k] * tv;
+        f[4 + 2 * k] += v[k] * nv;
       }
+  }
+  __shared__ double out[NK], scale;
+  __shared__ bool settled;
+  if (!chunk_reduce<NK>(f, 3 + 2 * m, a, pb, p, chunk, out)) return;
+  if (threadIdx.x == 0) {
+    settled = true;  // no second pass for t_q
+    bool add = false;
+    if (own) {
+      const double n0 = st.n0, n1 = out[0];
+      if (pass == 1) st.need2 = !(n1 > 0.25 * n0);
+      settled = pass == 2 || !st.need2;
+      // keep the correction if an independent direction is left
+      add = settled && n0 > 0 && n1 > 0 && n1 > 1e-20 * n0 && m < a.maxv;
     }
+    scale = add ? 1.0 / sqrt(out[0]) : 0.0;
+    st.pend = add ? q : -1;
+    if (add) {
+      st.scale = scale;
+      st.m = m + 1;
+    }
+    if (settled && next) st.n0 = out[1];
+  }
+  __syncthreads();
+  const int k = threadIdx.x;
+  if (!settled) {
+    if (k < m) st.c[k] = out[3 + 2 * k];
+  } else if (next) {
+    if (k < m) st.c[k] = out[4 + 2 * k];
+    else if (k == m && m < kMaxV) st.c[k] = scale * out[2];
   }
 }
 
-// V[:, m] = t * scale for an added correction
+// The last step's vector, if it became one; then a basis that did not grow
+// ends the solve, else the new vectors get their sigmas.  (A problem whose
+// basis did not grow has no vector to write, so its blocks need not agree on
+// `done`.)
 template <typename S>
-__global__ void __launch_bounds__(kET) eng_gs_finish(EArgs a, int q) {
+__global__ void __launch_bounds__(kET) eng_gs_finish(EArgs a) {
   ENG_CHUNK_PROLOGUE
-  if (st.done || q >= st.nact || !st.added) return;
-  const S *t = colp<S>(pb.T, pb.D, st.act[q]);
-  S *out = colp<S>(pb.V, pb.D, st.m);
-  const S sc = static_cast<S>(st.scale);
-  for (int e = 0; e < eper; ++e) {
-    const uint32_t jj = jbase + e * kET;
-    if (jj >= pb.D) break;
-    out[jj] = t[jj] * sc;
+  if (st.done) return;
+  const int m = st.m;
+  if (st.pend >= 0) {
+    const S *t = colp<S>(pb.T, pb.D, st.act[st.pend]);
+    S *out = colp<S>(pb.V, pb.D, m - 1);
+    const S sc = static_cast<S>(st.scale);
+    for (int e = 0; e < eper; ++e) {
+      const uint32_t jj = jbase + e * kET;
+      if (jj >= pb.D) break;
+      out[jj] = t[jj] * sc;
+    }
+  }
+  if (chunk == 0 && threadIdx.x == 0) {
+    if (m == st.m0) {
+      st.done = 1;
+      a.flags[p] = 0;
+    } else {
+      st.sigmas += m - st.m0;
+    }
   }
 }
 
@@ -608,7 +662,8 @@ __global__ void eng_init_state(EArgs a) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= a.n) return;
   EState &st = a.St[p];
-  st.m = st.m0 = st.its = st.done = st.converged = st.stall = st.restart = st.kk = st.added = st.sigmas = 0;
+  st.m = st.m0 = st.its = st.done = st.converged = st.stall = st.restart = st.kk = st.sigmas = 0;
+  st.pend = -1;
   st.best = 1e300;
   const int R = a.R < static_cast<int>(a.P[p].D) ? a.R : static_cast<int>(a.P[p].D);
   st.nact = R;
@@ -925,6 +980,7 @@ __global__ void eng_control(EArgs a) {
     if (st.res[r] > a.tol) st.act[nact++] = r;
   }
   st.nact = nact;
+  st.pend = -1;
   st.m0 = st.m;
   if (worst <= a.tol) {
     st.done = 1;
@@ -940,27 +996,6 @@ __global__ void eng_control(EArgs a) {
     }
   }
   if (st.done) a.flags[p] = 0;
-}
-
-// commit an added vector; after the last correction, a basis that did not
-// grow ends the solve, else the new vectors get their sigmas
-__global__ void eng_orth_commit(EArgs a, int q, int last) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= a.n) return;
-  EState &st = a.St[p];
-  if (st.done) return;
-  if (q < st.nact && st.added) {
-    ++st.m;
-    st.added = 0;
-  }
-  if (last) {
-    if (st.m == st.m0) {
-      st.done = 1;
-      a.flags[p] = 0;
-    } else {
-      st.sigmas += st.m - st.m0;
-    }
-  }
 }
 
 // ---------------------------------------------------------------- host side
@@ -1052,13 +1087,12 @@ int run_phase(EArgs &a, uint32_t ntiles, uint32_t nchunks, cudaStream_t st, bool
   // the orthonormalisation of the corrections and the sigmas and subspace
   // columns of the vectors added (the start block is the first "corrections")
   auto extend = [&]() -> int {
+    eng_gs<S, KM><<<nblk(nchunks), kET, 0, st>>>(a, -1, 0);
     for (int q = 0; q < R; ++q) {
-      eng_gs<S, KM><<<nblk(nchunks), kET, 0, st>>>(a, q, 0);
       eng_gs<S, KM><<<nblk(nchunks), kET, 0, st>>>(a, q, 1);
       eng_gs<S, KM><<<nblk(nchunks), kET, 0, st>>>(a, q, 2);
-      eng_gs_finish<S><<<nblk(nchunks), kET, 0, st>>>(a, q);
-      eng_orth_commit<<<small, 128, 0, st>>>(a, q, q == R - 1);
     }
+    eng_gs_finish<S><<<nblk(nchunks), kET, 0, st>>>(a);
     if (ntiles > 0) eng_sigma<S, NH><<<nblk(ntiles), kET, 0, st>>>(a);
     if (side.n > 0) DOCI_CUDA(side.fork(st));
     for (size_t b = 0, k = 0; b < big.size(); ++b) {

@@ -144,3 +144,26 @@ def test_subspace_eigenproblem_sizes(nroots, max_vec, synth, dg):
     assert r["status"] == 0 and r["converged"] == 1
     for e in r["energies"][:nroots]:
         assert np.abs(ref - e).min() < 1e-9
+
+
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+@pytest.mark.parametrize("L,N,nroots", [(1, 1, 1), (2, 1, 4), (3, 1, 2), (4, 2, 4), (4, 2, 8), (9, 4, 1), (12, 6, 5)])
+def test_orthogonalisation_step_edges(L, N, nroots, mode, synth, dg):
+    """Few determinants (corrections with nothing left of them), one root (no next
+    correction in a step), more than four: the lowest eigenvalues, each once,
+    with orthonormal vectors; more roots than determinants are refused, as ever.
+    Residuals below 1e-7 bound the energies' errors; vectors are FP64."""
+    p = synth(L, N, 150 + L + nroots)
+    with dg.Hamiltonian.from_fcidump(p) as h:
+        k = nroots
+        if k > h.D:
+            with pytest.raises(dg.DociError, match="DOCI_ERR_INVALID"):
+                dg.solve_roots(h, vectors=True, nroots=nroots, tol=1e-7, mode=mode, max_vec=32)
+            return
+        ref = dense_eigs(p, k)
+        r = dg.solve_roots(h, vectors=True, nroots=nroots, tol=1e-7, mode=mode, max_vec=32)
+        r, v = r if isinstance(r, tuple) else (r, r["vectors"])
+        v = np.asarray(v).reshape(-1, h.D)[:k]
+    assert r["status"] == 0 and r["converged"] == 1
+    assert np.allclose(r["energies"][:k], ref, atol=1e-7)
+    assert np.abs(v @ v.T - np.eye(k)).max() < 1e-6
