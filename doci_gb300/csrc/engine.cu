@@ -688,19 +688,18 @@ __global__ void eng_init_state(EArgs a) {
 // 3 E^2 / 8) is orthogonal to E^3), and the FP64 Jacobi then starts from V^T A V,
 // whose off-diagonal part is about 1e-6 of the whole: two sweeps instead of six
 // or seven, with fewer FP64 roundings than those (vectors orthogonal to 5e-15
-// instead of 1e-14 at n = 32).  A round rotates the 2 x 2 blocks of A, one
-// thread per block of the upper triangle (their columns and rows at once, the
-// mirror written along) while the free warps turn 7/16 of the vectors; then warp
-// 0 computes the next round's rotations while the others turn the rest (so that
-// the SM's four quarters have about the same FP64 work in both steps).  A rotation's tangent, which only steers the
-// convergence, is computed in FP32 from differences in the matrix's type, the
-// cosine in that type (an FP32 reciprocal square root and one third-order
-// step for FP64), so that the rotations stay orthogonal to its accuracy; and a
-// pair whose square is below `skip`, which cannot keep the off-diagonal part
-// above its limit, is left alone.
+// instead of 1e-14 at n = 32).
+//
+// A rotation's tangent, which only steers the convergence, is computed in FP32
+// from differences in the matrix's type, the cosine in that type (an FP32
+// reciprocal square root and one third-order step for FP64), so that the
+// rotations stay orthogonal to its accuracy; and a pair whose square is below
+// `skip`, which cannot keep the off-diagonal part above its limit, is left alone.
 // Measured on 12 problems of up to 32 vectors (average over a solve): 1,609 us
-// with one warp and FP64 tangents, 468 us with 256 threads in FP64 alone, 198
-// us so.
+// with one warp and FP64 tangents, 468 us with 256 threads in FP64 alone, 197 us
+// with FP32 sweeps of the FP64 sweeps' form and FP64 sums for the stopping test,
+// 163 us so.  At 24 vectors 150 us of FP32 and FP64 sweeps are latency (900
+// clocks a round) and FP64 work in about equal parts, 40 us the products.
 constexpr int kEigT = 256;
 constexpr int kLdA = kMaxV + 1;
 constexpr int kHalfV = kMaxV / 2;
@@ -712,46 +711,136 @@ struct Rotations {  // one round's pairs (twice: this round's and the next one's
   int p[2][kHalfV], q[2][kHalfV];
 };
 
-// rotation of pair `k` of a round (n2 = n rounded up to even; with n odd one
-// pair a round is idle)
-template <typename Real>
-__device__ __forceinline__ void eig_rotation(const Real *A, int n, int n2, int round, int k, Real skip,
-                                             Rotations<Real> &rot, int buf) {
+// pair `k` of a round (n2 = n rounded up to even; with n odd one pair a round
+// holds n and is idle)
+__device__ __forceinline__ void eig_pair(int n2, int round, int k, int &pp, int &qq) {
   auto player = [&](int i) {  // i - 1 + round modulo n2 - 1, plus one
     const int j = i + round;
     return i == 0 ? 0 : j > n2 - 1 ? j - (n2 - 1) : j;
   };
   const int pl = player(k), ql = player(n2 - 1 - k);
-  const int pp = min(pl, ql), qq = max(pl, ql);
-  Real cs = 1, sn = 0;
-  if (qq < n) {
-    const Real apq = A[qq * kLdA + pp];
-    if (apq * apq > skip) {
-      // t = sign(d) b / (|d| + sqrt(d^2 + b^2)), d = aqq - app, b = 2 apq (A is
-      // scaled to about 1 and apq not below `skip`: no under- or overflow)
-      const float d = static_cast<float>(A[qq * kLdA + qq] - A[pp * kLdA + pp]), b = 2 * static_cast<float>(apq);
-      const float h = d * d + b * b, tf = __fdividef(d >= 0 ? b : -b, fabsf(d) + h * rsqrtf(h));
-      const Real t = tf, u = 1 + t * t;
-      Real y = rsqrtf(static_cast<float>(u));
-      if constexpr (sizeof(Real) == 8) {  // y has 22 bits; 1/sqrt(u) = y / sqrt(1 - e), e = 1 - u y^2, to e^3
-        const Real e = 1 - u * (y * y);
-        y += y * (e * (0.5 + 0.375 * e));
-      }
-      cs = y;
-      sn = t * y;
-    }
-  }
-  rot.p[buf][k] = pp;
-  rot.q[buf][k] = qq;
-  rot.c[buf][k] = cs;
-  rot.s[buf][k] = sn;
+  pp = min(pl, ql);
+  qq = max(pl, ql);
 }
 
-// sweeps on A (symmetric, full) with the vectors V until the off-diagonal
-// squares are below `stop` of the whole (at most `sweeps`)
+// the rotation of a pair, without branches (the idle pair's entries are zero)
 template <typename Real>
-__device__ void eig_jacobi(Real *A, Real *V, int n, Real stop, Real skip_rel, int sweeps, Rotations<Real> &rot,
-                           double (*part)[kEigT / 32]) {
+__device__ __forceinline__ void eig_rotation(const Real *A, int pp, int qq, Real skip, Real &cs, Real &sn) {
+  const Real apq = A[qq * kLdA + pp];
+  // t = sign(d) b / (|d| + sqrt(d^2 + b^2)), d = aqq - app, b = 2 apq (A is
+  // scaled to about 1 and apq not below `skip`: no under- or overflow)
+  const float d = static_cast<float>(A[qq * kLdA + qq] - A[pp * kLdA + pp]), b = 2 * static_cast<float>(apq);
+  const float h = d * d + b * b, tf = __fdividef(d >= 0 ? b : -b, fabsf(d) + h * rsqrtf(h));
+  const Real t = tf, u = 1 + t * t;
+  Real y = rsqrtf(static_cast<float>(u));
+  if constexpr (sizeof(Real) == 8) {  // y has 22 bits; 1/sqrt(u) = y / sqrt(1 - e), e = 1 - u y^2, to e^3
+    const Real e = 1 - u * (y * y);
+    y += y * (e * (0.5 + 0.375 * e));
+  }
+  const bool turned = apq * apq > skip;
+  cs = turned ? y : Real(1);
+  sn = turned ? t * y : Real(0);
+}
+
+// off <= stop * tot for the squares of A's off-diagonal part and of all of it
+// (A is scaled to about 1: FP32 holds squares of 1e-30 of it); tot is returned
+template <typename Real>
+__device__ __forceinline__ bool eig_settled(const Real *A, int n, float stop, float (*part)[kEigT / 32], float &tot) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float off = 0;
+  tot = 0;
+  for (int c = warp; c < n; c += kEigT / 32) {
+    const float v = lane < n ? static_cast<float>(A[c * kLdA + lane]) : 0.f;
+    tot += v * v;
+    off += lane == c ? 0.f : v * v;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    off += __shfl_xor_sync(0xffffffffu, off, o);
+    tot += __shfl_xor_sync(0xffffffffu, tot, o);
+  }
+  if (lane == 0) {
+    part[0][warp] = off;
+    part[1][warp] = tot;
+  }
+  __syncthreads();
+  off = tot = 0;
+#pragma unroll
+  for (int w = 0; w < kEigT / 32; ++w) {
+    off += part[0][w];
+    tot += part[1][w];
+  }
+  return off == 0 || off <= stop * tot;
+}
+
+// The FP32 sweeps: a round is bound by its latency, so it has one barrier.
+// Every thread computes the two rotations of its 2 x 2 block (all blocks of a
+// pair get the same bits), reads the block from A and writes it to B, which
+// change places; the vectors are turned one round behind.
+__device__ void eig_jacobi32(float *A, float *B, float *V, int n, float stop, float skip_rel, int sweeps,
+                             Rotations<float> &rot, float (*part)[kEigT / 32]) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n2 = n + (n & 1), half = n2 / 2, bi = tid % kHalfV, bj = tid / kHalfV;
+  auto turn = [&](int b) {
+#pragma unroll
+    for (int i = 0; i < kHalfV * 32 / kEigT; ++i) {
+      const int k = warp + i * (kEigT / 32);
+      if (k >= half || lane >= n) continue;
+      const int pp = rot.p[b][k], qq = rot.q[b][k];
+      const float c = rot.c[b][k], s = rot.s[b][k];
+      const float vp = V[pp * kLdA + lane], vq = V[qq * kLdA + lane];
+      V[pp * kLdA + lane] = c * vp - s * vq;
+      V[qq * kLdA + lane] = s * vp + c * vq;
+    }
+  };
+  int done = 0;  // rounds so far
+  for (int sweep = 0; sweep < sweeps; ++sweep) {
+    float tot;
+    if (eig_settled<float>(A, n, stop, part, tot)) break;
+    const float skip = skip_rel * tot;
+    for (int round = 0; round < n2 - 1; ++round, ++done) {
+      if (bi < half && bj < half) {  // rows (p, q) of pair i, columns (p, q) of pair j
+        int pi, qi, pj, qj;
+        float ci, si, cj, sj;
+        eig_pair(n2, round, bi, pi, qi);
+        eig_pair(n2, round, bj, pj, qj);
+        const float a00 = A[pj * kLdA + pi], a01 = A[qj * kLdA + pi], a10 = A[pj * kLdA + qi], a11 = A[qj * kLdA + qi];
+        eig_rotation<float>(A, pi, qi, skip, ci, si);
+        eig_rotation<float>(A, pj, qj, skip, cj, sj);
+        const float x0 = cj * a00 - sj * a01, x1 = sj * a00 + cj * a01;
+        const float y0 = cj * a10 - sj * a11, y1 = sj * a10 + cj * a11;
+        B[pj * kLdA + pi] = ci * x0 - si * y0;
+        B[pj * kLdA + qi] = si * x0 + ci * y0;
+        B[qj * kLdA + pi] = ci * x1 - si * y1;
+        B[qj * kLdA + qi] = si * x1 + ci * y1;
+        if (bi == bj) {
+          rot.p[done & 1][bi] = pi;
+          rot.q[done & 1][bi] = qi;
+          rot.c[done & 1][bi] = ci;
+          rot.s[done & 1][bi] = si;
+        }
+      }
+      if (done > 0) turn((done - 1) & 1);
+      __syncthreads();
+      float *t = A;
+      A = B;
+      B = t;
+    }
+  }
+  if (done > 0) turn((done - 1) & 1);
+  __syncthreads();
+}
+
+// The FP64 sweeps on A (symmetric, full) with the vectors V until the
+// off-diagonal squares are below `stop` of the whole (at most `sweeps`).
+// A round rotates the 2 x 2 blocks of A, one thread per block of the upper
+// triangle (its columns and rows at once, the mirror written along) while the
+// free warps turn 7/16 of the vectors; then warp 0 computes the next round's
+// rotations while the others turn the rest, so that the SM's four quarters have
+// about the same FP64 work in both steps.
+__device__ void eig_jacobi64(double *A, double *V, int n, float stop, double skip_rel, int sweeps,
+                             Rotations<double> &rot, float (*part)[kEigT / 32]) {
+  using Real = double;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n2 = n + (n & 1), half = n2 / 2;
   int bi = tid, bj = 1;  // this thread's block of the upper triangle (threads 0 to 127)
@@ -759,41 +848,30 @@ __device__ void eig_jacobi(Real *A, Real *V, int n, Real stop, Real skip_rel, in
   const bool off_block = tid < half * (half - 1) / 2;
   auto turn = [&](int b, int first, int step, int end) {  // the vectors by the pairs first, first + step, ...
     if (lane >= n) return;
+#pragma unroll 3
     for (int k = first; k < end; k += step) {
       const int pp = rot.p[b][k], qq = rot.q[b][k];
       const Real c = rot.c[b][k], s = rot.s[b][k];
-      if (s == 0) continue;
       const Real vp = V[pp * kLdA + lane], vq = V[qq * kLdA + lane];
       V[pp * kLdA + lane] = c * vp - s * vq;
       V[qq * kLdA + lane] = s * vp + c * vq;
     }
   };
   for (int sweep = 0; sweep < sweeps && n > 1; ++sweep) {
-    double off = 0, tot = 0;
-    for (int i = tid; i < n * n; i += kEigT) {
-      const int r = i % n, c = i / n;
-      const double e = static_cast<double>(A[c * kLdA + r] * A[c * kLdA + r]);
-      tot += e;
-      if (r != c) off += e;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      off += __shfl_xor_sync(0xffffffffu, off, o);
-      tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    }
-    if (lane == 0) {
-      part[0][warp] = off;
-      part[1][warp] = tot;
-    }
-    __syncthreads();
-    off = tot = 0;
-    for (int w = 0; w < kEigT / 32; ++w) {
-      off += part[0][w];
-      tot += part[1][w];
-    }
-    if (off == 0 || off <= stop * tot) break;
-    const Real skip = static_cast<Real>(skip_rel * tot);
-    if (tid < half) eig_rotation<Real>(A, n, n2, 0, tid, skip, rot, 0);
+    float tot;
+    if (eig_settled<double>(A, n, stop, part, tot)) break;
+    const double skip = skip_rel * static_cast<double>(tot);
+    auto rotation = [&](int round, int k, int buf) {
+      int pp, qq;
+      double cs, sn;
+      eig_pair(n2, round, k, pp, qq);
+      eig_rotation<double>(A, pp, qq, skip, cs, sn);
+      rot.p[buf][k] = pp;
+      rot.q[buf][k] = qq;
+      rot.c[buf][k] = cs;
+      rot.s[buf][k] = sn;
+    };
+    if (tid < half) rotation(0, tid, 0);
     __syncthreads();
     for (int round = 0; round < n2 - 1; ++round) {
       const int b = round & 1;
@@ -826,7 +904,7 @@ __device__ void eig_jacobi(Real *A, Real *V, int n, Real stop, Real skip_rel, in
       if (warp > 4) turn(b, warp - 5, 3, early);
       __syncthreads();
       if (warp == 0) {
-        if (lane < half && round + 1 < n2 - 1) eig_rotation<Real>(A, n, n2, round + 1, lane, skip, rot, 1 - b);
+        if (lane < half && round + 1 < n2 - 1) rotation(round + 1, lane, 1 - b);
       } else if (warp != 4) {
         turn(b, early + (warp < 4 ? warp - 1 : warp - 2), 6, half);
       }
@@ -867,10 +945,11 @@ __global__ void __launch_bounds__(kEigT) eng_eig(EArgs a) {
   EState &st = a.St[p];
   if (st.done) return;
   __shared__ double A[kMaxV * kLdA], Vv[kMaxV * kLdA], T[kMaxV * kLdA];
-  __shared__ float A32[kMaxV * kLdA], V32[kMaxV * kLdA];
+  __shared__ float A32[kMaxV * kLdA], B32[kMaxV * kLdA], V32[kMaxV * kLdA];
   __shared__ Rotations<double> rot;
   __shared__ Rotations<float> rot32;
-  __shared__ double part[2][kEigT / 32];
+  __shared__ double sum[kEigT / 32];
+  __shared__ float part[2][kEigT / 32];
   __shared__ double wv[kMaxV];
   __shared__ int idx[kMaxV];
   const int n = st.m, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -885,10 +964,10 @@ __global__ void __launch_bounds__(kEigT) eng_eig(EArgs a) {
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) big += __shfl_xor_sync(0xffffffffu, big, o);
-  if (lane == 0) part[0][warp] = big;
+  if (lane == 0) sum[warp] = big;
   __syncthreads();
   big = 0;
-  for (int w = 0; w < kEigT / 32; ++w) big += part[0][w];
+  for (int w = 0; w < kEigT / 32; ++w) big += sum[w];
   __syncthreads();
   const int ex = big > 0 && big < 1e300 ? ilogb(big) : 0;  // A is scaled to about 1
   for (int i = tid; i < kMaxV * kMaxV; i += kEigT) {
@@ -899,7 +978,7 @@ __global__ void __launch_bounds__(kEigT) eng_eig(EArgs a) {
   }
   __syncthreads();
   if (n >= kPreMinN && big > 0 && big < 1e300) {
-    eig_jacobi<float>(A32, V32, n, 1e-10f, 1e-18f, 12, rot32, part);
+    eig_jacobi32(A32, B32, V32, n, 1e-10f, 1e-18f, 12, rot32, part);
     float *E = A32;
     eig_matmul<true>(V32, V32, n, [&](int r, int c, double v) {
       const double e = r == c ? v - 1.0 : v;
@@ -925,7 +1004,7 @@ __global__ void __launch_bounds__(kEigT) eng_eig(EArgs a) {
     });
     __syncthreads();
   }
-  eig_jacobi<double>(A, Vv, n, 1e-30, 1e-34, 100, rot, part);
+  eig_jacobi64(A, Vv, n, 1e-30f, 1e-34, 100, rot, part);
   if (tid < n) {  // rank of each eigenvalue (ties by index)
     const double w = A[tid * (kLdA + 1)];
     int rank = 0;
