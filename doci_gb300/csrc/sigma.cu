@@ -1237,7 +1237,11 @@ size_t nbr_table_bytes(int L, int N, uint64_t D) {
 int ham_build_nbr(doci_ham *h) {
   const size_t bytes = nbr_table_bytes(h->L, h->N, h->D);
   if (bytes == 0) return DOCI_OK;
-  DOCI_CUDA(cudaMallocAsync(&h->d_nbr, bytes, h->stream));
+  if (cudaMallocAsync(&h->d_nbr, bytes, h->stream) != cudaSuccess) {  // no memory: the kernels without a table
+    cudaGetLastError();
+    h->d_nbr = nullptr;
+    return DOCI_OK;
+  }
   nbr_table_kernel<<<grid_for(h->D), kThreads, 0, h->stream>>>(SigmaShape{h->D, h->L, h->N, h->nh}, h->d_binom,
                                                                h->d_nbr);
   DOCI_CUDA(cudaGetLastError());
