@@ -225,7 +225,7 @@ def fp64_like_for_like(h, D, dg, torch, steps: int):
         calls.append(time.perf_counter() - tc)
     te = (time.perf_counter() - t0) / steps
     return {"value": round(D / ms / 1e6, 4), "unit": UNIT, "sigma_ms": round(ms, 3),
-            "sigma_kernel": KERNEL_NAMES.get(kind, kind), "dtype": "f64 (float-float pair form)" if kind == 9 else "f64",
+            "sigma_kernel": KERNEL_NAMES.get(kind, kind), "dtype": "f64 (pair form, products exact in FP16 digits)" if kind == 9 else "f64",
             "e2e": {"value": round(D / te / 1e9, 4), "unit": UNIT, "ms_per_call": round(te * 1e3, 3),
                     "h2d_bytes_per_step": D * 8, "d2h_bytes_per_step": D * 8,
                     "call": "doci_sigma_host FP64 (C ABI, pinned host buffers)", "steps": steps,
