@@ -180,20 +180,22 @@ sigma_pair_warp_kernel(const __grid_constant__ PwShape s, const uint32_t *__rest
 #pragma unroll
         for (int o = 0; o < P; ++o) v[o] = lds(ca + (o & 1 ? w[o >> 1] >> 16 : w[o >> 1] & 0xffffu));
         if (n > 0 && !warp_wait(bar_done, (n - 1) & 1u, s.spin_limit, abort_flag, err, 21)) fail = true;
-        fence_after();
-        // split into TF32 high and low parts in this lane's row of the tile
+        if (!fail) {  // (else an MMA may still read the tile)
+          fence_after();
+          // split into TF32 high and low parts in this lane's row of the tile
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          uint32_t r[8];
+          for (int h = 0; h < 4; ++h) {
+            uint32_t r[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) r[i] = tf32_rna(v[8 * h + i]);
-          tst8(tw + 8 * h, r);
+            for (int i = 0; i < 8; ++i) r[i] = tf32_rna(v[8 * h + i]);
+            tst8(tw + 8 * h, r);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) r[i] = __float_as_uint(v[8 * h + i] - __uint_as_float(r[i]));
-          tst8(tw + 32 + 8 * h, r);
+            for (int i = 0; i < 8; ++i) r[i] = __float_as_uint(v[8 * h + i] - __uint_as_float(r[i]));
+            tst8(tw + 32 + 8 * h, r);
+          }
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          fence_before();
         }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        fence_before();
         if (group_meet(slot, fail)) {
           ok = false;
           break;
@@ -276,9 +278,9 @@ sigma_pair_warp_kernel(const __grid_constant__ PwShape s, const uint32_t *__rest
       __syncwarp();
     }
   }
-  // after a wait that ran out: the MMAs in flight complete by themselves; wait
+  // the last tile's MMAs complete by themselves; whatever side gave up, wait
   // for them (bounded) before the tensor memory is freed
-  if (gatherer && w4 == 0 && !ok && n > 0)
+  if (gatherer && w4 == 0 && n > 0)
     for (long i = 0; i < kTcSpinLimit && !mbar_try(bar_done, (n - 1) & 1u); ++i) {
     }
   fence_before();

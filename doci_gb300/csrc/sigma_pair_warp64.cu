@@ -255,43 +255,45 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
         const float f1 = inf ? __uint_as_float(0x7fc00000u) : __uint_as_float((262u - eb) << 23);  // 2^(135 - eb)
         const float f3 = __uint_as_float((284u - (inf ? 30u : eb)) << 23);                         // 2^(157 - eb)
         if (n > 0 && !warp_wait(bar_done, (n - 1) & 1u, s.spin_limit, abort_flag, err, 31)) fail = true;
-        fence_after();
-        // five signed digits of eleven bits, most significant first:
-        // X 2^(124 - eb) = sum_i d_i 2^(-11 i), below 1/4, d_i the nearest
-        // integer each time, every remainder exact but the last bits of h + l
-        // past 2^-57
-        const f2 c2048 = pk(2048.f, 2048.f), magic = pk(12582912.f, 12582912.f), nmagic = pk(-12582912.f, -12582912.f);
+        if (!fail) {  // (else an MMA may still read the tile)
+          fence_after();
+          // five signed digits of eleven bits, most significant first:
+          // X 2^(124 - eb) = sum_i d_i 2^(-11 i), below 1/4, d_i the nearest
+          // integer each time, every remainder exact but the last bits of h + l
+          // past 2^-57
+          const f2 c2048 = pk(2048.f, 2048.f), magic = pk(12582912.f, 12582912.f), nmagic = pk(-12582912.f, -12582912.f);
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          uint32_t d1[8], d2[8], d3[8], d4[8], d5[8];
+          for (int hf = 0; hf < 2; ++hf) {
+            uint32_t d1[8], d2[8], d3[8], d4[8], d5[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int a = 16 * hf + 2 * i;
-            const f2 r1 = pk(xh[a] * f1, xh[a + 1] * f1), lo = pk(xl[a] * f3, xl[a + 1] * f3);
-            const f2 s1 = addp(addp(r1, magic), nmagic);
-            const f2 r2 = mulp(subp(r1, s1), c2048);
-            const f2 s2 = addp(addp(r2, magic), nmagic);
-            const f2 u = subp(r2, s2);
-            const f2 s3 = addp(addp(fma2(u, c2048, lo), magic), nmagic);
-            const f2 r4 = mulp(addp(fma2(u, c2048, mulp(s3, pk(-1.f, -1.f))), lo), c2048);
-            const f2 s4 = addp(addp(r4, magic), nmagic);
-            const f2 r5 = mulp(subp(r4, s4), c2048);
-            const f2 s5 = addp(addp(r5, magic), nmagic);
-            d1[i] = half2_bits(s1);
-            d2[i] = half2_bits(s2);
-            d3[i] = half2_bits(s3);
-            d4[i] = half2_bits(s4);
-            d5[i] = half2_bits(s5);
+            for (int i = 0; i < 8; ++i) {
+              const int a = 16 * hf + 2 * i;
+              const f2 r1 = pk(xh[a] * f1, xh[a + 1] * f1), lo = pk(xl[a] * f3, xl[a + 1] * f3);
+              const f2 s1 = addp(addp(r1, magic), nmagic);
+              const f2 r2 = mulp(subp(r1, s1), c2048);
+              const f2 s2 = addp(addp(r2, magic), nmagic);
+              const f2 u = subp(r2, s2);
+              const f2 s3 = addp(addp(fma2(u, c2048, lo), magic), nmagic);
+              const f2 r4 = mulp(addp(fma2(u, c2048, mulp(s3, pk(-1.f, -1.f))), lo), c2048);
+              const f2 s4 = addp(addp(r4, magic), nmagic);
+              const f2 r5 = mulp(subp(r4, s4), c2048);
+              const f2 s5 = addp(addp(r5, magic), nmagic);
+              d1[i] = half2_bits(s1);
+              d2[i] = half2_bits(s2);
+              d3[i] = half2_bits(s3);
+              d4[i] = half2_bits(s4);
+              d5[i] = half2_bits(s5);
+            }
+            tst8(tw + 8 * hf, d1);
+            tst8(tw + 16 + 8 * hf, d2);
+            tst8(tw + 32 + 8 * hf, d3);
+            tst8(tw + 48 + 8 * hf, d4);
+            tst8(tw + 64 + 8 * hf, d5);
           }
-          tst8(tw + 8 * hf, d1);
-          tst8(tw + 16 + 8 * hf, d2);
-          tst8(tw + 32 + 8 * hf, d3);
-          tst8(tw + 48 + 8 * hf, d4);
-          tst8(tw + 64 + 8 * hf, d5);
+          tst1(tw + kColE + (n & 1u), eb);
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          fence_before();
         }
-        tst1(tw + kColE + (n & 1u), eb);
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        fence_before();
         if (group_meet(slot, fail)) {
           ok = false;
           break;
@@ -403,9 +405,9 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
       __syncwarp();
     }
   }
-  // after a wait that ran out: the MMAs in flight complete by themselves; wait
+  // the last tile's MMAs complete by themselves; whatever side gave up, wait
   // for them (bounded) before the tensor memory is freed
-  if (gatherer && w4 == 0 && !ok && n > 0)
+  if (gatherer && w4 == 0 && n > 0)
     for (long i = 0; i < kTcSpinLimit && !mbar_try(bar_done, (n - 1) & 1u); ++i) {
     }
   fence_before();

@@ -47,3 +47,51 @@ def test_wait_limit_reports_timeout(synth):
     lines = dict(ln.split(" ", 1) for ln in r.stdout.splitlines() if ln.startswith(("status", "after")))
     assert int(lines["status"]) == 12  # DOCI_ERR_DEVICE_TIMEOUT
     assert float(lines["after"]) <= 2e-6
+
+
+WARP_CHILD = r"""
+import ctypes as C, sys
+import numpy as np, torch
+sys.path.insert(0, {root!r})
+import doci_gb300 as dg, oracle
+p = {path!r}
+o = oracle.Ham(p)
+with dg.Hamiltonian.from_fcidump(p) as h:
+    for name, prec in (("pair", dg.FP32), ("rowff", dg.FP64)):
+        h.set_sigma_kernel(name)
+        assert h.sigma_plan(prec)[0] == (6 if prec == dg.FP32 else 9)
+        x = np.random.default_rng(1).standard_normal(h.D).astype(np.float32 if prec == dg.FP32 else np.float64)
+        y = np.empty_like(x)
+        for _ in range(3):
+            print("status", dg.lib().doci_sigma_host(h.handle, x.ctypes.data_as(C.c_void_p),
+                                                     y.ctypes.data_as(C.c_void_p), prec))
+        h.set_sigma_kernel("auto")
+        X = torch.from_numpy(np.stack([x, x])).cuda()
+        Y = torch.empty_like(X)
+        h.sigma_block_device(X.data_ptr(), h.D, Y.data_ptr(), h.D, 2, prec)
+        torch.cuda.synchronize()
+        h.set_sigma_kernel("gather")
+        st = dg.lib().doci_sigma_host(h.handle, x.ctypes.data_as(C.c_void_p), y.ctypes.data_as(C.c_void_p), prec)
+        print("block", st)
+        y2 = h.sigma(x, prec)
+        ref = o.matvec(x.astype(np.float64))
+        print("after", float(np.abs(y2 - ref).max() / np.abs(ref).max()))
+"""
+
+
+# one tile in the only slot; one to three tiles a slot; slots with many units
+@pytest.mark.parametrize("L,N", [(10, 1), (12, 6), (22, 11)])
+def test_warp_wait_limit_reports_timeout(L, N, synth):
+    """The same for the warp-per-unit pair forms (kinds 6 and 9, and their
+    reproducible forms in the block sigma on the space without a neighbour
+    table): a scattering warp whose wait runs out leaves the slot's last MMAs
+    to the issuing warp, which waits for them before the tensor memory goes."""
+    p = synth(L, N, 72)
+    env = dict(os.environ, DOCI_TC_SPIN_LIMIT="0")
+    r = subprocess.run([sys.executable, "-c", WARP_CHILD.format(root=ROOT, path=p)], capture_output=True, text=True,
+                       env=env, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    got = [ln.split() for ln in r.stdout.splitlines() if ln.startswith(("status", "block", "after"))]
+    assert [int(v) for k, v in got if k == "status"] == [12] * 6  # DOCI_ERR_DEVICE_TIMEOUT
+    assert [int(v) for k, v in got if k == "block"] == [12 if (L, N) == (22, 11) else 0] * 2
+    assert all(float(v) <= 2e-6 for k, v in got if k == "after")
