@@ -115,6 +115,7 @@ struct doci_ham {
   uint32_t *d_wstart = nullptr, *d_wunits = nullptr;
   uint16_t *d_kdig = nullptr;  // K in 11-bit digits (FP16) and their exponent
   int kdig_exp = 0;
+  bool kdig_ok = false;        // the digits' sums are exact for this K (sigma_pair_warp64.cu)
   const void *d_wtab_a = nullptr, *d_wtab_b = nullptr;  // insertion tables (per-process cache)
   // doci_sigma_host on the pair forms: x and sigma cross the host link in
   // pieces (chunk_off) on copy_stream while the pair units run in groups,
@@ -183,7 +184,8 @@ int launch_pair_host(doci_ham *h, const float *hx, float *dx, float *dy, float *
 int ham_build_pair_warp(doci_ham *h);
 bool pair_warp_fits(const doci_ham *h);
 int launch_pair_warp(const doci_ham *h, const float *x, float *y, cudaStream_t s);
-// the same in FP64 accuracy (sigma_pair_warp64.cu)
+// the same in FP64 accuracy (sigma_pair_warp64.cu), where K's digits allow it
+bool pair_warp64_fits(const doci_ham *h);
 int launch_pair_warp64(const doci_ham *h, const double *x, double *y, cudaStream_t s);
 // the reproducible forms: no atomic adds, pair_warp_slabs(h) vectors of D
 // elements of scratch
@@ -193,6 +195,8 @@ int launch_pair_warp64_det(const doci_ham *h, const double *x, double *y, double
 // FP64-accurate pair form in float-float arithmetic, one block per unit (sigma_pair.cu)
 bool pair_ff_fits(const doci_ham *h);
 int launch_pair_ff(const doci_ham *h, const double *x, double *y, cudaStream_t s);
+// its host-buffer form on the same piece and group schedule as launch_pair_host
+int launch_pair_ff_host(doci_ham *h, const double *hx, double *dx, double *dy, double *hy, cudaStream_t s);
 // tensor-core pair form (sigma_tc.cu), FP32 only, sm_103a; x 16-byte aligned.
 // A device wait that runs out writes a nonzero code to *d_err (spin_limit:
 // try_wait iterations per wait).

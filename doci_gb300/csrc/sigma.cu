@@ -1028,9 +1028,9 @@ int launch_sigma(const doci_ham *h, const void *x, void *y, int precision, cudaS
     case 4:
       return f64 ? launch_rowx<double>(h, x, y, st, 1) : launch_rowx<float>(h, x, y, st, 1);
     case 9:
-      // the pair form where it fits, else the phase-ordered row pass, both in float-float
-      // from 10 orbitals on the warp-per-unit form
-      if (pair_warp_fits(h))
+      // from 10 orbitals on the warp-per-unit form where K's digits allow it, else
+      // in float-float the pair form where it fits or the phase-ordered row pass
+      if (pair_warp64_fits(h))
         return launch_pair_warp64(h, static_cast<const double *>(x), static_cast<double *>(y), st);
       if (pair_ff_fits(h)) return launch_pair_ff(h, static_cast<const double *>(x), static_cast<double *>(y), st);
       return launch_rowx_ff(h, static_cast<const double *>(x), static_cast<double *>(y), st);
@@ -1071,7 +1071,7 @@ int multi_method_auto(const doci_ham *h, int precision) {
 // the gather kernel.)
 constexpr size_t kDetMaxBytes = size_t(5) << 30;
 bool det_fits(const doci_ham *h, size_t elem) {
-  return h->sigma_kernel == 0 && !h->d_nbr && pair_warp_fits(h) &&
+  return h->sigma_kernel == 0 && !h->d_nbr && (elem == 8 ? pair_warp64_fits(h) : pair_warp_fits(h)) &&
          static_cast<size_t>(pair_warp_slabs(h)) * h->D * elem <= kDetMaxBytes;
 }
 // *done = false: there is no memory for the scratch

@@ -523,6 +523,42 @@ unsigned init_grid(uint64_t n) {
   return static_cast<unsigned>(std::min((n + 255) / 256, cap));
 }
 
+template <int NO>
+int launch_pair_ff_host_no(doci_ham *h, const double *hx, double *dx, double *dy, double *hy, cudaStream_t st) {
+  int per_sm = 1;
+  int r = kernel_blocks(reinterpret_cast<const void *>(sigma_pair_ff_kernel<NO>), kPairThreads, 0, &per_sm);
+  if (r != DOCI_OK) return r;
+  const int slots = device_sm_count() * per_sm;
+  ff *xf = nullptr;
+  DOCI_CUDA(cudaMallocAsync(&xf, sizeof(ff) * static_cast<size_t>(h->D), st));
+  const uint2 *blocks = reinterpret_cast<const uint2 *>(h->d_pblocks_host);
+  r = run_host_schedule<double>(
+      h, hx, dx, dy, hy, st,
+      [&](uint64_t a, uint64_t n, cudaStream_t s) {
+        pair_init64_kernel<<<init_grid(n), 256, 0, s>>>(static_cast<uint32_t>(n), h->d_diag + a, dx + a, dy + a,
+                                                         xf + a);
+        DOCI_CUDA(cudaGetLastError());
+        return static_cast<int>(DOCI_OK);
+      },
+      [&](int first, int count, cudaStream_t s) {
+        const PairShape ps{h->D, h->L, h->N, h->split, h->L - h->split, count};
+        sigma_pair_ff_kernel<NO><<<std::min(slots, count), kPairThreads, 0, s>>>(
+            ps, blocks + first, h->d_rowstart, h->d_binom, h->d_Kmir64, h->d_ins_t, h->d_tab_off, xf, dy);
+        DOCI_CUDA(cudaGetLastError());
+        return static_cast<int>(DOCI_OK);
+      });
+  // the side stream's groups read xf: st is ordered after them (the
+  // schedule's own join is skipped when it returns early with an error)
+  if (r != DOCI_OK && h->side_stream) {
+    cudaEventRecord(h->side_ev, h->side_stream);
+    cudaStreamWaitEvent(st, h->side_ev, 0);
+  }
+  const cudaError_t ef = cudaFreeAsync(xf, st);
+  if (r != DOCI_OK) return r;
+  DOCI_CUDA(ef);
+  return DOCI_OK;
+}
+
 }  // namespace
 
 int launch_pair_host(doci_ham *h, const float *hx, float *dx, float *dy, float *hy, cudaStream_t st) {
@@ -547,6 +583,15 @@ int launch_pair_host(doci_ham *h, const float *hx, float *dx, float *dy, float *
         DOCI_CUDA(cudaGetLastError());
         return static_cast<int>(DOCI_OK);
       });
+}
+
+int launch_pair_ff_host(doci_ham *h, const double *hx, double *dx, double *dy, double *hy, cudaStream_t st) {
+  if (!pair_ff_fits(h) || !h->d_pblocks_host || h->host_steps.empty()) return DOCI_ERR_INVALID;
+  const int no = h->L - h->N + 1;
+  if (no <= 8) return launch_pair_ff_host_no<8>(h, hx, dx, dy, hy, st);
+  if (no <= 17) return launch_pair_ff_host_no<17>(h, hx, dx, dy, hy, st);
+  if (no <= 24) return launch_pair_ff_host_no<24>(h, hx, dx, dy, hy, st);
+  return launch_pair_ff_host_no<32>(h, hx, dx, dy, hy, st);
 }
 
 bool pair_ff_fits(const doci_ham *h) { return pair_fits(h) && h->L - h->N + 1 <= 32; }

@@ -1,6 +1,7 @@
 // sigma_pair_warp64.cu -- FP64-accurate sigma in the (N-1)-pair form, one warp
 // per unit, the product with K in exact integer arithmetic on the
-// 5th-generation tensor cores.  This is what kind 9 runs from 10 orbitals on.
+// 5th-generation tensor cores.  This is what kind 9 runs from 10 orbitals on,
+// where K allows it (ham_build_kdigits).
 //
 // The tiling, unit lists and tables are those of the FP32 form
 // (sigma_pair_warp.cu).  The product Y_S = X_S K of a set needs about 50 bits.
@@ -12,22 +13,24 @@
 // open slots is an integer that FP32 accumulates exactly (Ozaki, Ogita, Oishi
 // and Rump, "Error-free transformations of matrix multiplication by using fast
 // routines of matrix multiplication and its applications", 2012).  Digits i of
-// X and j of K go into the accumulator of i + j = 2..6: digit i of X multiplies
-// digits 1..6-i of K in one MMA of 32 (6 - i) columns.  |x_1| <= 512 and the
-// host's check of K's digits keep the accumulators of i + j = 2 and 3 below
-// 2^24 for any X; those of the smaller sums could round only if the digits'
-// signs conspired, and then by 2^-44 of the largest sum.  What is cut is below
-// 2^-51 of the largest |x| |K|.  The five sums are put together as a float
+// X and j of K go into the accumulator of i + j = 2..6, digit 2 times digit 2 into
+// one of its own.  |x_1| <= 512 and the host's check of K's digits keep the
+// accumulators of i + j = 2, 3 and 4 below 2^24 for any X (with 2 x 2 in the
+// accumulator of 4 a constant K of 24 open slots passed 2^24, at 1.5e-13); those of
+// the smaller sums could round only if the digits' signs conspired, and then by
+// 2^-55 of the largest |x| |K|.  What is cut is below
+// 2^-51 of the largest |x| |K|.  The six sums are put together as a float
 // pair with exact rounding errors.  The own row's sums stay float pairs in
 // shared memory; what leaves the SM is widened to double by integer
 // operations and added with FP64 atomics to sigma = diag x.
 //
-// Tensor memory holds two tiles (five digits of X: 80 columns, five
-// accumulators: 160), so that warps 0-7 gather, cut and hand over the next
-// tile of a slot while warps 8-15 read and scatter the one before.
+// Tensor memory holds two tiles (four digits of X: 64 columns, six
+// accumulators: 192; the fifth digits lie in shared memory), so that warps 0-7
+// gather, cut and hand over the next tile of a slot while warps 8-15 read and
+// scatter the one before.
 //
-// Measured: L=28 N=14 7.33 -> 3.46 ms, L=32 N=16 134.6 -> 53.7 ms, L=23 N=9
-// 159 -> 79 us, L=18 N=9 46 -> 22 us, against one unit per block with float
+// Measured: L=28 N=14 7.33 -> 3.84 ms, L=23 N=9 159 -> 84 us (3.58 ms and 80 us
+// with 2 x 2 in the accumulator of 4), against one unit per block with float
 // pairs on the FP32 units; the hop sums' error against FP64 sums 2.0e-15 to
 // 3.3e-15 of their norm, from 3.5e-15 to 5.4e-15.  Bound by instruction issue
 // (1,870 warp instructions per 32 sets, 60 % of the issue slots).
@@ -50,14 +53,19 @@ namespace {
 
 constexpr int kSlots = 2;                   // tiles in flight
 constexpr int kThreads64 = 2 * 128 * kSlots;
-constexpr uint32_t kTmemCols = 512;         // per slot: A 5 x 16 (0..79) | exponents (80) | D 5 x 32 (96..255)
-constexpr int kColE = 80, kColD = 96;
+constexpr uint32_t kTmemCols = 512;         // per slot: A digits 1-4, 16 each (0..63) | D 6 x 32 (64..255)
+// the accumulators of i + j = 2, 3, 4 (without 2 + 2), 5, 6 and of digits 2 and 2
+constexpr int kColD = 64, kCol22 = kColD + 5 * 32;
 // tcgen05 instruction descriptor: D FP32, A and B FP16, both K-major, M = 128
 __host__ __device__ constexpr uint32_t idesc16(uint32_t n) {
   return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
-constexpr int kOffBar = 160 * 128;          // after K: 5 digits x 32 rows of 32 FP16 (64 of 128 bytes), swizzled
-constexpr int kOffStart = kOffBar + 128;
+// after K (5 digits x 32 rows of 32 FP16, 64 of 128 bytes, swizzled): a slot's
+// fifth digits of X, 128 rows of the same form
+constexpr int kOffX5 = 160 * 128, kX5Bytes = 128 * 128;
+constexpr int kOffBar = kOffX5 + kSlots * kX5Bytes;
+constexpr int kOffExp = kOffBar + 128;      // the sets' exponents: two tiles of 128 per slot
+constexpr int kOffStart = kOffExp + kSlots * 2 * 128 * 4;
 constexpr int kOffCells = kOffStart + 4 * 24 * (kThreads64 / 32);
 constexpr size_t kMinSmem = 120 * 1024;     // one block per SM: it allocates all of the tensor memory
 
@@ -113,6 +121,16 @@ __device__ __forceinline__ void red64_if(double *p, double v, uint32_t on) {
                "r"(on)
                : "memory");
 }
+__device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+// D = A B (+ D), A in tensor memory or, by its descriptor, in shared memory
+__device__ __forceinline__ void mma_f16_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(id), "r"(acc));
+}
 __device__ __forceinline__ void mma_f16(uint32_t d, uint32_t a, uint64_t b, uint32_t id, uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -166,7 +184,8 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
   }
   if (tid == 0) {
     for (int i = 0; i < kSlots; ++i) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(base + kOffBar + 8 * i));
+      // a tile's MMAs and the issuing thread (which makes the exponents visible)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(base + kOffBar + 8 * i));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(base + kOffBar + 16 + 8 * i));
       reinterpret_cast<volatile int *>(sm + kOffBar + 64)[i] = 0;
     }
@@ -185,7 +204,9 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
   const uint32_t tmem = *tslot;
   const uint32_t tg = tmem + 256u * slot, tw = tg + (static_cast<uint32_t>(32 * w4) << 16);
   const int nks = (s.L + 15) >> 4;
-  const uint64_t desc = smem_desc(base);
+  const uint64_t desc = smem_desc(base), desc5 = smem_desc(base + kOffX5 + slot * kX5Bytes);
+  const uint32_t row5 = base + kOffX5 + slot * kX5Bytes + (4 * w4 + (lane >> 3)) * 1024 + (lane & 7) * 128;
+  volatile uint32_t *exps = reinterpret_cast<volatile uint32_t *>(sm + kOffExp) + slot * 256 + 32 * w4 + lane;
 
   uint32_t n = 0;  // tiles of this slot so far
   bool ok = true, fail = false;
@@ -288,10 +309,12 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
             tst8(tw + 16 + 8 * hf, d2);
             tst8(tw + 32 + 8 * hf, d3);
             tst8(tw + 48 + 8 * hf, d4);
-            tst8(tw + 64 + 8 * hf, d5);
+            sts128(row5 + (((2 * hf) ^ (lane & 7)) << 4), d5[0], d5[1], d5[2], d5[3]);
+            sts128(row5 + (((2 * hf + 1) ^ (lane & 7)) << 4), d5[4], d5[5], d5[6], d5[7]);
           }
-          tst1(tw + kColE + (n & 1u), eb);
+          exps[128 * (n & 1u)] = eb;
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           fence_before();
         }
         if (group_meet(slot, fail)) {
@@ -303,16 +326,27 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
           if (n > 0 && !warp_wait(bar_free, (n - 1) & 1u, s.spin_limit, abort_flag, err, 32)) fail = true;
           if (!fail && lane == 0) {
             fence_after();
-            // digit i of X times digits 1..6-i of K (128-byte rows, 32 rows per
-            // digit): into the accumulators of i + j = i + 1 .. 6
+            // digit i of X times digits 1..6-i of K (32 rows of 128 bytes per
+            // digit) into the accumulators of i + j; 2 x 2 apart
+            auto kd = [&](int j, int ks) { return desc + 256 * (j - 1) + 2 * ks; };
+            auto col = [&](int g) { return tg + kColD + 32 * (g - 2); };
 #pragma unroll
-            for (int i = 0; i < 5; ++i)
+            for (int ks = 0; ks < 2; ++ks)
+              if (ks < nks) mma_f16(col(2), tg + 8 * ks, kd(1, ks), idesc16(160), ks);
 #pragma unroll
-              for (int ks = 0; ks < 2; ++ks)
-                if (ks < nks)
-                  mma_f16(tg + kColD + 32 * i, tg + 16 * i + 8 * ks, desc + 2 * ks, idesc16(160 - 32 * i), i + ks > 0);
+            for (int ks = 0; ks < 2; ++ks)
+              if (ks < nks) {
+                const uint32_t x2 = tg + 16 + 8 * ks;
+                mma_f16(col(3), x2, kd(1, ks), idesc16(32), 1);
+                mma_f16(tg + kCol22, x2, kd(2, ks), idesc16(32), ks);
+                mma_f16(col(5), x2, kd(3, ks), idesc16(64), 1);
+                mma_f16(col(4), tg + 32 + 8 * ks, kd(1, ks), idesc16(96), 1);
+                mma_f16(col(5), tg + 48 + 8 * ks, kd(1, ks), idesc16(64), 1);
+                mma_f16_ss(col(6), desc5 + 2 * ks, kd(1, ks), idesc16(32), 1);
+              }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_done)
                          : "memory");
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_done) : "memory");
           }
           __syncwarp();
         }
@@ -332,21 +366,24 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
         }
         fence_after();
         float yh[32], yl[32];
-        const uint32_t eb = tld1(tw + kColE + (n & 1u));
+        const uint32_t eb = exps[128 * (n & 1u)];
         const f2 q11 = pk(0x1p-11f, 0x1p-11f);
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch) {
-          float D[5][8];
+          float D[6][8];
 #pragma unroll
-          for (int g = 0; g < 5; ++g) tld8(tw + kColD + 32 * g + 8 * ch, D[g]);
+          for (int g = 0; g < 6; ++g) tld8(tw + kColD + 32 * g + 8 * ch, D[g]);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           // sum_g D_g 2^(-11 (g - 1)) as a pair: each step's rounding error is
-          // exact and carried (D_g are integers up to 2^25)
+          // exact and carried (the first four are integers below 2^24, so the sum
+          // of the two of i + j = 4 is off by at most one)
 #pragma unroll
           for (int i = 0; i < 8; i += 2) {
-            const f2 D1 = pk(D[0][i], D[0][i + 1]), D2 = pk(D[1][i], D[1][i + 1]), D3 = pk(D[2][i], D[2][i + 1]);
+            const f2 D1 = pk(D[0][i], D[0][i + 1]), D2 = pk(D[1][i], D[1][i + 1]);
+            const f2 D4 = pk(D[2][i], D[2][i + 1]), D22 = pk(D[5][i], D[5][i + 1]), D3 = addp(D4, D22);
+            const f2 off = subp(D22, subp(D3, D4));
             const f2 a = fma2(pk(D[4][i], D[4][i + 1]), q11, pk(D[3][i], D[3][i + 1]));
-            const f2 bh = fma2(a, q11, D3), bl = fma2(a, q11, subp(D3, bh));
+            const f2 bh = fma2(a, q11, D3), bl = addp(fma2(a, q11, subp(D3, bh)), off);
             const f2 ch2 = fma2(bh, q11, D2), cl = fma2(bl, q11, fma2(bh, q11, subp(D2, ch2)));
             const f2 dh = fma2(ch2, q11, D1), dl = fma2(cl, q11, fma2(ch2, q11, subp(D1, dh)));
             const f2 h = addp(dh, dl), l = subp(dl, subp(h, dh));
@@ -443,49 +480,66 @@ int launch_p(const doci_ham *h, const PwShape &s, const ff *x, double *y, double
 }  // namespace
 
 // K (mirrored orbitals) as five signed digits of eleven bits, below 1/4:
-// K = 2^exp sum_j k_j 2^(-11 j), FP16, digit j at [j - 1][32][32]
+// K = 2^exp sum_j k_j 2^(-11 j), FP16, digit j at [j - 1][32][32].  The
+// accumulators of i + j = 2, 3 and 4 (2 x 2 apart) have to hold their sums
+// exactly whatever X: |x_1| <= 512, |x_i| <= 1024 over the L - N + 1 open slots of a
+// set.  Where K's digits do not allow that, other digits are tried (a larger
+// exponent, at a bit of K each); kdig_ok is false when none do.
 int ham_build_kdigits(doci_ham *h) {
   const int L = h->L, open = L - h->N + 1;
   double big = 0;
-  for (double k : h->Kp) big = std::max(big, std::fabs(k));
+  bool finite = true;
+  for (double k : h->Kp) {
+    big = std::max(big, std::fabs(k));
+    finite = finite && std::isfinite(k);
+  }
+  h->kdig_ok = false;
+  if (!finite) return DOCI_OK;
   int ex = 0;
-  if (big > 0 && std::isfinite(big)) std::frexp(big, &ex);  // big < 2^ex
+  std::frexp(big, &ex);  // big < 2^ex
+  if (ex < -100 || ex > 100) return DOCI_OK;  // (the kernel's scale factors are floats)
   std::vector<uint16_t> dig(5 * 1024, 0);
-  for (h->kdig_exp = ex + 2;; ++h->kdig_exp) {
-    // the accumulators of the first two digit sums have to hold them exactly:
-    // |x_1| <= 512, |x_2| <= 1024 over the at most `open` slots of a set
+  for (h->kdig_exp = ex + 2; !h->kdig_ok && h->kdig_exp <= ex + 6; ++h->kdig_exp) {
     double worst = 0;
     for (int a = 0; a < L; ++a) {
-      std::vector<double> row;
+      std::vector<double> sums[3];
       for (int b = 0; b < L; ++b) {
-        double v = std::ldexp(h->Kp[(L - 1 - a) * L + (L - 1 - b)], -h->kdig_exp), k12[2] = {0, 0};
+        double v = std::ldexp(h->Kp[(L - 1 - a) * L + (L - 1 - b)], -h->kdig_exp), k[5];
         for (int j = 0; j < 5; ++j) {
           v *= 2048;
           const double d = std::nearbyint(v);
           v -= d;
-          if (j < 2) k12[j] = std::fabs(d);
+          k[j] = std::fabs(d);
           const __half hd = __float2half(static_cast<float>(d));
           dig[j * 1024 + a * 32 + b] = *reinterpret_cast<const uint16_t *>(&hd);
         }
-        row.push_back(1024 * k12[0] + 512 * k12[1]);
+        sums[0].push_back(1024 * k[0] + 512 * k[1]);  // (i + j = 2, 512 k[0], is below it)
+        sums[1].push_back(1024 * k[0] + 512 * k[2]);
+        sums[2].push_back(1024 * k[1]);
       }
-      std::sort(row.rbegin(), row.rend());
-      double sum = 0;
-      for (int t = 0; t < open && t < L; ++t) sum += row[t];
-      worst = std::max(worst, sum);
+      for (auto &s : sums) {
+        std::sort(s.rbegin(), s.rend());
+        double sum = 0;
+        for (int t = 0; t < open && t < L; ++t) sum += s[t];
+        worst = std::max(worst, sum);
+      }
     }
-    // (the second digits alone stay below it: 31 x 512 x 1024)
-    if (!(worst > 16777216.0) || h->kdig_exp >= ex + 6) break;
+    // (a margin for the sum of the two of i + j = 4, formed from their rounded sum)
+    h->kdig_ok = worst <= 16777216.0 - 1024.0;
   }
+  --h->kdig_exp;
+  if (!h->kdig_ok) return DOCI_OK;
   DOCI_CUDA(cudaMallocAsync(&h->d_kdig, dig.size() * sizeof(uint16_t), h->stream));
   DOCI_CUDA(cudaMemcpyAsync(h->d_kdig, dig.data(), dig.size() * sizeof(uint16_t), cudaMemcpyHostToDevice, h->stream));
   return DOCI_OK;
 }
 
+bool pair_warp64_fits(const doci_ham *h) { return pair_warp_fits(h) && h->kdig_ok; }
+
 namespace {
 template <bool DET>
 int launch64(const doci_ham *h, const double *x, double *y, double *slab, cudaStream_t st) {
-  if (!pair_warp_fits(h)) return DOCI_ERR_INVALID;
+  if (!pair_warp64_fits(h)) return DOCI_ERR_INVALID;
   ff *xf = nullptr;
   DOCI_CUDA(cudaMallocAsync(&xf, sizeof(ff) * static_cast<size_t>(h->D), st));
   init64_kernel<<<static_cast<unsigned>(std::min<uint64_t>((static_cast<uint64_t>(h->D) + 255) / 256,

@@ -509,3 +509,39 @@ def test_sigma_neighbour_table(L, N, seed, nv, synth, dg):
                 ref = o.matvec(X[v])
                 assert torch.equal(y1[:D], yb[v, :D]) and bool((yb[v, D:] == 7.0).all() and (y1[D:] == 7.0).all())
                 assert np.abs(y1[:D].double().cpu().numpy() - ref).max() <= tol * max(np.abs(ref).max(), 1e-300)
+
+
+def pair_integrals(h1, K):
+    """Integrals with the pair hops K (symmetric) and no Coulomb part: the
+    diagonal is sum_i 2 h_i - sum_{i,j} K_ij over the pairs."""
+    L = len(h1)
+    eri = np.zeros((L, L, L, L))
+    i, j = np.nonzero(~np.eye(L, dtype=bool))
+    for a, b, c, d in ((i, j, i, j), (i, j, j, i)):
+        eri[a, b, c, d] = K[i, j]
+    return np.diag(np.asarray(h1, dtype=np.float64)), eri
+
+
+@pytest.mark.parametrize("L,N", [(27, 3), (32, 2), (19, 3)])
+def test_fp64_pair_form_constant_hops(L, N, dg):
+    """A pure pairing Hamiltonian (constant K) on constant vectors with 17 to 31
+    open slots, whose digits all add up with one sign: within 2^-45 of the sum
+    of the terms' magnitudes.  (What is cut is below 2^-51, a set's product is
+    rounded to 2^-48, and the own rows' pairs of floats to 2^-47 per addition.)"""
+    torch = torch_cuda()
+    rng = np.random.default_rng(L)
+    for k in range(8):
+        c = rng.uniform(0.5, 1)
+        K = c * (1 - np.eye(L))
+        with dg.Hamiltonian.from_integrals(L, N, 0.0, *pair_integrals(np.linspace(-1, 1, L), K)) as h:
+            h.set_sigma_kernel("rowff")
+            assert h.sigma_plan(dg.FP64)[0] == 9
+            dx = h.diagonal().astype(np.longdouble)
+            y = torch.empty(h.D, dtype=torch.float64, device="cuda")
+            for v in rng.uniform(0.5, 1, 12):
+                x = torch.full((h.D,), v, dtype=torch.float64, device="cuda")
+                h.sigma_device(x.data_ptr(), y.data_ptr(), dg.FP64)
+                torch.cuda.synchronize()
+                hops = N * (L - N) * np.longdouble(c) * np.longdouble(v)
+                err = np.abs(y.cpu().numpy() - (dx * v + hops))
+                assert (err <= 2.0 ** -45 * (np.abs(dx * v) + hops)).all(), (k, v, float((err / hops).max()))
