@@ -1005,15 +1005,16 @@ __global__ void __launch_bounds__(kEigT) eng_eig(EArgs a) {
     __syncthreads();
   }
   eig_jacobi64(A, Vv, n, 1e-30f, 1e-34, 100, rot, part);
-  if (tid < n) {  // rank of each eigenvalue (ties by index)
-    const double w = A[tid * (kLdA + 1)];
+  if (tid < n) {  // rank of each eigenvalue (ties by index; NaNs, from integrals that are not finite, last)
+    auto before = [&](int i, int j) {
+      const double wi = A[i * (kLdA + 1)], wj = A[j * (kLdA + 1)];
+      const bool ni = isnan(wi), nj = isnan(wj);
+      return wi < wj || (!ni && nj) || ((wi == wj || (ni && nj)) && i < j);
+    };
     int rank = 0;
-    for (int j = 0; j < n; ++j) {
-      const double wj = A[j * (kLdA + 1)];
-      rank += (wj < w || (wj == w && j < tid)) ? 1 : 0;
-    }
+    for (int j = 0; j < n; ++j) rank += before(j, tid) ? 1 : 0;
     idx[rank] = tid;
-    wv[rank] = scalbn(w, ex);
+    wv[rank] = scalbn(A[tid * (kLdA + 1)], ex);
   }
   __syncthreads();
   for (int i = warp; i < n; i += kEigT / 32) {

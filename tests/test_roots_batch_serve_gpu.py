@@ -167,3 +167,23 @@ def test_orthogonalisation_step_edges(L, N, nroots, mode, synth, dg):
     assert r["status"] == 0 and r["converged"] == 1
     assert np.allclose(r["energies"][:k], ref, atol=1e-7)
     assert np.abs(v @ v.T - np.eye(k)).max() < 1e-6
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("nroots", [1, 2, 8])
+def test_integrals_not_finite(nroots, bad, synth, dg):
+    """An integral that is not finite makes the subspace matrix and its
+    eigenvalues NaN: they are ordered all the same (every one has a place), the
+    solve ends, and the next one on the device is as ever."""
+    from doci_gb300.fcidump import raw_integrals
+    one, two = raw_integrals(10, 160)
+    two = np.array(two, dtype=np.float64).reshape(10, 10, 10, 10)
+    for i, j, k, l in ((0, 9, 0, 9), (0, 9, 9, 0), (9, 0, 0, 9), (9, 0, 9, 0)):
+        two[i, j, k, l] = bad
+    with dg.Hamiltonian.from_integrals(10, 5, 0.0, one, two) as h:
+        r = dg.solve_roots(h, nroots=nroots, tol=1e-7, mode="fp64", max_vec=16, max_its=20)
+    assert r["status"] == 0 and not np.isfinite(r["energies"][0])
+    p = synth(10, 5, 161)
+    with dg.Hamiltonian.from_fcidump(p) as h:
+        r = dg.solve_roots(h, nroots=2, tol=1e-7, mode="fp64")
+    assert r["converged"] == 1 and np.allclose(r["energies"][:2], dense_eigs(p, 2), atol=1e-9)
