@@ -485,12 +485,23 @@ int launch_p(const doci_ham *h, const PwShape &s, const ff *x, double *y, double
 // exactly whatever X: |x_1| <= 512, |x_i| <= 1024 over the L - N + 1 open slots of a
 // set.  Where K's digits do not allow that, other digits are tried (a larger
 // exponent, at a bit of K each); kdig_ok is false when none do.
+//
+// The digits keep K to 2^-56 of 2^exp, the float-pair kernel each element of K
+// to itself, so small elements beside large ones have fewer bits here.  kdig_ok
+// asks that 2^(exp - 2), which is the power of two above the largest element (or
+// up to four bits more), be at most 18 times the smallest one that is not
+// zero: up to there this form's products are as exact, element by element
+// (largest error of a product with that smallest element, emulated, against
+// float pairs: 16 times 1.1e-14 and 1.4e-14, 18 times 1.25e-14 and 1.3e-14, 20
+// times 1.35e-14 and 1.2e-14; 1e4 times 3e-12).  A K that is graded more (core
+// orbitals, separate fragments) runs the float-pair kernel.
 int ham_build_kdigits(doci_ham *h) {
   const int L = h->L, open = L - h->N + 1;
-  double big = 0;
+  double big = 0, small = INFINITY;
   bool finite = true;
   for (double k : h->Kp) {
     big = std::max(big, std::fabs(k));
+    if (k != 0) small = std::min(small, std::fabs(k));
     finite = finite && std::isfinite(k);
   }
   h->kdig_ok = false;
@@ -500,6 +511,7 @@ int ham_build_kdigits(doci_ham *h) {
   if (ex < -100 || ex > 100) return DOCI_OK;  // (the kernel's scale factors are floats)
   std::vector<uint16_t> dig(5 * 1024, 0);
   for (h->kdig_exp = ex + 2; !h->kdig_ok && h->kdig_exp <= ex + 6; ++h->kdig_exp) {
+    if (big > 0 && std::ldexp(1.0, h->kdig_exp - 2) > 18 * small) break;
     double worst = 0;
     for (int a = 0; a < L; ++a) {
       std::vector<double> sums[3];
@@ -527,8 +539,8 @@ int ham_build_kdigits(doci_ham *h) {
     // (a margin for the sum of the two of i + j = 4, formed from their rounded sum)
     h->kdig_ok = worst <= 16777216.0 - 1024.0;
   }
-  --h->kdig_exp;
   if (!h->kdig_ok) return DOCI_OK;
+  --h->kdig_exp;
   DOCI_CUDA(cudaMallocAsync(&h->d_kdig, dig.size() * sizeof(uint16_t), h->stream));
   DOCI_CUDA(cudaMemcpyAsync(h->d_kdig, dig.data(), dig.size() * sizeof(uint16_t), cudaMemcpyHostToDevice, h->stream));
   return DOCI_OK;

@@ -545,3 +545,89 @@ def test_fp64_pair_form_constant_hops(L, N, dg):
                 hops = N * (L - N) * np.longdouble(c) * np.longdouble(v)
                 err = np.abs(y.cpu().numpy() - (dx * v + hops))
                 assert (err <= 2.0 ** -45 * (np.abs(dx * v) + hops)).all(), (k, v, float((err / hops).max()))
+
+
+def exact_sigma(h, L, K, X):
+    """sigma of the vectors X in long double, with the handle's diagonal, and
+    the sum of its terms' magnitudes, for small spaces."""
+    torch = torch_cuda()
+    bits = torch.empty(h.D, dtype=torch.int32, device="cuda")
+    h.bitstrings_device(0, h.D, bits.data_ptr())
+    bits = bits.cpu().numpy().astype(np.int64) & 0xffffffff
+    at = {int(b): r for r, b in enumerate(bits)}
+    y = h.diagonal().astype(np.longdouble) * X
+    mag = np.abs(y)
+    for r, b in enumerate(int(v) for v in bits):
+        for i in range(L):
+            for a in range(L):
+                if b >> i & 1 and not b >> a & 1:
+                    t = np.longdouble(K[i, a]) * X[:, at[b ^ (1 << i) ^ (1 << a)]]
+                    y[:, r] += t
+                    mag[:, r] += np.abs(t)
+    return y, mag
+
+
+def graded_hops(L, how, f, rng):
+    """K between 1/2 and 1, graded by f: "core" K_ij s_i s_j with s falling from 1
+    to f over the orbitals, "small" with every other orbital's row at f, "fragments" two halves
+    with f between them."""
+    K = rng.uniform(0.5, 1, (L, L))
+    K = np.triu(K, 1) + np.triu(K, 1).T
+    if how == "core":
+        s = f ** (np.arange(L) / (L - 1))
+        return K * s[:, None] * s[None, :]
+    if how == "small":
+        s = np.where(np.arange(L) % 2, f, 1.0)
+        return K * np.minimum(s[:, None], s[None, :])
+    half = np.arange(L) < L // 2
+    return np.where(half[:, None] == half[None, :], K, f * K)
+
+
+@pytest.mark.parametrize("how,f", [("core", 0.5), ("core", 1e-2), ("core", 1e-5), ("small", 1e-2), ("small", 1e-4),
+                                   ("small", 1e-10), ("fragments", 1e-1), ("fragments", 1e-6)])
+def test_fp64_pair_form_graded_hops(how, f, dg):
+    """Every component of the FP64-accurate pair form, also one that only small
+    elements of K reach (one-hot vectors), to the float pairs' accuracy: seven
+    open slots at 2^-47 each, 2^-44 of the sum of the terms' magnitudes."""
+    torch = torch_cuda()
+    L, N = 12, 6
+    rng = np.random.default_rng(12)
+    K = graded_hops(L, how, f, rng)
+    with dg.Hamiltonian.from_integrals(L, N, 0.0, *pair_integrals(np.linspace(-1, 1, L), K)) as h:
+        h.set_sigma_kernel("rowff")
+        assert h.sigma_plan(dg.FP64)[0] == 9
+        X = np.concatenate([np.eye(h.D)[[0, h.D // 3, h.D - 1]], rng.standard_normal((2, h.D))])
+        ref, mag = exact_sigma(h, L, K, X)
+        y = torch.empty(h.D, dtype=torch.float64, device="cuda")
+        for v, x in enumerate(X):
+            xd = torch.from_numpy(x).cuda()
+            h.sigma_device(xd.data_ptr(), y.data_ptr(), dg.FP64)
+            torch.cuda.synchronize()
+            assert (np.abs(y.cpu().numpy() - ref[v]) <= 2.0 ** -44 * mag[v]).all(), v
+
+
+@pytest.mark.parametrize("how,f", [("core", 0.5), ("small", 1e-8)])
+def test_fp64_graded_hops_automatic(how, f, dg):
+    """The same on a space without a neighbour table, through the automatic
+    single and block sigmas: on one-hot vectors every element of sigma is one product, as
+    the FP64 row pass forms it."""
+    torch = torch_cuda()
+    L, N = 20, 10
+    K = graded_hops(L, how, f, np.random.default_rng(20))
+    with dg.Hamiltonian.from_integrals(L, N, 0.0, *pair_integrals(np.linspace(-1, 1, L), K)) as h:
+        D = h.D
+        x = torch.zeros((3, D), dtype=torch.float64, device="cuda")
+        x[torch.arange(3), torch.tensor([0, D // 2, D - 1])] = 1.0
+        out = []
+        for kind in ("rowx", "auto", "block"):
+            h.set_sigma_kernel("auto" if kind == "block" else kind)
+            y = torch.full((3, D), float("nan"), dtype=torch.float64, device="cuda")
+            if kind == "block":
+                h.sigma_block_device(x.data_ptr(), D, y.data_ptr(), D, 3, dg.FP64)
+            else:
+                for v in range(3):
+                    h.sigma_device(x[v].data_ptr(), y[v].data_ptr(), dg.FP64)
+            torch.cuda.synchronize()
+            out.append(y)
+        for y in out[1:]:
+            assert bool(((y - out[0]).abs() <= 2.0 ** -46 * out[0].abs()).all())
