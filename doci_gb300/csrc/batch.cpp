@@ -41,7 +41,8 @@ double clock_s() {
 int solve_roots(doci_ham *h, const doci_batch_opts &o, cudaStream_t st, doci_root_result *res, double *vecs) {
   if (o.nroots < 1 || o.nroots > 8 || static_cast<uint64_t>(o.nroots) > h->D) return DOCI_ERR_INVALID;
   double *const v[1] = {vecs};
-  return engine_solve(1, &h, o, st, res, v);
+  const int s = engine_solve(1, &h, o, st, res, v);
+  return s ? s : res->status;
 }
 
 int64_t roots_footprint(int L, int N, const doci_batch_opts &o) {
@@ -377,12 +378,12 @@ int doci_batch_solve(int n, doci_ham *const *hams, const doci_batch_opts *opts, 
     int s = (used > budget) ? DOCI_ERR_ADMISSION : engine_solve(j - i, hams + i, o, st, results + i, nullptr);
     const double te = clock_s() - t0;
     for (int k = i; k < j; ++k) {
-      results[k].status = s;
+      if (s != DOCI_OK) results[k].status = s;
+      if (results[k].status != DOCI_OK && first_err == DOCI_OK) first_err = results[k].status;
       results[k].queued_s = 0;
       results[k].start_s = ts;
       results[k].end_s = te;
     }
-    if (s != DOCI_OK && first_err == DOCI_OK) first_err = s;
     i = j;
   }
   cudaStreamDestroy(st);

@@ -759,6 +759,7 @@ int davidson(double *result, double *energy, int max_vectors, int keep_deflate, 
   DavidsonOut out;
   st = davidson_run<double>(ctx.op, n, ctx.d_diag, static_cast<double *>(t.p), a, ctx.st, &out,
                             static_cast<double *>(x.p));
+  if (!st && ctx.h) st = ham_device_error(ctx.h, ctx.st);
   if (st) die_cuda("davidson", st);
   if (cudaMemcpy(result, x.p, sizeof(double) * n, cudaMemcpyDeviceToHost) != cudaSuccess)
     die_cuda("davidson", DOCI_ERR_CUDA);
@@ -786,6 +787,7 @@ int ray_q(void (*matvec)(double *, double *, void *), double *M, double *vec, in
   a.print = 1;
   CgOut out;
   st = ray_q_run(ctx.op, n, precond ? ctx.d_diag : nullptr, static_cast<double *>(x.p), a, ctx.st, &out);
+  if (!st && ctx.h) st = ham_device_error(ctx.h, ctx.st);
   if (st) die_cuda("ray_q", st);
   if (cudaMemcpy(vec, x.p, sizeof(double) * n, cudaMemcpyDeviceToHost) != cudaSuccess) die_cuda("ray_q", DOCI_ERR_CUDA);
   *energy = out.energy;

@@ -1388,6 +1388,7 @@ int engine_tune(doci_ham *h, int nv, int *dpt_out) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   DOCI_CUDA(cudaGetLastError());
+  if ((s = ham_device_error(h, st))) return s;
   {
     std::lock_guard<std::mutex> lk(g_tile_mu);
     TileChoice c;
@@ -1497,6 +1498,17 @@ int engine_solve(int n, doci_ham *const *hams, const doci_batch_opts &o, cudaStr
       off += h->D;
     }
   };
+  // a device wait that ran out in a large problem's sigmas (its FP32 view shares
+  // the handle's error word)
+  std::vector<int> status(n, DOCI_OK);
+  auto check_waits = [&]() -> int {
+    for (int i : big_idx) {
+      const int e = ham_device_error(hams[i], st);
+      if (e == DOCI_ERR_DEVICE_TIMEOUT) status[i] = e;
+      else if (e) return e;
+    }
+    return DOCI_OK;
+  };
   std::vector<double> e32(static_cast<size_t>(n) * R, 0.0);
   std::vector<int> its32v(n, 0), sig32(n, 0);
   bool have_start = false;  // the FP64 phase starts from the FP32 phase's Ritz vectors
@@ -1554,7 +1566,7 @@ int engine_solve(int n, doci_ham *const *hams, const doci_batch_opts &o, cudaStr
     for (int i = 0; i < n; ++i) P[i].max_its = o.max_its;
     if ((s = upload())) return s;
     s = run_phase_km<float>(a32, nh_max, ntiles, nchunks, st, true, big);
-    if (s) return s;
+    if (s || (s = check_waits())) return s;
     DOCI_CUDA(cudaMemcpyAsync(host_st.data(), dS.p, sizeof(EState) * n, cudaMemcpyDeviceToHost, st));
     DOCI_CUDA(cudaStreamSynchronize(st));
     for (int i = 0; i < n; ++i) {
@@ -1596,7 +1608,7 @@ int engine_solve(int n, doci_ham *const *hams, const doci_batch_opts &o, cudaStr
                             hams[i]->D});
     }
     s = run_phase_km<double>(a64, nh_max, ntiles, nchunks, st, !have_start, big);
-    if (s) return s;
+    if (s || (s = check_waits())) return s;
     DOCI_CUDA(cudaMemcpyAsync(host_st.data(), dS.p, sizeof(EState) * n, cudaMemcpyDeviceToHost, st));
     DOCI_CUDA(cudaStreamSynchronize(st));
   }
@@ -1615,7 +1627,7 @@ int engine_solve(int n, doci_ham *const *hams, const doci_batch_opts &o, cudaStr
     r.iterations_fp32 = its32v[i];
     r.sigmas = es.sigmas + sig32[i];
     r.converged = es.converged;
-    r.status = DOCI_OK;
+    r.status = status[i];
     if (vecs && vecs[i]) {
       DOCI_CUDA(cudaMemcpyAsync(vecs[i], dX.p + off * R, sizeof(double) * hams[i]->D * R, cudaMemcpyDeviceToHost,
                                 st));

@@ -1224,7 +1224,8 @@ int autotune_sigma(doci_ham *h, int precision, int nv, cudaStream_t st, int *cho
   DOCI_CUDA(cudaFreeAsync(buf, st));
   DOCI_CUDA(cudaStreamSynchronize(st));
   if (choice) *choice = best;
-  return best ? DOCI_OK : DOCI_ERR_INVALID;
+  if (!best) return DOCI_ERR_INVALID;
+  return ham_device_error(h, st);
 }
 
 bool sigma_tuned(const doci_ham *h, int precision, int nv) { return tuned_choice(h, precision, nv, false) != 0; }

@@ -197,8 +197,10 @@ int doci_sigma_block(doci_ham *ham, const void *d_X, int64_t ldx, void *d_Y, int
  * requests for 6 and 8 use the automatic choice.  3-9 fall back to 1 when the
  * handle has no row tiling.  Other values: DOCI_ERR_INVALID.  A device wait
  * of kind 6, 8 or 9 that runs out (it never should) is reported as
- * DOCI_ERR_DEVICE_TIMEOUT by the handle's next synchronous call
- * (doci_sigma_host, doci_solve).  For tests and tuning. */
+ * DOCI_ERR_DEVICE_TIMEOUT by the handle's next synchronous call that runs these
+ * kernels or may have (doci_sigma_host, doci_solve, doci_solve_roots and
+ * doci_batch_solve and requests of large spaces, the autotuning calls; davidson, ray_q
+ * and sparse_eigensolve print it and exit).  For tests and tuning. */
 int doci_ham_set_sigma_kernel(doci_ham *ham, int kind);
 
 /* Autotuning: time the sigma paths that fit this handle's shape and keep

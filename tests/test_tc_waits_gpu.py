@@ -95,3 +95,65 @@ def test_warp_wait_limit_reports_timeout(L, N, synth):
     assert [int(v) for k, v in got if k == "status"] == [12] * 6  # DOCI_ERR_DEVICE_TIMEOUT
     assert [int(v) for k, v in got if k == "block"] == [12 if (L, N) == (22, 11) else 0] * 2
     assert all(float(v) <= 2e-6 for k, v in got if k == "after")
+
+
+SOLVE_CHILD = r"""
+import ctypes as C, sys
+import numpy as np
+sys.path.insert(0, {root!r})
+import doci_gb300 as dg
+small, p = {small!r}, {path!r}
+with dg.Hamiltonian.from_fcidump(p) as h, dg.Hamiltonian.from_fcidump(small) as hs:
+    for mode in ("fp64", "mixed"):
+        try:
+            dg.solve_roots(h, nroots=2, max_vec=6, max_its=2, mode=mode)
+        except dg.DociError as e:
+            print("roots", e)
+        st, res = dg.batch_solve([hs, h], nroots=2, max_vec=6, max_its=2, mode=mode)
+        print("batch", st, [r["status"] for r in res])
+    for nvec in (1, 2):
+        try:
+            h.autotune(dg.FP32, nvec)
+            print("tune ok")
+        except dg.DociError as e:
+            print("tune", e)
+    # nothing is left for a later call that ran no such kernel
+    h.set_sigma_kernel("gather")
+    x = np.ones(h.D)
+    print("clean", dg.lib().doci_sigma_host(h.handle, x.ctypes.data_as(C.c_void_p),
+                                            np.empty_like(x).ctypes.data_as(C.c_void_p), dg.FP64))
+if len(sys.argv) > 1:  # the reference's entry points print the error and exit
+    L = dg.lib()
+    dat = C.c_void_p()
+    L.fill_doci_data(p.encode(), C.byref(dat))
+    D = L.doci_get_basis_size(dat)
+    vec = np.zeros(D)
+    vec[0] = 1.0
+    e = C.c_double()
+    L.sparse_eigensolve(vec.ctypes.data_as(C.POINTER(C.c_double)), D, C.byref(e), C.cast(L.doci_matvec, C.c_void_p),
+                        L.doci_get_diagonal(dat), None, 1e-8, 2, sys.argv[1].encode(), 2, 4, dat)
+    print("returned")
+"""
+
+
+@pytest.mark.parametrize("solver", [None, "D", "CG"])
+def test_wait_limit_reaches_the_solvers(solver, synth):
+    """With a wait limit of 0 the solves that run the warp-per-unit kernels (a
+    space large enough for the batch engine to take them) report
+    DOCI_ERR_DEVICE_TIMEOUT, a problem beside them that does not stays fine,
+    and no error is left for a later call."""
+    p, small = synth(25, 12, 73), synth(10, 5, 74)
+    env = dict(os.environ, DOCI_TC_SPIN_LIMIT="0")
+    code = SOLVE_CHILD.format(root=ROOT, path=p, small=small)
+    r = subprocess.run([sys.executable, "-u", "-c", code] + ([solver] if solver else []), capture_output=True, text=True,
+                       env=env, timeout=300)
+    out = r.stdout.splitlines()
+    assert sum(ln.startswith("roots") and "DOCI_ERR_DEVICE_TIMEOUT" in ln for ln in out) == 2, r.stdout + r.stderr
+    assert out.count("batch 12 [0, 12]") == 2, r.stdout
+    assert any(ln.startswith("tune") and "DOCI_ERR_DEVICE_TIMEOUT" in ln for ln in out)
+    assert "clean 0" in out
+    if solver is None:
+        assert r.returncode == 0, r.stderr
+    else:
+        assert r.returncode != 0 and "returned" not in out
+        assert "device wait timed out" in r.stderr + r.stdout
