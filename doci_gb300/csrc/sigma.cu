@@ -946,7 +946,10 @@ int tuned_choice(const doci_ham *h, int precision, int nv, bool allow_pair) {
   return it == g_tuned.end() ? 0 : it->second;
 }
 
-// the FP64 pair form is a candidate of the autotuning from here on
+// the FP64 pair form is a candidate of the autotuning from here on.  (Below, the
+// tuned choice is one of the paths without atomic adds, which the tuning's callers
+// and its test at 184,756 determinants expect; untuned, kind 9 runs there in 38 us,
+// where the tuned choice takes 60.)
 constexpr uint32_t kTunedPairMinD = 1u << 18;
 
 // The path of kind `kind` (0 = the heuristics) for this handle; a kind that
@@ -1141,7 +1144,9 @@ int launch_sigma_multi(const doci_ham *h, const void *x, size_t ldx, void *y, si
   if (nv < 1 || nv > 4 || ldx < h->D || ldy < h->D) return DOCI_ERR_INVALID;
   if (precision != DOCI_FP64 && precision != DOCI_FP32) return DOCI_ERR_INVALID;
   // block sigmas are reproducible from run to run: no atomic adds here
-  int method = h->sigma_kernel == 0 ? tuned_choice(h, precision, nv, false) : 0;
+  // (a tuned nv = 1 is a choice among the single-vector kernels, made without the
+  // reproducible pair form)
+  int method = h->sigma_kernel == 0 && nv > 1 ? tuned_choice(h, precision, nv, false) : 0;
   if (method == 0 && det_fits(h, precision == DOCI_FP64 ? 8 : 4)) {
     bool done;
     const int r = run_det(h, static_cast<const char *>(x), ldx, static_cast<char *>(y), ldy, nv, precision, st, &done);
@@ -1182,10 +1187,9 @@ int autotune_sigma(doci_ham *h, int precision, int nv, cudaStream_t st, int *cho
       int pick = 0;
       for (int kind : {1, 3, 4, 6, 8, 9}) {
         if ((kind == 6 || kind == 8) && (!allow || precision != DOCI_FP32)) continue;
-        // small tuned FP64 shapes keep to the kernels without atomic adds, whose
-        // results repeat bit for bit (they were the fastest there before kind 9
-        // ran on the tensor cores: 184,756 determinants, 60 us against 38 now)
-        if (kind == 9 && (precision != DOCI_FP64 || h->D < kTunedPairMinD)) continue;
+        // kind 9 adds with atomics: not for the callers without the pair forms,
+        // whose results repeat bit for bit
+        if (kind == 9 && (!allow || precision != DOCI_FP64 || h->D < kTunedPairMinD)) continue;
         hm->sigma_kernel = kind;
         const SigmaPlan p = plan_sigma(h, precision, allow != 0);
         if (p.kind != kind) continue;  // the path does not fit this shape

@@ -159,8 +159,9 @@ const double *doci_ham_diagonal_device(const doci_ham *ham);
 int doci_sigma(doci_ham *ham, const void *d_x, void *d_y, int precision, void *stream);
 
 /* Block sigma Y_v = H X_v for v < nv on device buffers: X and Y column-major
- * with leading dimensions ldx, ldy >= D (elements).  Without atomic adds:
- * results repeat bit for bit.  On large spaces one vector after the other in
+ * with leading dimensions ldx, ldy >= D (elements).  Without atomic adds (unless
+ * doci_ham_set_sigma_kernel set kind 9): results repeat bit for bit.  On large
+ * spaces one vector after the other in
  * the pair form with every contribution in a place of its own (stream-ordered
  * scratch of at most min(N, L - 8) x D elements, up to 5 GiB); else, and when
  * there is no memory for that, the neighbour ranks and hop weights of each

@@ -631,3 +631,29 @@ def test_fp64_graded_hops_automatic(how, f, dg):
             out.append(y)
         for y in out[1:]:
             assert bool(((y - out[0]).abs() <= 2.0 ** -46 * out[0].abs()).all())
+
+
+@pytest.mark.parametrize("L,N,seed", [(21, 12, 141), (22, 14, 142)])
+def test_sigma_block_reproducible_after_tuning(L, N, seed, synth, dg):
+    """Block sigmas of one vector and of four and one repeat bit for bit on an FP64
+    shape that was tuned (where the fastest single sigma adds with atomics), and
+    agree with the oracle."""
+    torch = torch_cuda()
+    p = synth(L, N, seed)
+    o = oracle.Ham(p)
+    with dg.Hamiltonian.from_fcidump(p) as h:
+        h.autotune(dg.FP64, 1)
+        D = h.D
+        X = np.random.default_rng(seed).standard_normal((5, D))
+        xb = torch.from_numpy(X).cuda()
+        refs = [o.matvec(x) for x in X]
+        for nv in (1, 5):
+            outs = []
+            for _ in range(4):
+                y = torch.empty((nv, D), dtype=torch.float64, device="cuda")
+                h.sigma_block_device(xb.data_ptr(), D, y.data_ptr(), D, nv, dg.FP64)
+                torch.cuda.synchronize()
+                outs.append(y)
+            assert all(torch.equal(outs[0], y) for y in outs[1:])
+            for v in range(nv):
+                assert np.abs(outs[0][v].cpu().numpy() - refs[v]).max() <= TOL64 * np.abs(refs[v]).max()
