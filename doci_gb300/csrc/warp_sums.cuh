@@ -49,7 +49,8 @@ __device__ __forceinline__ void warp_sums(double *v, double *out) {
 // addition's rounding error (Knuth's two-sum, exact) goes to e, whose own
 // rounding is 2^-24 of terms already 2^-24 small.  Eight FP32 instructions take
 // the place of a conversion and an FP64 add that holds its quarter of the SM
-// for 64 clocks.
+// for 64 clocks.  Values whose sums could leave FP32's range, or infinities
+// (two-sum makes them NaN), are summed in FP64.
 __device__ __forceinline__ void pair_add(float &s, float &e, float t) {
   const float r = __fadd_rn(s, t), z = __fadd_rn(r, -s);
   e = __fadd_rn(e, __fadd_rn(__fadd_rn(s, -__fadd_rn(r, -z)), __fadd_rn(t, -z)));
@@ -59,6 +60,15 @@ __device__ __forceinline__ void pair_add(float &s, float &e, float t) {
 template <int K>
 __device__ __forceinline__ double warp_sum_pow2(float *v) {
   const int lane = threadIdx.x & 31;
+  float big = 0.f;
+#pragma unroll
+  for (int i = 0; i < K; ++i) big = fmaxf(big, fabsf(v[i]));
+  if (__any_sync(0xffffffffu, big > 0x1p120f)) {
+    double d[K];
+#pragma unroll
+    for (int i = 0; i < K; ++i) d[i] = static_cast<double>(v[i]);
+    return warp_sum_pow2<K>(d);
+  }
   float e[K];
 #pragma unroll
   for (int i = 0; i < K; ++i) e[i] = 0.f;

@@ -187,3 +187,26 @@ def test_integrals_not_finite(nroots, bad, synth, dg):
     with dg.Hamiltonian.from_fcidump(p) as h:
         r = dg.solve_roots(h, nroots=2, tol=1e-7, mode="fp64")
     assert r["converged"] == 1 and np.allclose(r["energies"][:2], dense_eigs(p, 2), atol=1e-9)
+
+
+@pytest.mark.parametrize("power", [0, 60, 63])
+def test_mixed_solve_scales(power, dg):
+    """A Hamiltonian and tolerances times a power of two give the same solve times
+    that power, as long as the values' squares are in FP32's range (up to 2^126
+    here): a thread's FP32 sums then are, and a block's, formed in FP64, are in any case."""
+    L, N, s = 10, 5, 2.0 ** power
+    rng = np.random.default_rng(170)
+    K = rng.uniform(0.9, 0.99, (L, L))
+    K = np.triu(K, 1) + np.triu(K, 1).T
+    eri = np.zeros((L, L, L, L))
+    i, j = np.nonzero(~np.eye(L, dtype=bool))
+    eri[i, j, i, j] = eri[i, j, j, i] = K[i, j]
+    h1 = np.diag(np.linspace(-4, 4, L))
+    out = []
+    for f in (1.0, s):
+        with dg.Hamiltonian.from_integrals(L, N, 0.0, h1 * f, eri * f) as h:
+            out.append(dg.solve_roots(h, nroots=2, tol=1e-7 * f, mixed_tol=1e-4 * f, mode="mixed", max_vec=16))
+    a, b = out
+    assert a["converged"] == b["converged"] == 1
+    assert a["iterations_fp32"] == b["iterations_fp32"] > 3 and a["iterations"] == b["iterations"]
+    assert np.allclose(np.array(b["energies"][:2]) / s, a["energies"][:2], rtol=1e-12, atol=0)
