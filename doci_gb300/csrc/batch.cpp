@@ -164,8 +164,12 @@ struct doci_server {
       in.one = std::move(r.one);
       in.two = std::move(r.two);
     }
-    const int64_t fp = roots_footprint(L, N, opts);
+    int64_t fp = roots_footprint(L, N, opts);
     if (fp < 0) return DOCI_ERR_INVALID;
+    // a budget that has no room for the neighbour table beside the solve: the
+    // request runs without one
+    const bool table = fp <= budget;
+    if (!table) fp -= static_cast<int64_t>(nbr_table_bytes(L, N, binom64(L, N)));
     if (fp > budget) return DOCI_ERR_ADMISSION;
     {
       std::unique_lock<std::mutex> lk(mu);
@@ -179,6 +183,7 @@ struct doci_server {
     bool own = false;
     if (!h) {
       h = new doci_ham();
+      h->want_nbr = table;
       s = ham_build(h, in);
       own = true;
     }
@@ -369,7 +374,8 @@ int doci_batch_solve(int n, doci_ham *const *hams, const doci_batch_opts *opts, 
     int64_t used = 0;
     int j = i;
     while (j < n) {
-      const int64_t f = engine_footprint(hams[j]->L, hams[j]->N, o) - static_cast<int64_t>(hams[j]->D) * 12;
+      const int64_t f = engine_footprint(hams[j]->L, hams[j]->N, o) - static_cast<int64_t>(hams[j]->D) * 12 -
+                        static_cast<int64_t>(nbr_table_bytes(hams[j]->L, hams[j]->N, hams[j]->D));
       if (j > i && used + f > budget) break;
       used += f;
       ++j;

@@ -102,6 +102,7 @@ struct doci_ham {
   // small spaces: every neighbour's rank and hop weight (sigma.cu,
   // nbr_table_kernel); null where the table would be too large
   uint32_t *d_nbr = nullptr;
+  bool want_nbr = true;  // (false: not built, a server's budget has no room for it)
   // pair form (sigma_pair.cu): one block per (N-1)-pair set's row part R',
   // {own row start or ~0, mask | k' << 24}, largest first; the K matrix split
   // into TF32 high and low parts (2 x 32 x 32 floats, mirrored orbitals; also

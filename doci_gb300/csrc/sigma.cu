@@ -1241,7 +1241,7 @@ size_t nbr_table_bytes(int L, int N, uint64_t D) {
 
 int ham_build_nbr(doci_ham *h) {
   const size_t bytes = nbr_table_bytes(h->L, h->N, h->D);
-  if (bytes == 0) return DOCI_OK;
+  if (bytes == 0 || !h->want_nbr) return DOCI_OK;
   if (cudaMallocAsync(&h->d_nbr, bytes, h->stream) != cudaSuccess) {  // no memory: the kernels without a table
     cudaGetLastError();
     h->d_nbr = nullptr;

@@ -210,3 +210,40 @@ def test_mixed_solve_scales(power, dg):
     assert a["converged"] == b["converged"] == 1
     assert a["iterations_fp32"] == b["iterations_fp32"] > 3 and a["iterations"] == b["iterations"]
     assert np.allclose(np.array(b["energies"][:2]) / s, a["energies"][:2], rtol=1e-12, atol=0)
+
+
+def nbr_table_bytes(L, N):
+    import math
+    n = math.comb(L, N) * N * (L - N)
+    return 4 * n if n <= 1 << 23 else 0
+
+
+@pytest.mark.parametrize("nroots", [1, 2])
+@pytest.mark.parametrize("L,N", [(14, 7), (18, 8)])
+def test_admission_leaves_room_for_the_solve_alone(L, N, nroots, dg):
+    """A budget that holds the solve but not the neighbour table beside it admits
+    the request (which runs without the table), and a batch of handles that
+    exist already, tables and all, needs room for its solves alone."""
+    import ctypes as C
+    from doci_gb300.fcidump import raw_integrals
+    one, two = raw_integrals(L, 180)
+    opts = dict(nroots=nroots, tol=1e-6, mode="mixed", max_vec=16)
+    fp = dg.lib().doci_roots_footprint(L, N, C.byref(dg.batch_opts(**opts)))
+    table = nbr_table_bytes(L, N)
+    assert 0 < table < fp
+    got = {}
+    for budget in (fp, fp - table, fp - table - 1):
+        with dg.Server(workers=1, hbm_budget=budget, **opts) as srv:
+            got[budget] = srv.wait(srv.submit(L, N, one, two))
+    assert got[fp - table - 1]["status"] == 9  # DOCI_ERR_ADMISSION
+    for b in (fp, fp - table):
+        assert got[b]["status"] == 0 and got[b]["converged"] == 1
+        assert np.allclose(got[b]["energies"][:nroots], got[fp]["energies"][:nroots], rtol=0, atol=1e-9)
+    if nroots > 1:  # (the footprint of one root is that of the single-root solver)
+        with dg.Hamiltonian.from_integrals(L, N, 0.0, one, two) as h:
+            solve = fp - 12 * h.D - table
+            for budget, want in ((solve, 0), (solve - 1, 9)):
+                st, res = dg.batch_solve([h], hbm_budget=budget, **opts)
+                assert st == res[0]["status"] == want
+            assert np.allclose(dg.batch_solve([h], hbm_budget=solve, **opts)[1][0]["energies"][:nroots],
+                               got[fp]["energies"][:nroots], rtol=0, atol=1e-9)
