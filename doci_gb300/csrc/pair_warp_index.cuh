@@ -102,5 +102,24 @@ inline Groups groups(int P, int na, int N, const uint32_t *B, int stride) {
   return g;
 }
 
+// Column orbitals of an (L, N) space for `slots` tile rows in flight, and the unit
+// list (0: fewer than 10 orbitals).  The more the fewer units: 12 as long as that
+// leaves four units per tile row, else 10 as long as each has one, else 8; but no
+// more than 20 row orbitals, whose row starts take 4 MiB.  (That bounds only
+// spaces of few pairs or holes, up to 35,960 determinants, which run from their
+// neighbour table unless asked: L=32, N=2 would have 2^24 row starts for its 496
+// determinants.)
+constexpr int kMaxRowOrbitals = 20;
+inline int column_orbitals(int L, int N, uint32_t slots, const uint32_t *B, int stride, Groups *g) {
+  int P = 0;
+  for (int p : {12, 10, 8}) {
+    if (L - p < 2 || L - p > kMaxRowOrbitals) continue;
+    P = p;
+    *g = groups(P, L - P, N, B, stride);
+    if (g->first[g->n] / 4 >= (p == 12 ? 4 : 1) * slots) break;
+  }
+  return P;
+}
+
 }  // namespace pw
 }  // namespace doci

@@ -22,8 +22,7 @@
 // cycles for 32 and for 64 columns on GB300 (24.6 ns in a run of 96; 72 cycles
 // at 128 columns).  The two halves are added when they are read back.
 //
-// Column orbitals: 12 as long as that leaves four units per tile row in
-// flight, else 10 as long as each has one, else 8.  Larger rows mean fewer
+// Column orbitals: 12, 10 or 8 (pw::column_orbitals).  Larger rows mean fewer
 // set-ups and fewer row-part orbitals to look at, smaller ones more units to
 // spread.  Measured with one warp doing both jobs (us, 12 / 10 / 8): L=32 N=16
 // 19,120 / 22,940 / 38,470; L=26 N=13 347 / 362 / 562; L=24 N=12
@@ -391,15 +390,8 @@ int ham_build_pair_warp(doci_ham *h) {
   if (major != 10 || minor != 3) return DOCI_OK;
   std::vector<uint32_t> B(kBinomRows * kBinomCols);
   fill_binom_table(B.data());
-  int P = 0;
   pw::Groups g;
-  for (int p : {12, 10, 8}) {
-    if (L - p < 2 || L - p > 24) continue;
-    P = p;
-    g = pw::groups(P, L - P, N, B.data(), kBinomCols);
-    const uint32_t slots = static_cast<uint32_t>(kSlots * device_sm_count());
-    if (g.first[g.n] / 4 >= (p == 12 ? 4 : 1) * slots) break;
-  }
+  const int P = pw::column_orbitals(L, N, static_cast<uint32_t>(kSlots * device_sm_count()), B.data(), kBinomCols, &g);
   const int na = L - P;
   const uint32_t total = g.first[g.n];
   DOCI_CUDA(cudaMallocAsync(&h->d_wstart, sizeof(uint32_t) << na, h->stream));

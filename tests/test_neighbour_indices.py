@@ -173,3 +173,15 @@ def test_warp_pair_form_ranks(warp_exe, L, N, P, us, ss):
     r = subprocess.run([warp_exe, str(L), str(N), str(P), str(us), str(ss)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
     assert "bad=0" in r.stdout
+
+
+def test_warp_pair_form_column_orbitals(tmp_path):
+    """The tiling that every (L, N) gets: row starts of at most 4 MiB."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not available")
+    exe = str(tmp_path / "choice")
+    subprocess.run([nvcc, "-O2", "-std=c++17", "-diag-suppress=20011",
+                    os.path.join(HERE, "host_checks", "pair_warp_choice_check.cu"), "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0 and "shapes=483 bad=0" in r.stdout, r.stdout + r.stderr
