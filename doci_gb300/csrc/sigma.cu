@@ -1073,8 +1073,18 @@ int multi_method_auto(const doci_ham *h, int precision) {
 // FP64 L=24 2,915 / 3,113 -> 725 / 1,444.  (Spaces with a neighbour table take
 // the gather kernel.)
 constexpr size_t kDetMaxBytes = size_t(5) << 30;
-bool det_fits(const doci_ham *h, size_t elem) {
-  return h->sigma_kernel == 0 && !h->d_nbr && (elem == 8 ? pair_warp64_fits(h) : pair_warp_fits(h)) &&
+// Not while `st` is captured: an allocation in it would make a graph that can be
+// instantiated once at a time and not be part of another.
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return s != cudaStreamCaptureStatusNone;
+}
+bool det_fits(const doci_ham *h, size_t elem, cudaStream_t st) {
+  return h->sigma_kernel == 0 && !capturing(st) && !h->d_nbr && (elem == 8 ? pair_warp64_fits(h) : pair_warp_fits(h)) &&
          static_cast<size_t>(pair_warp_slabs(h)) * h->D * elem <= kDetMaxBytes;
 }
 // *done = false: there is no memory for the scratch
@@ -1125,7 +1135,7 @@ int run_multi(const doci_ham *h, int method, const void *x, size_t ldx, void *y,
   if (method == kMultiGather)
     return precision == DOCI_FP64 ? launch_gather_multi_typed<double>(h, x, ldx, y, ldy, nv, st)
                                   : launch_gather_multi_typed<float>(h, x, ldx, y, ldy, nv, st);
-  if (det_fits(h, elem)) {
+  if (det_fits(h, elem, st)) {
     bool done;
     const int r = run_det(h, xc, ldx, yc, ldy, nv, precision, st, &done);
     if (done || r != DOCI_OK) return r;
@@ -1147,7 +1157,7 @@ int launch_sigma_multi(const doci_ham *h, const void *x, size_t ldx, void *y, si
   // (a tuned nv = 1 is a choice among the single-vector kernels, made without the
   // reproducible pair form)
   int method = h->sigma_kernel == 0 && nv > 1 ? tuned_choice(h, precision, nv, false) : 0;
-  if (method == 0 && det_fits(h, precision == DOCI_FP64 ? 8 : 4)) {
+  if (method == 0 && det_fits(h, precision == DOCI_FP64 ? 8 : 4, st)) {
     bool done;
     const int r = run_det(h, static_cast<const char *>(x), ldx, static_cast<char *>(y), ldy, nv, precision, st, &done);
     if (done || r != DOCI_OK) return r;

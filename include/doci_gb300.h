@@ -163,8 +163,9 @@ int doci_sigma(doci_ham *ham, const void *d_x, void *d_y, int precision, void *s
  * doci_ham_set_sigma_kernel set kind 9): results repeat bit for bit.  On large
  * spaces one vector after the other in
  * the pair form with every contribution in a place of its own (stream-ordered
- * scratch of at most min(N, L - 8) x D elements, up to 5 GiB); else, and when
- * there is no memory for that, the neighbour ranks and hop weights of each
+ * scratch of at most min(N, L - 8) x D elements, up to 5 GiB); else, when there is
+ * no memory for that, and while the stream is captured (so that the graph holds no
+ * allocation), the neighbour ranks and hop weights of each
  * determinant are computed once per launch for up to four vectors (larger nv
  * runs in groups of four).  Results agree with doci_sigma to
  * rounding (identical when both use the same kernel).  No counterpart in the

@@ -657,3 +657,50 @@ def test_sigma_block_reproducible_after_tuning(L, N, seed, synth, dg):
             assert all(torch.equal(outs[0], y) for y in outs[1:])
             for v in range(nv):
                 assert np.abs(outs[0][v].cpu().numpy() - refs[v]).max() <= TOL64 * np.abs(refs[v]).max()
+
+
+@pytest.mark.parametrize("prec_name,nv", [("FP32", 1), ("FP32", 4), ("FP32", 6)])
+def test_sigma_block_captured_without_allocations(prec_name, nv, synth, dg):
+    """A captured FP32 block sigma on a space whose automatic form takes scratch
+    holds no allocation, so its graph can be instantiated more than once; the
+    graph gives the oracle's matvec."""
+    import ctypes as C
+    torch = torch_cuda()
+    rt = C.CDLL("libcudart.so.13")
+    prec = getattr(dg, prec_name)
+    p = synth(20, 10, 151)
+    o = oracle.Ham(p)
+
+    def ok(st):
+        assert st == 0, st
+
+    with dg.Hamiltonian.from_fcidump(p) as h:
+        D = h.D
+        X = np.random.default_rng(9).standard_normal((nv, D)).astype(np.float32)
+        x = torch.from_numpy(X).cuda()
+        y = torch.zeros_like(x)
+        torch.cuda.synchronize()
+        st = C.c_void_p(torch.cuda.Stream().cuda_stream)
+        graph, execs, n = C.c_void_p(), [C.c_void_p(), C.c_void_p()], C.c_size_t()
+        ok(rt.cudaStreamBeginCapture(st, 2))  # relaxed
+        h.sigma_block_device(x.data_ptr(), D, y.data_ptr(), D, nv, prec, stream=st.value)
+        ok(rt.cudaStreamEndCapture(st, C.byref(graph)))
+        ok(rt.cudaGraphGetNodes(graph, None, C.byref(n)))
+        nodes, kind = (C.c_void_p * n.value)(), C.c_int()
+        ok(rt.cudaGraphGetNodes(graph, nodes, C.byref(n)))
+        for node in nodes:
+            ok(rt.cudaGraphNodeGetType(C.c_void_p(node), C.byref(kind)))
+            assert kind.value not in (10, 11)  # cudaGraphNodeTypeMemAlloc, cudaGraphNodeTypeMemFree
+        for e in execs:
+            ok(rt.cudaGraphInstantiate(C.byref(e), graph, C.c_ulonglong(0)))
+        for e in execs:
+            y.zero_()
+            torch.cuda.synchronize()
+            ok(rt.cudaGraphLaunch(e, st))
+            torch.cuda.synchronize()
+            for v in range(nv):
+                ref = o.matvec(X[v].astype(np.float64))
+                assert np.abs(y[v].cpu().numpy() - ref).max() <= TOL32 * np.abs(ref).max()
+        for e in execs:
+            ok(rt.cudaGraphExecDestroy(e))
+        ok(rt.cudaGraphDestroy(graph))
