@@ -1017,12 +1017,12 @@ int launch_sigma(const doci_ham *h, const void *x, void *y, int precision, cudaS
     case 8:
       if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0)
         return launch_tc(h, static_cast<const float *>(x), static_cast<float *>(y), st, h->d_tc_err, tc_spin_limit());
-      // bulk copies need a 16-byte aligned x: the mma.sync pair form instead
-      return pair_fits(h) ? launch_pair(h, static_cast<const float *>(x), static_cast<float *>(y), st)
-                          : launch_row<float>(h, x, y, st, 1);
+      // bulk copies need a 16-byte aligned x: kind 6 instead
+      if (!pair_fits(h)) return launch_row<float>(h, x, y, st, 1);
+      [[fallthrough]];
     case 6:
       // from 10 orbitals on the warp-per-unit form (faster at every size measured
-      // from L=18 on: 18.8 -> 16.7 us there, 33.9 -> 19.1 ms at L=32)
+      // from L=18 on: 18.8 -> 16.7 us there, 33.9 -> 16.9 ms at L=32)
       if (pair_warp_fits(h))
         return launch_pair_warp(h, static_cast<const float *>(x), static_cast<float *>(y), st);
       return launch_pair(h, static_cast<const float *>(x), static_cast<float *>(y), st);

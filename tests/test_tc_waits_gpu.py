@@ -157,3 +157,43 @@ def test_wait_limit_reaches_the_solvers(solver, synth):
     else:
         assert r.returncode != 0 and "returned" not in out
         assert "device wait timed out" in r.stderr + r.stdout
+
+
+UNALIGNED_CHILD = r"""
+import ctypes as C, sys
+import numpy as np, torch
+sys.path.insert(0, {root!r})
+import doci_gb300 as dg, oracle
+p = {path!r}
+o = oracle.Ham(p)
+with dg.Hamiltonian.from_fcidump(p) as h:
+    h.set_sigma_kernel("tc")
+    x = np.random.default_rng(1).standard_normal(h.D).astype(np.float32)
+    xs = torch.zeros(h.D + 1, dtype=torch.float32, device="cuda")
+    xs[1:] = torch.from_numpy(x)
+    y = torch.empty(h.D, dtype=torch.float32, device="cuda")
+    h.sigma_device(xs[1:].data_ptr(), y.data_ptr(), dg.FP32)
+    torch.cuda.synchronize()
+    ref = o.matvec(x.astype(np.float64))
+    print("err", float(np.abs(y.cpu().numpy() - ref).max() / np.abs(ref).max()))
+    h.set_sigma_kernel("gather")
+    print("status", dg.lib().doci_sigma_host(h.handle, x.ctypes.data_as(C.c_void_p),
+                                             np.empty_like(x).ctypes.data_as(C.c_void_p), dg.FP32))
+"""
+
+
+def test_unaligned_tc_runs_kind_6(synth):
+    """Kind 8 on an x that is not 16-byte aligned runs what kind 6 runs: right with
+    the ordinary wait limit, and a timeout with none (the kernel of kind 6 has
+    device waits; the one it took the place of has not)."""
+    p = synth(20, 10, 75)
+    for limit in (None, "0"):
+        env = dict(os.environ, **({"DOCI_TC_SPIN_LIMIT": limit} if limit else {}))
+        r = subprocess.run([sys.executable, "-c", UNALIGNED_CHILD.format(root=ROOT, path=p)], capture_output=True,
+                           text=True, env=env, timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+        got = dict(ln.split() for ln in r.stdout.splitlines() if ln.startswith(("err", "status")))
+        if limit:
+            assert int(got["status"]) == 12
+        else:
+            assert int(got["status"]) == 0 and float(got["err"]) <= 2e-6
