@@ -306,7 +306,7 @@ int doci_sigma_host(doci_ham *h, const void *x, void *y, int precision) {
   // (601M: 134 against 103 ms; 10M: 4.0 against 1.8) and into pageable y (601M
   // FP32: 56 against 44 ms).
   const bool y_pinned = mapped_host(y) != nullptr;
-  if (sched && precision == DOCI_FP32 && kind == 6 && pair_fits(h) && h->D >= kHostOverlapMinD && y_pinned) {
+  if (sched && precision == DOCI_FP32 && kind == 6 && pair_fits(h) && y_pinned) {
     st = launch_pair_host(h, static_cast<const float *>(x), static_cast<float *>(h->d_stage_x),
                           static_cast<float *>(h->d_stage_y), static_cast<float *>(y), h->stream);
     if (st) return st;

@@ -16,8 +16,10 @@ namespace doci {
 constexpr int kMaxOrbitals = 32;
 // doci_sigma_host overlaps its copies with the sigma from here on (in FP32,
 // between pinned buffers: 155M determinants 9.4 ms against 11.0, 40M 4.4 ms
-// against 2.9)
+// against 2.9); the environment variable DOCI_HOST_OVERLAP_MIN_D (read once)
+// lowers it, so that a test can run that path on a small space
 constexpr uint32_t kHostOverlapMinD = 1u << 27;
+uint32_t host_overlap_min_d();
 // binomial table C(n, k) for n = 0..32 and k = 0..34 (k up to N + 2 is read
 // by the neighbour-rank prefix sums)
 constexpr int kBinomRows = 33;
@@ -123,7 +125,7 @@ struct doci_ham {
   // alternately on the handle's stream and side_stream (host_plan.h):
   // d_pblocks_host holds the units in group order, host_steps what each
   // group's launch waits for and which pieces go down after it.  Built for the
-  // spaces that take that path, D >= kHostOverlapMinD.
+  // spaces that take that path, D >= host_overlap_min_d().
   static constexpr int kHostChunks = doci::hostplan::kPieces;
   uint32_t *d_pblocks_host = nullptr;
   std::vector<doci::hostplan::Group> host_groups;

@@ -352,6 +352,14 @@ bool pair_fits(const doci_ham *h) {
   return static_cast<size_t>(h->max_row) * sizeof(float) <= 100 * 1024;
 }
 
+uint32_t host_overlap_min_d() {
+  static const uint32_t v = [] {
+    const char *e = std::getenv("DOCI_HOST_OVERLAP_MIN_D");
+    return e ? static_cast<uint32_t>(std::strtoul(e, nullptr, 10)) : kHostOverlapMinD;
+  }();
+  return v;
+}
+
 int ham_build_pairs(doci_ham *h, const std::vector<uint32_t> &start) {
   const int L = h->L, N = h->N, sp = h->split, na = L - sp;
   // K (mirrored orbitals, zero outside 0..L-1) split into TF32 high and low
@@ -385,7 +393,7 @@ int ham_build_pairs(doci_ham *h, const std::vector<uint32_t> &start) {
   // steps (host_plan.h).  The search for the schedule is serial host work, 6.3
   // of a Hamiltonian's 8.7 ms at 2.7M determinants, so nobody else pays for it.
   std::vector<uint32_t> flat_host;
-  if (h->D >= kHostOverlapMinD) {
+  if (h->D >= host_overlap_min_d()) {
     hostplan::pieces(h->D, h->chunk_off);
     std::vector<hostplan::Unit> hu;
     hu.reserve(bl.size());
