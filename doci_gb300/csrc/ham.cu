@@ -96,6 +96,7 @@ void ham_release(doci_ham *h) {
     if (e) cudaEventDestroy(e);
     e = nullptr;
   }
+  if (st) slab_pool_trim(h->device);
   for (auto &e : h->group_ev)
     if (e) cudaEventDestroy(e);
   h->group_ev.clear();

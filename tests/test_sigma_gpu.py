@@ -704,3 +704,19 @@ def test_sigma_block_captured_without_allocations(prec_name, nv, synth, dg):
         for e in execs:
             ok(rt.cudaGraphExecDestroy(e))
         ok(rt.cudaGraphDestroy(graph))
+
+
+def test_sigma_block_scratch_is_given_back(synth, dg):
+    """The block sigma's scratch (13 vectors of 10.4M elements here) is the
+    device's again when the handle is destroyed."""
+    torch = torch_cuda()
+    L, N, nv = 26, 13, 2
+    h = dg.Hamiltonian.from_fcidump(synth(L, N, 152))
+    x = torch.randn((nv, h.D), dtype=torch.float32, device="cuda")
+    y = torch.empty_like(x)
+    h.sigma_block_device(x.data_ptr(), h.D, y.data_ptr(), h.D, nv, dg.FP32)
+    torch.cuda.synchronize()
+    held = torch.cuda.mem_get_info()[0]
+    h.close()
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] - held >= 0.9 * 13 * x.shape[1] * 4
