@@ -126,66 +126,118 @@ multidot_kernel(const double *__restrict__ V, size_t ld, int m, const double *__
 // The same for FP32 vectors with exact products (doci_multidot), without the
 // FP64 units, whose rate (1/64 of FP32) and widening conversions held the
 // pass at 2.44 ms for 16 columns of 40.1M (1.1 TB/s).  A thread sums runs of
-// kRun products as pairs of floats: p = v w and its rounding error from an
-// FMA (v w = p + e exactly), s + p by Knuth's two-sum (exact), the errors in
-// c; then s and c go to an FP64 sum.  c's own rounding is 2^-24 of terms
-// already 2^-24 small.  That holds while the run's largest product is well
+// kRun products as triples of floats: p = v w and its rounding error from an
+// FMA (v w = p + e exactly), s + p by Knuth's two-sum (exact), the two errors
+// into c by two-sums likewise, and their errors in r; then s + c + r goes to an FP64
+// sum.  r's own rounding is 2^-24 of terms already 2^-48 small, so a run is
+// more exact than FP64 additions would be (with the errors only added up in c, at
+// 2^-48, sums that cancel were off by 2e-17 of their terms' magnitudes, where FP64
+// sums are by 2e-19).  That holds while the run's largest product is well
 // inside FP32's range; a run where it is not (all products tiny, an overflow,
 // an infinity, or all zero) is done again in FP64, skipping finite products
 // with a zero factor.
-// Columns go in groups of four, one per block (blockIdx.x, so that the groups
-// of a stretch run together and w comes from L2 after the first): 64 registers,
-// four blocks per SM, sixteen loads of V in flight per thread.  538 us there
-// (5.1 TB/s); groups of eight 568 us with two blocks per SM and 981 us with
-// three (spills), all sixteen columns in one block 770-850 us.
-constexpr int kRun = 64;
+// Columns go in groups of two, one per block (blockIdx.x, so that the groups of
+// a stretch run together and w comes from L2 after the first), whose values share
+// register pairs (packed FP32 instructions): 64 registers, four blocks per SM, eight
+// loads of V in flight per thread.  658 us there (4.1 TB/s), bound by the 22 packed
+// instructions per element and two columns; groups of four with packed instructions
+// 665 us with two blocks per SM, 716 with four (spills), one column at a time 720
+// to 800.  (491 us in pairs of floats, eleven instructions.)
+constexpr int kRun = 64, KF = 2;  // (columns per block)
+typedef unsigned long long f2;  // two floats
+__device__ __forceinline__ f2 pk(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void up(f2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 addp(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 mulp(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 __global__ void __launch_bounds__(kT, 4)
 multidot_exact_f32_kernel(const float *__restrict__ V, size_t ld, int m, const float *__restrict__ w, size_t n,
                           double *__restrict__ partials) {
-  const int k0 = blockIdx.x * KG, mk = min(KG, m - k0);
+  const int k0 = blockIdx.x * KF, mk = min(KF, m - k0);
   V += k0 * ld;
-  double acc[KG];
+  double acc[KF];
 #pragma unroll
-  for (int k = 0; k < KG; ++k) acc[k] = 0;
+  for (int k = 0; k < KF; ++k) acc[k] = 0;
   const size_t stride = (size_t)gridDim.y * blockDim.x;
   for (size_t j0 = blockIdx.y * (size_t)blockDim.x + threadIdx.x; j0 < n; j0 += stride * kRun) {
-    float s[KG], c[KG], big[KG];
+    // two columns to a register pair
+    f2 s[KF / 2], c[KF / 2], r[KF / 2];
+    float big[KF];
 #pragma unroll
-    for (int k = 0; k < KG; ++k) s[k] = c[k] = big[k] = 0.f;
-    auto add = [&](int k, float v, float wj) {
-      const float p = __fmul_rn(v, wj), e = fmaf(v, wj, -p);
-      const float t = __fadd_rn(s[k], p), z = __fadd_rn(t, -s[k]);
-      const float d = __fadd_rn(__fadd_rn(s[k], -__fadd_rn(t, -z)), __fadd_rn(p, -z));
+    for (int k = 0; k < KF; ++k) {
+      s[k / 2] = c[k / 2] = r[k / 2] = pk(0.f, 0.f);
+      big[k] = 0.f;
+    }
+    const f2 minus = pk(-1.f, -1.f);
+    auto two_sum = [&](f2 &a, f2 b) {  // a + b rounded in a; its error is returned
+      const f2 t = addp(a, b), z = fma2(a, minus, t);
+      const f2 d = addp(fma2(fma2(z, minus, t), minus, a), fma2(z, minus, b));
+      a = t;
+      return d;
+    };
+    auto add = [&](int k, f2 v, f2 w2, f2 nw) {  // columns 2 k and 2 k + 1
+      const f2 np = mulp(v, nw), e = fma2(v, w2, np);  // -p (as exact) and p's rounding error
+      const f2 t = fma2(np, minus, s[k]), z = fma2(s[k], minus, t);
+      const f2 d = fma2(addp(np, z), minus, fma2(fma2(z, minus, t), minus, s[k]));  // the two-sum with -np
       s[k] = t;
-      c[k] = __fadd_rn(c[k], __fadd_rn(e, d));
-      big[k] = fmaxf(big[k], fabsf(p));
+      const f2 f = two_sum(c[k], e), g = two_sum(c[k], d);
+      r[k] = addp(r[k], addp(f, g));
+      float p0, p1;
+      up(np, p0, p1);
+      big[2 * k] = fmaxf(big[2 * k], fabsf(p0));
+      big[2 * k + 1] = fmaxf(big[2 * k + 1], fabsf(p1));
     };
     const size_t left = (n - j0 + stride - 1) / stride;  // this thread's elements from j0 on
     const int run = left < kRun ? static_cast<int>(left) : kRun;
     const float *vp = V + j0, *wp = w + j0;
     int u = 0;
     for (; u + kAhead <= run; u += kAhead, vp += kAhead * stride, wp += kAhead * stride) {
-      float wj[kAhead], v[kAhead][KG];
+      float wj[kAhead], v[kAhead][KF];
 #pragma unroll
       for (int a = 0; a < kAhead; ++a) {
         wj[a] = wp[a * stride];
 #pragma unroll
-        for (int k = 0; k < KG; ++k) v[a][k] = k < mk ? vp[k * ld + a * stride] : 0.f;
+        for (int k = 0; k < KF; ++k) v[a][k] = k < mk ? vp[k * ld + a * stride] : 0.f;
       }
 #pragma unroll
       for (int a = 0; a < kAhead; ++a)
 #pragma unroll
-        for (int k = 0; k < KG; ++k) add(k, v[a][k], wj[a]);
+        for (int k = 0; k < KF / 2; ++k)
+          add(k, pk(v[a][2 * k], v[a][2 * k + 1]), pk(wj[a], wj[a]), pk(-wj[a], -wj[a]));
     }
     for (; u < run; ++u, vp += stride, wp += stride)
 #pragma unroll
-      for (int k = 0; k < KG; ++k)
-        if (k < mk) add(k, vp[k * ld], wp[0]);
+      for (int k = 0; k < KF / 2; ++k)
+        add(k, pk(2 * k < mk ? vp[2 * k * ld] : 0.f, 2 * k + 1 < mk ? vp[(2 * k + 1) * ld] : 0.f), pk(wp[0], wp[0]),
+            pk(-wp[0], -wp[0]));
+    float sk[KF], ck[KF], rk[KF];
 #pragma unroll
-    for (int k = 0; k < KG; ++k)
+    for (int k = 0; k < KF / 2; ++k) {
+      up(s[k], sk[2 * k], sk[2 * k + 1]);
+      up(c[k], ck[2 * k], ck[2 * k + 1]);
+      up(r[k], rk[2 * k], rk[2 * k + 1]);
+    }
+#pragma unroll
+    for (int k = 0; k < KF; ++k)
       if (k < mk) {
         if (big[k] >= 0x1p-80f && big[k] <= 0x1p120f) {
-          acc[k] += static_cast<double>(s[k]) + static_cast<double>(c[k]);
+          acc[k] += static_cast<double>(sk[k]) + (static_cast<double>(ck[k]) + static_cast<double>(rk[k]));
         } else {
           for (int i = 0; i < run; ++i) {
             const size_t j = j0 + i * stride;
@@ -196,7 +248,7 @@ multidot_exact_f32_kernel(const float *__restrict__ V, size_t ld, int m, const f
         }
       }
   }
-  block_reduce_store<KG>(acc, mk, partials, m, k0);
+  block_reduce_store<KF>(acc, mk, partials, m, k0);
 }
 
 // FP64 Davidson passes.  The FP64 units bound them (two lanes per clock and SM:
@@ -1102,7 +1154,7 @@ int vec_multidot(const S *V, size_t ld, int m, const S *w, size_t n, double *par
     multidot_kernel<<<dim3(groups, static_cast<unsigned>(rows)), kT, 0, st>>>(V, ld, m, w, n, partials);
   } else if (fp64_products) {
     // two rows of blocks per SM (at most grid_blocks(): the partial-sum buffers' sizes hold)
-    multidot_exact_f32_kernel<<<dim3(groups, 2 * device_sm_count()), kT, 0, st>>>(V, ld, m, w, n, partials);
+    multidot_exact_f32_kernel<<<dim3((m + KF - 1) / KF, 2 * device_sm_count()), kT, 0, st>>>(V, ld, m, w, n, partials);
   } else {
     return dispatch_k<S, MultidotL>(m, st, V, ld, m, w, n, partials);
   }

@@ -111,3 +111,26 @@ def test_fp64_davidson_basis_sizes(L, N, max_vec, synth):
     assert res["converged"] and abs(np.linalg.norm(v) - 1) < 1e-12
     assert np.linalg.norm(H @ v - (v @ H @ v) * v) < 1e-9
     assert np.abs(np.linalg.eigvalsh(H) - e).min() < 1e-9
+
+
+@pytest.mark.parametrize("n,m", [(1001, 3), (300_001, 4), (3_000_001, 5), (5_000_003, 9)])
+def test_multidot_f32_cancelling_sums(n, m):
+    """FP32 vectors whose products nearly cancel: the error of the sums is no more
+    than that of FP64 additions of the exact products in the kernel's order (runs
+    of 64 or less per thread, then the threads', warps' and blocks' sums: at most 2 sqrt(64)
+    roundings at 2^-53 of a thread's sum, and the result's own), where pairs of
+    floats in a run would leave 2^-48 of each term."""
+    import math
+    import torch
+    import doci_gb300
+    g = torch.Generator(device="cuda").manual_seed(n + m)
+    V = torch.randn(m, n, device="cuda", generator=g)
+    w = torch.randn(n, device="cuda", generator=g)
+    out = torch.empty(m, dtype=torch.float64, device="cuda")
+    assert doci_gb300.lib().doci_multidot(V.data_ptr(), n, m, w.data_ptr(), n, 1, out.data_ptr(), None) == 0
+    p = (V.double() * w.double()).cpu().numpy()
+    for k in range(m):
+        exact, size = math.fsum(p[k]), np.abs(p[k]).sum()
+        # independent roundings: those of the terms' sums add up as sqrt(n) of sqrt(run) 2^-53 |p|
+        bound = 16 * 2.0 ** -53 * np.sqrt(n) * (size / n) + 4 * 2.0 ** -53 * abs(exact)
+        assert abs(out[k].item() - exact) <= bound, (k, abs(out[k].item() - exact) / size)
