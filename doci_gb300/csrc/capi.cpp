@@ -312,8 +312,8 @@ int doci_sigma_host(doci_ham *h, const void *x, void *y, int precision) {
     if (st) return st;
     DOCI_CUDA(cudaStreamSynchronize(h->stream));
     return ham_device_error(h, h->stream);
-  } else if (sched && precision == DOCI_FP64 && kind == 9 && !pair_warp64_fits(h) && pair_ff_fits(h)) {
-    // a K that the digits cannot hold: the float-pair form, overlapped (601M
+  } else if (sched && precision == DOCI_FP64 && kind == 9 && !pair_warp64_wanted(h) && pair_ff_fits(h)) {
+    // a K that the digits cannot hold (or few open slots): the float-pair form, overlapped (601M
     // determinants 134 ms; in turn 184).  A pageable y is copied after it.
     st = launch_pair_ff_host(h, static_cast<const double *>(x), static_cast<double *>(h->d_stage_x),
                              static_cast<double *>(h->d_stage_y), y_pinned ? static_cast<double *>(y) : nullptr,

@@ -189,6 +189,7 @@ bool pair_warp_fits(const doci_ham *h);
 int launch_pair_warp(const doci_ham *h, const float *x, float *y, cudaStream_t s);
 // the same in FP64 accuracy (sigma_pair_warp64.cu), where K's digits allow it
 bool pair_warp64_fits(const doci_ham *h);
+bool pair_warp64_wanted(const doci_ham *h);  // and where it is the faster for one vector
 int launch_pair_warp64(const doci_ham *h, const double *x, double *y, cudaStream_t s);
 // the reproducible forms: no atomic adds, pair_warp_slabs(h) vectors of D
 // elements of scratch

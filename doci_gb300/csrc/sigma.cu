@@ -1031,9 +1031,10 @@ int launch_sigma(const doci_ham *h, const void *x, void *y, int precision, cudaS
     case 4:
       return f64 ? launch_rowx<double>(h, x, y, st, 1) : launch_rowx<float>(h, x, y, st, 1);
     case 9:
-      // from 10 orbitals on the warp-per-unit form where K's digits allow it, else
-      // in float-float the pair form where it fits or the phase-ordered row pass
-      if (pair_warp64_fits(h))
+      // from 10 orbitals on the warp-per-unit form where K's digits allow it and it
+      // is the faster, else in float-float the pair form where it fits or the
+      // phase-ordered row pass
+      if (pair_warp64_wanted(h))
         return launch_pair_warp64(h, static_cast<const double *>(x), static_cast<double *>(y), st);
       if (pair_ff_fits(h)) return launch_pair_ff(h, static_cast<const double *>(x), static_cast<double *>(y), st);
       return launch_rowx_ff(h, static_cast<const double *>(x), static_cast<double *>(y), st);

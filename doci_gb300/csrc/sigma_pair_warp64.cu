@@ -1,7 +1,7 @@
 // sigma_pair_warp64.cu -- FP64-accurate sigma in the (N-1)-pair form, one warp
 // per unit, the product with K in exact integer arithmetic on the
 // 5th-generation tensor cores.  This is what kind 9 runs from 10 orbitals on,
-// where K allows it (ham_build_kdigits).
+// where K allows it (ham_build_kdigits) and sets have more than eight open slots.
 //
 // The tiling, unit lists and tables are those of the FP32 form
 // (sigma_pair_warp.cu).  The product Y_S = X_S K of a set needs about 50 bits.
@@ -547,6 +547,14 @@ int ham_build_kdigits(doci_ham *h) {
 }
 
 bool pair_warp64_fits(const doci_ham *h) { return pair_warp_fits(h) && h->kdig_ok; }
+
+// A set's work here is the same whatever its open slots, a float pair's goes with
+// their square: with up to eight slots (L - N + 1) the float-pair kernel is the faster,
+// from nine on this one.  Measured (us, float pairs / here): 7 slots L=26 N=20 116
+// / 162, L=32 N=26 632 / 714; 8 slots L=30 N=23 631 / 822, L=32 N=25 1,298 / 1,637,
+// L=22 N=15 equal; 9 slots L=28 N=20 1.19 times, L=24 N=16 1.21 and L=22 N=14 1.28
+// times faster here.  (The reproducible form runs here in any case.)
+bool pair_warp64_wanted(const doci_ham *h) { return pair_warp64_fits(h) && h->L - h->N + 1 > 8; }
 
 namespace {
 template <bool DET>

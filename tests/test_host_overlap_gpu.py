@@ -58,7 +58,7 @@ for prec, tdt in ((dg.FP32, torch.float32), (dg.FP64, torch.float64)):
 
 
 @pytest.mark.parametrize("L,N,seed,off,graded", [(22, 11, 31, 0, False), (24, 12, 30, 3, False), (20, 7, 33, 1, False),
-                                                 (12, 6, 35, 0, False), (22, 11, 36, 1, True), (13, 4, 37, 0, True)])
+                                                 (13, 5, 35, 0, False), (22, 11, 36, 1, True), (13, 4, 37, 0, True)])
 def test_overlapped_copies(L, N, seed, off, graded, synth):
     """FP32 between pinned buffers, and FP64 on a K that the float-pair kernel
     takes (into pinned and pageable y), go through the overlapped path: right

@@ -720,3 +720,21 @@ def test_sigma_block_scratch_is_given_back(synth, dg):
     h.close()
     torch.cuda.synchronize()
     assert torch.cuda.mem_get_info()[0] - held >= 0.9 * 13 * x.shape[1] * 4
+
+
+@pytest.mark.parametrize("L,N,seed", [(20, 11, 161), (20, 12, 162), (21, 14, 163), (22, 14, 164), (22, 15, 165), (26, 20, 166)])
+def test_sigma_fp64_open_slots(L, N, seed, synth, dg):
+    """The FP64-accurate pair form on both sides of the step from eight open slots per
+    set (float pairs) to nine (digits), on spaces without a neighbour table: the oracle's matvec."""
+    torch = torch_cuda()
+    p = synth(L, N, seed)
+    o = oracle.Ham(p)
+    with dg.Hamiltonian.from_fcidump(p) as h:
+        h.set_sigma_kernel("rowff")  # (the automatic choice too, unless the shape was tuned in this process)
+        assert h.sigma_plan(dg.FP64)[0] == 9
+        x = np.random.default_rng(seed).standard_normal(h.D)
+        xd, y = torch.from_numpy(x).cuda(), torch.full((h.D,), float("nan"), dtype=torch.float64, device="cuda")
+        h.sigma_device(xd.data_ptr(), y.data_ptr(), dg.FP64)
+        torch.cuda.synchronize()
+        ref = o.matvec(x)
+        assert np.abs(y.cpu().numpy() - ref).max() <= TOL64 * np.abs(ref).max()

@@ -80,7 +80,7 @@ with dg.Hamiltonian.from_fcidump(p) as h:
 
 
 # one tile in the only slot; one to three tiles a slot; slots with many units
-@pytest.mark.parametrize("L,N", [(10, 1), (12, 6), (22, 11)])
+@pytest.mark.parametrize("L,N", [(10, 1), (12, 4), (22, 11)])
 def test_warp_wait_limit_reports_timeout(L, N, synth):
     """The same for the warp-per-unit pair forms (kinds 6 and 9, and their
     reproducible forms in the block sigma on the space without a neighbour
