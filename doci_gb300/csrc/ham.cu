@@ -214,11 +214,11 @@ int ham_build(doci_ham *h, const Integrals &in) {
   DOCI_CUDA(cudaMemcpyAsync(h->d_tab64, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
   int st = launch_diagonal(h, h->stream);
   if (st) return st;
+  st = ham_build_nbr(h);  // runs while the host builds the other tables
+  if (st) return st;
   st = ham_build_rows(h);
   if (st) return st;
   st = ham_build_pair_warp(h);
-  if (st) return st;
-  st = ham_build_nbr(h);
   if (st) return st;
   DOCI_CUDA(cudaStreamSynchronize(h->stream));
   return DOCI_OK;
