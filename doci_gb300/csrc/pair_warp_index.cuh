@@ -104,7 +104,10 @@ inline Groups groups(int P, int na, int N, const uint32_t *B, int stride) {
 
 // Column orbitals of an (L, N) space for `slots` tile rows in flight, and the unit
 // list (0: fewer than 10 orbitals).  The more the fewer units: 12 as long as that
-// leaves four units per tile row, else 10 as long as each has one, else 8; but no
+// leaves four units per tile row, else 10 as long as it leaves one and a half (with
+// 1.36 the second round keeps a third of the rows busy: FP32 L=22 N=7 30.0 us, with
+// 8 24.6; with 1.56 both take 30.8 at L=22 N=8, with 2.1 10 is the faster, 37.0
+// against 43.0 at L=22 N=11), else 8; but no
 // more than 20 row orbitals, whose row starts take 4 MiB.  (That bounds only
 // spaces of few pairs or holes, up to 35,960 determinants, which run from their
 // neighbour table unless asked: L=32, N=2 would have 2^24 row starts for its 496
@@ -116,7 +119,7 @@ inline int column_orbitals(int L, int N, uint32_t slots, const uint32_t *B, int 
     if (L - p < 2 || L - p > kMaxRowOrbitals) continue;
     P = p;
     *g = groups(P, L - P, N, B, stride);
-    if (g->first[g->n] / 4 >= (p == 12 ? 4 : 1) * slots) break;
+    if (g->first[g->n] / 2 >= (p == 12 ? 8 : 3) * slots) break;
   }
   return P;
 }

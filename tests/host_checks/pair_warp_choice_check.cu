@@ -34,7 +34,7 @@ int main() {
           if (L - p < 2) continue;
           units = p;
           const doci::pw::Groups h = doci::pw::groups(p, L - p, N, B.data(), BC);
-          if (h.first[h.n] / 4 >= (p == 12 ? 4 : 1) * slots) break;
+          if (h.first[h.n] / 4.0 >= (p == 12 ? 4.0 : 1.5) * slots) break;
         }
         ok = ok && P == units;
       }
