@@ -210,7 +210,7 @@ bool tc_fits(const doci_ham *h);
 int tc_launches(const doci_ham *h);
 int launch_tc(const doci_ham *h, const float *x, float *y, cudaStream_t s, int *d_err, long spin_limit);
 int ham_build_pairs(doci_ham *h, const std::vector<uint32_t> &row_start);
-// block sigma scratch that no call uses goes back to the device (sigma.cu)
+// block sigma scratch that no call uses goes back to the device, all but 256 MiB (sigma.cu)
 void slab_pool_trim(int device);
 int launch_bitstrings(const doci_ham *h, int64_t first, int64_t count, uint32_t *out, cudaStream_t s);
 int launch_ranks(const doci_ham *h, const uint32_t *bits, int64_t count, int64_t *out, cudaStream_t s);

@@ -1076,7 +1076,10 @@ int multi_method_auto(const doci_ham *h, int precision) {
 constexpr size_t kDetMaxBytes = size_t(5) << 30;
 // The scratch has a pool of its own, which keeps it for the next call (mapped anew
 // for each, four vectors of 40.1M determinants took 9.4 ms in FP32 instead of 5.9)
-// and gives it back to the device when a handle is destroyed (slab_pool_trim).
+// and gives it back to the device, all but kSlabKeep, when a handle is destroyed
+// (slab_pool_trim).  Without kSlabKeep the first block sigma of the next handle
+// mapped its scratch again (2.7M determinants 768 us instead of 526).
+constexpr size_t kSlabKeep = size_t(256) << 20;
 std::mutex g_slab_mu;
 std::map<int, cudaMemPool_t> g_slab_pools;  // by device
 cudaMemPool_t slab_pool(int device) {
@@ -1273,8 +1276,8 @@ void slab_pool_trim(int device) {
   auto it = g_slab_pools.find(device);
   uint64_t held = 0;
   if (it != g_slab_pools.end() &&
-      cudaMemPoolGetAttribute(it->second, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess && held > 0)
-    cudaMemPoolTrimTo(it->second, 0);  // (what calls still use stays)
+      cudaMemPoolGetAttribute(it->second, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess && held > kSlabKeep)
+    cudaMemPoolTrimTo(it->second, kSlabKeep);  // (what calls still use stays)
   cudaGetLastError();
 }
 

@@ -164,7 +164,8 @@ int doci_sigma(doci_ham *ham, const void *d_x, void *d_y, int precision, void *s
  * spaces one vector after the other in
  * the pair form with every contribution in a place of its own (stream-ordered
  * scratch of at most min(N, L - 8) x D elements, up to 5 GiB, which no footprint call
- * counts and which is kept for the next call until a handle is destroyed; FP64
+ * counts and which is kept for the next call until a handle is destroyed, up to
+ * 256 MiB of it longer; FP64
  * also D x 8 bytes as doci_sigma); else, when there is
  * no memory for that, and while the stream is captured (so that the graph holds no
  * allocation), the neighbour ranks and hop weights of each

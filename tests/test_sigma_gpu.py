@@ -707,10 +707,10 @@ def test_sigma_block_captured_without_allocations(prec_name, nv, synth, dg):
 
 
 def test_sigma_block_scratch_is_given_back(synth, dg):
-    """The block sigma's scratch (13 vectors of 10.4M elements here) is the
-    device's again when the handle is destroyed."""
+    """The block sigma's scratch (14 vectors of 40.1M elements here) is the
+    device's again when the handle is destroyed, all but 256 MiB."""
     torch = torch_cuda()
-    L, N, nv = 26, 13, 2
+    L, N, nv = 28, 14, 2
     h = dg.Hamiltonian.from_fcidump(synth(L, N, 152))
     x = torch.randn((nv, h.D), dtype=torch.float32, device="cuda")
     y = torch.empty_like(x)
@@ -719,7 +719,7 @@ def test_sigma_block_scratch_is_given_back(synth, dg):
     held = torch.cuda.mem_get_info()[0]
     h.close()
     torch.cuda.synchronize()
-    assert torch.cuda.mem_get_info()[0] - held >= 0.9 * 13 * x.shape[1] * 4
+    assert torch.cuda.mem_get_info()[0] - held >= 14 * x.shape[1] * 4 - (256 << 20)
 
 
 @pytest.mark.parametrize("L,N,seed", [(20, 11, 161), (20, 12, 162), (21, 14, 163), (22, 14, 164), (22, 15, 165), (26, 20, 166)])
