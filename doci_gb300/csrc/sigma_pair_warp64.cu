@@ -39,6 +39,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <functional>
+#include <numeric>
 #include <vector>
 
 #include "addressing.cuh"
@@ -513,10 +515,11 @@ int ham_build_kdigits(doci_ham *h) {
   for (h->kdig_exp = ex + 2; !h->kdig_ok && h->kdig_exp <= ex + 6; ++h->kdig_exp) {
     if (big > 0 && std::ldexp(1.0, h->kdig_exp - 2) > 18 * small) break;
     double worst = 0;
+    const double scale = std::ldexp(1.0, -h->kdig_exp);
     for (int a = 0; a < L; ++a) {
-      std::vector<double> sums[3];
+      double sums[3][kMaxOrbitals];
       for (int b = 0; b < L; ++b) {
-        double v = std::ldexp(h->Kp[(L - 1 - a) * L + (L - 1 - b)], -h->kdig_exp), k[5];
+        double v = h->Kp[(L - 1 - a) * L + (L - 1 - b)] * scale, k[5];
         for (int j = 0; j < 5; ++j) {
           v *= 2048;
           const double d = std::nearbyint(v);
@@ -525,15 +528,14 @@ int ham_build_kdigits(doci_ham *h) {
           const __half hd = __float2half(static_cast<float>(d));
           dig[j * 1024 + a * 32 + b] = *reinterpret_cast<const uint16_t *>(&hd);
         }
-        sums[0].push_back(1024 * k[0] + 512 * k[1]);  // (i + j = 2, 512 k[0], is below it)
-        sums[1].push_back(1024 * k[0] + 512 * k[2]);
-        sums[2].push_back(1024 * k[1]);
+        sums[0][b] = 1024 * k[0] + 512 * k[1];  // (i + j = 2, 512 k[0], is below it)
+        sums[1][b] = 1024 * k[0] + 512 * k[2];
+        sums[2][b] = 1024 * k[1];
       }
+      const int n = std::min(open, L);
       for (auto &s : sums) {
-        std::sort(s.rbegin(), s.rend());
-        double sum = 0;
-        for (int t = 0; t < open && t < L; ++t) sum += s[t];
-        worst = std::max(worst, sum);
+        if (n < L) std::nth_element(s, s + n, s + L, std::greater<double>());
+        worst = std::max(worst, std::accumulate(s, s + n, 0.0));
       }
     }
     // (a margin for the sum of the two of i + j = 4, formed from their rounded sum)
