@@ -303,7 +303,7 @@ int doci_sigma_host(doci_ham *h, const void *x, void *y, int precision) {
   // down on the copy engines while the unit groups run).  Measured against
   // copy, warp-per-unit sigma, copy: 155M determinants 9.4 ms against 11.0,
   // 601M 35.6 against 43.0; but 40M 4.4 against 2.9, and at every size in FP64
-  // (601M: 134 against 103 ms; 10M: 4.0 against 1.8) and into pageable y (601M
+  // (601M: 134 against 107 ms; 10M: 4.0 against 1.9) and into pageable y (601M
   // FP32: 56 against 44 ms).
   const bool y_pinned = mapped_host(y) != nullptr;
   if (sched && precision == DOCI_FP32 && kind == 6 && pair_fits(h) && y_pinned) {

@@ -166,7 +166,8 @@ int launch_typed(const doci_ham *h, const void *x, void *y, cudaStream_t st) {
 // 1,287 determinants 7.8 (what a call costs the host) against 10.5; 12,870 8.5
 // against 13.7; 48,620 14.6 against 26.8 / 22.3; 92,378 24.7 against 33.0 /
 // 27.0.  FP32 12,870 8.5 against 12.5 / 16.6; 48,620 12.4 against 16.5 / 16.6;
-// 92,378 16.6 against 18.6 / 16.8.  The table is at most 32 MiB: from there on
+// 92,378 16.6 against 18.6 / 16.8.  (On a vector not seen before, with the table out
+// of L2, FP32 48,620 42.9 against 49.4.)  The table is at most 32 MiB: from there on
 // the pair form is the faster.  Error against 64 bits in FP32 3.5e-8 to 4e-8
 // (gather kernel 1.4e-7 to 2.5e-7, pair form 6.6e-8 to 8.8e-8), in FP64 against
 // 128-bit sums 4.5e-17 to 1.3e-16 (gather kernel 1.5e-16 to 4e-15).
@@ -972,7 +973,7 @@ SigmaPlan plan_kind(const doci_ham *h, int precision, bool allow_pair, int kind)
   if (kind == 9 && precision == DOCI_FP64 && (pair_ff_fits(h) || (h->nrows >= 1 && rowx_fits(h, sizeof(ff)))))
     return {9, 2};
   // the automatic FP64 choice where the pair tiling gives every SM work: the
-  // FP64-accurate pair form (L=32, N=16: 53.7 ms; the row pass 444.9 ms)
+  // FP64-accurate pair form (L=32, N=16: 59.4 ms; the row pass 444.9 ms)
   if (kind == 0 && !h->d_nbr && allow_pair && precision == DOCI_FP64 && h->npblocks >= device_sm_count() &&
       pair_ff_fits(h))
     return {9, 2};
@@ -1022,7 +1023,7 @@ int launch_sigma(const doci_ham *h, const void *x, void *y, int precision, cudaS
       [[fallthrough]];
     case 6:
       // from 10 orbitals on the warp-per-unit form (faster at every size measured
-      // from L=18 on: 18.8 -> 16.7 us there, 33.9 -> 16.9 ms at L=32)
+      // from L=18 on: 18.8 -> 16.7 us there, 33.9 -> 17.1 ms at L=32)
       if (pair_warp_fits(h))
         return launch_pair_warp(h, static_cast<const float *>(x), static_cast<float *>(y), st);
       return launch_pair(h, static_cast<const float *>(x), static_cast<float *>(y), st);
@@ -1071,7 +1072,7 @@ int multi_method_auto(const doci_ham *h, int precision) {
 // order, up to kDetMaxBytes of scratch (40.1M determinants in FP64: 4.2 GiB).
 // Measured against the multi-vector row and gather kernels (us, nv = 2 / 4):
 // FP32 L=24 N=12 1,256 / 1,455 -> 247 / 490; L=20 N=10 140 / 155 -> 52 / 101;
-// FP64 L=24 2,915 / 3,113 -> 725 / 1,444.  (Spaces with a neighbour table take
+// FP64 L=24 2,915 / 3,113 -> 770 / 1,530.  (Spaces with a neighbour table take
 // the gather kernel.)
 constexpr size_t kDetMaxBytes = size_t(5) << 30;
 // The scratch has a pool of its own, which keeps it for the next call (mapped anew

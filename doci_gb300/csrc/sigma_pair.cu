@@ -1,9 +1,10 @@
 // sigma_pair.cu -- the (N-1)-pair intermediate form with one block per unit:
 // FP32 on the warp-level mma.sync path (below 10 orbitals, and in
 // doci_sigma_host on large spaces, where its units run in groups between the
-// pieces of the copies) and FP64-accurate in float pairs (below 10 orbitals).
-// From 10 orbitals on kinds 6 and 9 run sigma_pair_warp.cu and
-// sigma_pair_warp64.cu; the tcgen05 version with one block per unit is
+// pieces of the copies) and FP64-accurate in float pairs (below 10 orbitals, with
+// up to eight open slots per set, and for a K that the digits of
+// sigma_pair_warp64.cu do not hold as well).  Otherwise kinds 6 and 9 run
+// sigma_pair_warp.cu and sigma_pair_warp64.cu; the tcgen05 version with one block per unit is
 // sigma_tc.cu (kind 8).
 //
 // Every off-diagonal element of the DOCI Hamiltonian is a pair hop

@@ -30,8 +30,8 @@
 // L=18 N=9 69 / 27 / 16.8.
 //
 // Measured against the one-block-per-unit mma.sync kernel of sigma_pair.cu:
-// L=32 N=16 33.9 -> 16.9 ms (one warp for both jobs 19.1), L=28 N=14 1.82 ->
-// 1.11 ms (1.23), L=27 N=11 524 -> 303 us (331), L=20 N=10 28.0 -> 20.4 us
+// L=32 N=16 33.9 -> 17.1 ms (one warp for both jobs 19.1), L=28 N=14 1.82 ->
+// 1.11 ms (1.23), L=27 N=11 524 -> 305 us (331), L=20 N=10 28.0 -> 20.4 us
 // (20.9).  Bound by instruction issue (65 % of the slots, 690 warp instructions
 // per 32 sets), the shared-memory pipe (60 %) and the latency of the hole rows.
 // Two sets per lane, two tiles per warp pair: fewer instructions (628), but

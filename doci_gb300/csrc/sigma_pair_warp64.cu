@@ -6,7 +6,7 @@
 // The tiling, unit lists and tables are those of the FP32 form
 // (sigma_pair_warp.cu).  The product Y_S = X_S K of a set needs about 50 bits.
 // On the FP32 units a product and its sum in float pairs take 12 operations,
-// and GB300's FP64 units do two lanes per clock and SM.  Here a set's values
+// and GB300's FP64 units do 1/64 of the FP32 rate.  Here a set's values
 // are brought to a common exponent (the largest value's) and cut into five
 // signed digits of eleven bits, K likewise once per handle; both are integers of magnitude at most
 // 1,088 and exact in FP16, and a digit of X times a digit of K over the set's
@@ -29,11 +29,11 @@
 // gather, cut and hand over the next tile of a slot while warps 8-15 read and
 // scatter the one before.
 //
-// Measured: L=28 N=14 7.33 -> 3.84 ms, L=23 N=9 159 -> 84 us (3.58 ms and 80 us
-// with 2 x 2 in the accumulator of 4), against one unit per block with float
+// Measured: L=32 N=16 134.6 -> 59.4 ms, L=28 N=14 7.33 -> 3.84 ms, L=23 N=9 159 ->
+// 84 us (3.58 ms and 80 us with 2 x 2 in the accumulator of 4), against one unit per block with float
 // pairs on the FP32 units; the hop sums' error against FP64 sums 2.0e-15 to
 // 3.3e-15 of their norm, from 3.5e-15 to 5.4e-15.  Bound by instruction issue
-// (1,870 warp instructions per 32 sets, 60 % of the issue slots).
+// (1,980 warp instructions per 32 sets, 58 % of the issue slots).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 

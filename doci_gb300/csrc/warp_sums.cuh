@@ -1,7 +1,7 @@
 // warp_sums.cuh -- sums of many FP64 (or FP32) values over a warp, in FP64.
 //
 // Reducing K values one after the other takes 5 K shuffle-and-add steps on all
-// 32 lanes, and FP64 adds run at two lanes per clock and SM on GB300: for the
+// 32 lanes, and FP64 adds run at 1/64 of the FP32 rate on GB300: for the
 // 33 projections of a block of 8 warps that is about 10 us per block, more
 // than the pass's own reads on a small vector.  Here the lanes split the
 // values instead: in the first step a lane keeps half of them and hands the

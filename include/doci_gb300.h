@@ -194,8 +194,12 @@ int doci_sigma_block(doci_ham *ham, const void *d_X, int64_t ldx, void *d_Y, int
  * written once; needs a 16-byte aligned x, else kind 6 runs), 9 the
  * (N-1)-pair form in FP64 accuracy (FP64 only: x as pairs of FP32 values in
  * stream-ordered scratch of D x 8 bytes, converted once per call, the products
- * exact in digits on the tensor cores, or below 10 orbitals in float pairs on
- * the FP32 units, FP64 atomic adds into sigma; the phase-ordered row
+ * exact in digits on the tensor cores, or in float pairs on the FP32 units below 10
+ * orbitals, with up to eight open orbitals per (N-1)-pair set (L - N + 1) and where
+ * the smallest element of K that is not zero is below about 1/18 of the largest, FP64
+ * atomic adds into sigma; a set's values have one exponent in the digit form, so
+ * the hops of a determinant are good to about 2^-50 of the largest |x| of its
+ * neighbours' sets times the largest |K|; the phase-ordered row
  * pass in float pairs where the pair tiling does not fit; FP32
  * requests for it use the automatic choice).  Kinds 6, 8 and 9 reduce into
  * sigma with atomic adds, so their last bits vary between runs; FP64
@@ -215,8 +219,8 @@ int doci_ham_set_sigma_kernel(doci_ham *ham, int kind);
  * pair form allowed) and the pair-free path of the block solves; nvec = 2..4
  * tunes the block sigma of nvec vectors (doci_sigma_block, doci_solve_roots
  * with that many roots; *choice = 1 row pass in groups, 2 gather, 3 one
- * vector at a time).  FP64 shapes below 2^18 determinants keep to the paths
- * without atomic adds (kinds 1, 3, 4).  Synchronous; a few sigma calls per candidate.  The
+ * vector at a time).  The pair-free path and FP64 shapes below 2^18 determinants
+ * keep to the paths without atomic adds (kinds 1, 3, 4).  Synchronous; a few sigma calls per candidate.  The
  * choices change which kernels run, so results computed before and after a
  * tuning may differ in their last bits; tune before a batch whose results
  * are compared to single solves.  No counterpart in the reference. */
