@@ -335,7 +335,9 @@ int doci_solve(doci_ham *ham, const doci_solve_opts *opts, double *vec,
 int doci_solve_trace(doci_ham *ham, const doci_solve_opts *opts, double *vec, doci_solve_result *result,
                      double *trace, int trace_len, int *trace_count);
 
-/* Bytes of device memory a solve of ham with opts needs (admission). */
+/* Bytes of device memory a solve of ham with opts needs (admission): the vectors,
+ * the diagonals and the neighbour table; a handle's other tables (at most about 16
+ * MiB at the largest sizes) are not counted. */
 int64_t doci_solve_footprint(int L, int n_pairs, const doci_solve_opts *opts, int nroots);
 
 /* ------------------------------------------------------------------------ */

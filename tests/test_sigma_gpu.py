@@ -738,3 +738,28 @@ def test_sigma_fp64_open_slots(L, N, seed, synth, dg):
         torch.cuda.synchronize()
         ref = o.matvec(x)
         assert np.abs(y.cpu().numpy() - ref).max() <= TOL64 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("ratio", [1.5, 8.0, 17.9, 18.6, 64.0])
+def test_fp64_hops_at_the_digits_limit(ratio, dg):
+    """Elements of K up to 18 times smaller than the power of two above the
+    largest go through the digits, smaller ones through float pairs: on one-hot
+    vectors each product is good to 2^-45 either way (in the digits at 18: what is
+    cut is 4 x 2^20 x 2^-77 of x k > 2^-9.2, K's rounding 2^-49.8 of it, the pair's 2^-48)."""
+    torch = torch_cuda()
+    L, N = 20, 10
+    rng = np.random.default_rng(21)
+    K = np.where(rng.random((L, L)) < 0.5, rng.uniform(0.9, 0.999, (L, L)), rng.uniform(1.0, 1.03, (L, L)) / ratio)
+    K = np.triu(K, 1) + np.triu(K, 1).T
+    with dg.Hamiltonian.from_integrals(L, N, 0.0, *pair_integrals(np.linspace(-1, 1, L), K)) as h:
+        D = h.D
+        x = torch.zeros(D, dtype=torch.float64, device="cuda")
+        ref, y = torch.empty_like(x), torch.empty_like(x)
+        for at in rng.integers(0, D, 6):
+            x.zero_()
+            x[int(at)] = float(rng.standard_normal())
+            for kind, out in (("rowx", ref), ("rowff", y)):
+                h.set_sigma_kernel(kind)
+                h.sigma_device(x.data_ptr(), out.data_ptr(), dg.FP64)
+            torch.cuda.synchronize()
+            assert bool(((y - ref).abs() <= 2.0 ** -45 * ref.abs()).all())
