@@ -484,9 +484,10 @@ int launch_p(const doci_ham *h, const PwShape &s, const ff *x, double *y, double
 // K (mirrored orbitals) as five signed digits of eleven bits, below 1/4:
 // K = 2^exp sum_j k_j 2^(-11 j), FP16, digit j at [j - 1][32][32].  The
 // accumulators of i + j = 2, 3 and 4 (2 x 2 apart) have to hold their sums
-// exactly whatever X: |x_1| <= 512, |x_i| <= 1024 over the L - N + 1 open slots of a
-// set.  Where K's digits do not allow that, other digits are tried (a larger
-// exponent, at a bit of K each); kdig_ok is false when none do.
+// exactly whatever X: |x_1| <= 512, |x_2| <= 1024, |x_3| <= 1088 (the low part comes in
+// there) over the L - N + 1 open slots of a set.  Where K's digits do not allow that,
+// other digits are tried (a larger exponent, at a bit of K each); kdig_ok is false when
+// none do.
 //
 // The digits keep K to 2^-56 of 2^exp, the float-pair kernel each element of K
 // to itself, so small elements beside large ones have fewer bits here.  kdig_ok
@@ -529,7 +530,7 @@ int ham_build_kdigits(doci_ham *h) {
           dig[j * 1024 + a * 32 + b] = *reinterpret_cast<const uint16_t *>(&hd);
         }
         sums[0][b] = 1024 * k[0] + 512 * k[1];  // (i + j = 2, 512 k[0], is below it)
-        sums[1][b] = 1024 * k[0] + 512 * k[2];
+        sums[1][b] = 1088 * k[0] + 512 * k[2];
         sums[2][b] = 1024 * k[1];
       }
       const int n = std::min(open, L);
