@@ -8,18 +8,19 @@
 // On the FP32 units a product and its sum in float pairs take 12 operations,
 // and GB300's FP64 units do 1/64 of the FP32 rate.  Here a set's values
 // are brought to a common exponent (the largest value's) and cut into five
-// signed digits of eleven bits, K likewise once per handle; both are integers of magnitude at most
-// 1,088 and exact in FP16, and a digit of X times a digit of K over the set's
-// open slots is an integer that FP32 accumulates exactly (Ozaki, Ogita, Oishi
+// signed digits of eleven bits, K likewise once per handle; both are integers of
+// magnitude at most 1,088 and exact in FP16, and a digit of X times a digit of K over
+// the set's open slots is an integer that FP32 accumulates exactly (Ozaki, Ogita, Oishi
 // and Rump, "Error-free transformations of matrix multiplication by using fast
 // routines of matrix multiplication and its applications", 2012).  Digits i of
 // X and j of K go into the accumulator of i + j = 2..6, digit 2 times digit 2 into
 // one of its own.  |x_1| <= 512 and the host's check of K's digits keep the
 // accumulators of i + j = 2, 3 and 4 below 2^24 for any X (with 2 x 2 in the
 // accumulator of 4 a constant K of 24 open slots passed 2^24, at 1.5e-13); those of
-// the smaller sums could round only if the digits' signs conspired, and then by
-// 2^-55 of the largest |x| |K|.  What is cut is below
-// 2^-51 of the largest |x| |K|.  The six sums are put together as a float
+// the smaller sums round only if the digits' signs conspire, by a few units of 2^-55
+// where the largest |x| |K| is 2^-6 to 2^-4 (constant vectors and K, emulated: 2.6e-15
+// of the sum of the terms).  What is cut is below 2^-51 of the largest |x| |K|.  The
+// six sums are put together as a float
 // pair with exact rounding errors.  The own row's sums stay float pairs in
 // shared memory; what leaves the SM is widened to double by integer
 // operations and added with FP64 atomics to sigma = diag x.
@@ -29,9 +30,9 @@
 // gather, cut and hand over the next tile of a slot while warps 8-15 read and
 // scatter the one before.
 //
-// Measured: L=32 N=16 134.6 -> 59.4 ms, L=28 N=14 7.33 -> 3.84 ms, L=23 N=9 159 ->
-// 84 us (3.58 ms and 80 us with 2 x 2 in the accumulator of 4), against one unit per block with float
-// pairs on the FP32 units; the hop sums' error against FP64 sums 2.0e-15 to
+// Measured against one unit per block with float pairs on the FP32 units: L=32 N=16
+// 134.6 -> 59.4 ms, L=28 N=14 7.33 -> 3.84 ms, L=23 N=9 159 -> 84 us (3.58 ms and
+// 80 us with 2 x 2 in the accumulator of 4); the hop sums' error against FP64 sums 2.0e-15 to
 // 3.3e-15 of their norm, from 3.5e-15 to 5.4e-15.  Bound by instruction issue
 // (1,980 warp instructions per 32 sets, 58 % of the issue slots).
 #include <cuda_fp16.h>
@@ -44,6 +45,7 @@
 #include <vector>
 
 #include "addressing.cuh"
+#include "f32x2.cuh"
 #include "ff.cuh"
 #include "internal.h"
 #include "pair_warp.h"
@@ -71,29 +73,6 @@ constexpr int kOffStart = kOffExp + kSlots * 2 * 128 * 4;
 constexpr int kOffCells = kOffStart + 4 * 24 * (kThreads64 / 32);
 constexpr size_t kMinSmem = 120 * 1024;     // one block per SM: it allocates all of the tensor memory
 
-typedef unsigned long long f2;              // two floats
-__device__ __forceinline__ f2 pk(float a, float b) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void up(f2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ f2 addp(f2 a, f2 b) {
-  f2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 mulp(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 subp(f2 a, f2 b) { return fma2(b, pk(-1.f, -1.f), a); }
 __device__ __forceinline__ uint32_t half2_bits(f2 v) {  // (FP16 of the first) | (FP16 of the second) << 16
   float a, b;
   up(v, a, b);
@@ -284,7 +263,8 @@ sigma_pair_warp64_kernel(const __grid_constant__ PwShape s, const uint32_t *__re
           // X 2^(124 - eb) = sum_i d_i 2^(-11 i), below 1/4, d_i the nearest
           // integer each time, every remainder exact but the last bits of h + l
           // past 2^-57
-          const f2 c2048 = pk(2048.f, 2048.f), magic = pk(12582912.f, 12582912.f), nmagic = pk(-12582912.f, -12582912.f);
+          const f2 c2048 = pk(2048.f, 2048.f);
+          const f2 magic = pk(12582912.f, 12582912.f), nmagic = pk(-12582912.f, -12582912.f);
 #pragma unroll
           for (int hf = 0; hf < 2; ++hf) {
             uint32_t d1[8], d2[8], d3[8], d4[8], d5[8];

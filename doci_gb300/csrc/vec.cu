@@ -24,6 +24,7 @@
 #include <atomic>
 #include <type_traits>
 
+#include "f32x2.cuh"
 #include "internal.h"
 #include "vec.h"
 #include "warp_sums.cuh"
@@ -143,29 +144,7 @@ multidot_kernel(const double *__restrict__ V, size_t ld, int m, const double *__
 // instructions per element and two columns; groups of four with packed instructions
 // 665 us with two blocks per SM, 716 with four (spills), one column at a time 720
 // to 800.  (491 us in pairs of floats, eleven instructions.)
-constexpr int kRun = 64, KF = 2;  // (columns per block)
-typedef unsigned long long f2;  // two floats
-__device__ __forceinline__ f2 pk(float a, float b) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void up(f2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ f2 addp(f2 a, f2 b) {
-  f2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 mulp(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
+constexpr int kRun = 64, KF = 2;  // products per run, columns per block
 __global__ void __launch_bounds__(kT, 4)
 multidot_exact_f32_kernel(const float *__restrict__ V, size_t ld, int m, const float *__restrict__ w, size_t n,
                           double *__restrict__ partials) {

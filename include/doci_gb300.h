@@ -161,20 +161,17 @@ int doci_sigma(doci_ham *ham, const void *d_x, void *d_y, int precision, void *s
 /* Block sigma Y_v = H X_v for v < nv on device buffers: X and Y column-major
  * with leading dimensions ldx, ldy >= D (elements).  Without atomic adds (unless
  * doci_ham_set_sigma_kernel set kind 9): results repeat bit for bit.  On large
- * spaces one vector after the other in
- * the pair form with every contribution in a place of its own (stream-ordered
- * scratch of at most min(N, L - 8) x D elements, up to 5 GiB, which no footprint call
- * counts and which is kept for the next call until a handle is destroyed, up to
- * 256 MiB of it longer; FP64
- * also D x 8 bytes as doci_sigma); else, when there is
- * no memory for that, and while the stream is captured (so that the graph holds no
- * allocation), the neighbour ranks and hop weights of each
- * determinant are computed once per launch for up to four vectors (larger nv
- * runs in groups of four).  Results agree with doci_sigma to
- * rounding (identical when both use the same kernel).  No counterpart in the
- * reference, whose matvec (doci.c:164-238) takes one vector; for callers with
- * block methods.  Asynchronous on stream (NULL = the
- * default stream). */
+ * spaces one vector after the other in the pair form, with every contribution in
+ * a place of its own: stream-ordered scratch of at most min(N, L - 8) x D elements,
+ * up to 5 GiB (FP64 also D x 8 bytes, as doci_sigma), which no footprint call counts
+ * and which is kept for the next call until a handle is destroyed, up to 256 MiB of
+ * it longer.  Else, when there is no memory for that, and while the stream is
+ * captured (so that the graph holds no allocation), the neighbour ranks and hop
+ * weights of each determinant are computed once per launch for up to four vectors
+ * (larger nv runs in groups of four).  Results agree with doci_sigma to rounding
+ * (identical when both use the same kernel).  No counterpart in the reference,
+ * whose matvec (doci.c:164-238) takes one vector; for callers with block methods.
+ * Asynchronous on stream (NULL = the default stream). */
 int doci_sigma_block(doci_ham *ham, const void *d_X, int64_t ldx, void *d_Y, int64_t ldy, int nv, int precision,
                      void *stream);
 
